@@ -634,17 +634,16 @@ namespace
         return ISAACB_OK;
     }
 
-    // the merge's launch parameters from a context's state (no launch, no stream work)
     // Slot order of the combined textures for the camera of the merge about to run
-    // (Geom::yfast).  The ray-march reads a brick's slots in the order the image's pixels
-    // walk the volume: x fastest suits views whose image x axis stays close to the volume's
-    // x axis, y fastest (with warps of 4 x 8 pixels) views about the y axis seen from the
-    // side, whose image columns follow y.  Measured over an orbit about y at 20 degrees of
-    // pitch on 4 x 512^3 sources (a 2.5 GB texture), the two orders cross at 45 degrees of
-    // yaw (|image x . volume x| = 0.71); on a 0.33 GB texture (256^3) y fastest was 1 %
-    // slower at 94 degrees, as L2 then holds much of the texture and the access order
-    // matters less, so the automatic choice applies to textures beyond 4x the L2 cache.
-    // Only the speed depends on it: both orders hold the same texels.
+    // (Geom::yfast).  The march's warps walk the slots' fast axis with image rows (x fastest)
+    // or image columns (y fastest), and L1 serves a load the faster the closer those stay to
+    // the axis: y fastest is taken when the image y axis is closer to the volume's y axis
+    // than the image x axis to the volume's x.  Counted over sampled warps of a 512^3 volume
+    // at 1920x1080 (L1 cycles a load, x / y fastest): pitch 20 degrees 5.7 / 5.9 at yaw 0,
+    // 7.5 / 6.1 at 30, 12.8 / 6.2 at 45, 14.5 / 5.9 at 90; pitch 34 degrees 7.0 / 10.9 at yaw
+    // 30, 11.8 / 10.5 at 45.  On textures that L2 holds much of the choice is left at x
+    // fastest: for the full-feature scene (256^3, 0.33 GB) y fastest costs its pixel passes
+    // more than it gains.  Only the speed depends on it: both orders hold the same texels.
     int32_t slot_order_for_camera(const isaacb_ctx* c)
     {
         if(c->slotOrder >= 0)
@@ -659,9 +658,10 @@ namespace
         if(!(nx > 0.0) || !(ny > 0.0))
             return 0;
         const double ex = std::fabs(ix[0]) / nx, ey = std::fabs(iy[1]) / ny;
-        return ex < 0.7071 && ey > ex ? 1 : 0;
+        return ey > ex ? 1 : 0;
     }
 
+    // the merge's launch parameters from a context's state (no launch, no stream work)
     void prepare_merge(isaacb_ctx* c, MergeParams& p)
     {
         p.g = c->g;
@@ -1756,6 +1756,17 @@ namespace
         inverse4(PM, out);
     }
 
+    // Slot order of the textures that the batch's own merges write: the views look from every
+    // side, and y fastest suits any yaw at moderate pitch (slot_order_for_camera: 5.4-6.2 L1
+    // cycles a load up to 20 degrees of pitch, 10-11 at 34) where x fastest is as good only
+    // within 20 degrees of one axis and takes 12-15 beyond 45.  Set before the tables and the
+    // merge parameters are formed.
+    void batch_slot_orders(isaacb_batch* b)
+    {
+        for(isaacb_ctx* c : b->ctxs)
+            c->g.yfast = c->slotOrder >= 0 ? c->slotOrder : 1;
+    }
+
     // host mirror of the device tables from the contexts' current state; uploaded on `st`
     isaacb_status batch_refresh(isaacb_batch* b, cudaStream_t st)
     {
@@ -1832,8 +1843,6 @@ namespace
                         return batch_fail(ISAACB_NOT_READY, "isaacb_batch: a source has no memory");
                 if(compact_guarded(c, st) != ISAACB_OK)
                     return batch_fail(ISAACB_CUDA_ERROR, std::string("isaacb_batch: ") + c->lastError);
-                // the batch kernel's views look from every side: x-fastest slots
-                c->g.yfast = 0;
                 MergeParams p{};
                 prepare_merge(c, p);
                 if(capture)
@@ -2005,6 +2014,8 @@ extern "C"
         if(!b)
             return ISAACB_INVALID_ARG;
         cudaStream_t st = (cudaStream_t) stream;
+        if(update)
+            batch_slot_orders(b);
         isaacb_status r = batch_upload_luts(b, st);
         if(r == ISAACB_OK)
             r = batch_refresh(b, st);
@@ -2018,6 +2029,8 @@ extern "C"
         if(!b || !stream)
             return batch_fail(ISAACB_INVALID_ARG, "isaacb_batch_capture: needs a non-default stream");
         cudaStream_t st = (cudaStream_t) stream;
+        if(update)
+            batch_slot_orders(b);
         isaacb_status r = batch_upload_luts(b, st);
         if(r == ISAACB_OK)
             r = batch_refresh(b, st);
@@ -2050,6 +2063,8 @@ extern "C"
         if(!b || !b->graphExec)
             return batch_fail(ISAACB_NOT_READY, "isaacb_batch_launch_graph: no captured graph");
         cudaStream_t st = (cudaStream_t) stream;
+        if(b->graphUpdate)
+            batch_slot_orders(b);
         // functors, weights, storage or source memory changed: the merges in the graph are out of date
         if(batch_graph_stale(b))
         {

@@ -176,3 +176,26 @@ def test_batch_rejects_unbatchable_contexts():
     with pytest.raises(_lib.IsaacError):
         b.setConfig(24, 8)  # not 256 pixels
     b.close()
+
+
+@pytest.mark.parametrize("order", [0, 1])
+@pytest.mark.parametrize("tile", [(32, 8), (64, 4)])
+def test_batch_slot_orders(order, tile):
+    """Views of textures in either slot order, merged by the batch or by the context
+    itself (whose own order may differ from the other contexts'), equal single views."""
+    sc = _scenes()
+    vis = [build_gpu(s) for s in sc]
+    vis[0].setSlotOrder(order)
+    views = [(ci, w, h, *_camera(w, h, seed, sc[ci])) for ci, w, h, seed in VIEWS]
+    batch = IsaacBatch(vis, views)
+    refs = [_reference(sc[ci], w, h, seed) for ci, w, h, seed in VIEWS]
+    batch.setConfig(*tile)
+    batch.render(update=True)
+    _check(batch, refs)
+    vis[0].setSlotOrder(1 - order)
+    vis[0].update()
+    batch.render(update=False)
+    _check(batch, refs)
+    batch.close()
+    for v in vis:
+        v.close()
