@@ -22,6 +22,7 @@ namespace isaacb
         int Ho, Wo, Cout, Npad, Kpad;
         int ks, stride, pad, transposed;
         int relu, accumulate;
+        int step, tiles; // set by the launcher: residue classes per axis of the output pixels, and all classes' tiles
         int* errorFlag;
         // failure-detection check: non-zero = before any copy or MMA, wait this many ns on
         // an mbarrier that nothing arrives at, raise errorFlag, release TMEM and return
@@ -80,6 +81,6 @@ namespace isaacb
     // the row-tile kernel takes this convolution (and then honours xUp)
     bool row_tiles_apply(const ConvGemmParams& p);
     size_t conv_wgrad_smem(int Npad);
-    bool launch_conv_gemm(const ConvGemmParams& p, cudaStream_t s);
+    bool launch_conv_gemm(ConvGemmParams p, cudaStream_t s);
     bool launch_conv_wgrad(WgradParams p, cudaStream_t s);
 } // namespace isaacb

@@ -143,10 +143,11 @@ namespace isaacb
                 return;
             }
 
-            const int P = p.B * p.Ho * p.Wo;
-            const int nTiles = (P + kTileM - 1) / kTileM;
-            const int nk = p.Kpad / kChunkK;
-            const int taps = p.ks * p.ks;
+            // Output pixels go by residue class (y mod step, x mod step): an input gradient of
+            // stride s reaches a pixel only through the taps of its class, so with step = s a
+            // tile walks those taps alone ((ks / s)^2 on average) instead of all ks^2 with the
+            // others multiplied as zeros.  Every other convolution is one class of all taps.
+            const int step = p.step;
             const int m = tid & (kTileM - 1);
             const int jBase = tid >> 7;
             const uint32_t idesc = tc::idesc_bf16(kTileM, p.Npad, false, false);
@@ -154,32 +155,66 @@ namespace isaacb
             uint32_t G0 = 0;
             uint32_t donePhase = 0;
 
-            for(int tile = blockIdx.x; tile < nTiles; tile += gridDim.x)
+            for(int tile = blockIdx.x; tile < p.tiles; tile += gridDim.x)
             {
-                const int pix = tile * kTileM + m;
-                const bool valid = pix < P;
+                // the tile's class (cy, cx), its Hc x Wc grid of pixels and its taps
+                int cy = 0, cx = 0, Hc = p.Ho, Wc = p.Wo, local = tile;
+                for(int c = 0; c < step * step; ++c)
+                {
+                    cy = c / step;
+                    cx = c - cy * step;
+                    Hc = (p.Ho - cy + step - 1) / step;
+                    Wc = (p.Wo - cx + step - 1) / step;
+                    const int n = (p.B * Hc * Wc + kTileM - 1) / kTileM;
+                    if(local < n)
+                        break;
+                    local -= n;
+                }
+                const int ty0 = step > 1 ? (cy + p.pad) % step : 0, tx0 = step > 1 ? (cx + p.pad) % step : 0;
+                const int nty = max(0, (p.ks - ty0 + step - 1) / step), ntx = max(0, (p.ks - tx0 + step - 1) / step);
+                const int kTotal = nty * ntx * p.Cg;
+                const int nk = (kTotal + kChunkK - 1) / kChunkK;
+                const int pc = local * kTileM + m;
+                const bool valid = pc < p.B * Hc * Wc;
                 int b = 0, oy = 0, ox = 0;
                 if(valid)
                 {
-                    ox = pix % p.Wo;
-                    const int t = pix / p.Wo;
-                    oy = t % p.Ho;
-                    b = t / p.Ho;
+                    ox = pc % Wc;
+                    const int t = pc / Wc;
+                    oy = t % Hc;
+                    b = t / Hc;
+                    ox = cx + step * ox;
+                    oy = cy + step * oy;
                 }
-                auto load_chunk = [&](int kc, uint32_t G) {
+                const int pix = (b * p.Ho + oy) * p.Wo + ox;
+                // a thread's four 16-byte pieces of a chunk: tap (its place in the class's
+                // list, by row and column) and channel, advanced chunk by chunk
+                int pty[4], ptx[4], pch[4];
+#pragma unroll
+                for(int q = 0; q < 4; ++q)
+                {
+                    pty[q] = ptx[q] = 0;
+                    pch[q] = (jBase + 2 * q) * 8;
+                }
+                auto load_chunk = [&](uint32_t G) {
                     const uint32_t stage = sA + (G % kStages) * uint32_t(kStageBytesA);
 #pragma unroll
                     for(int q = 0; q < 4; ++q)
                     {
-                        const int j = jBase + 2 * q;
-                        const int k = kc * kChunkK + j * 8;
-                        const int t = k / p.Cg;
-                        const int c = k - t * p.Cg;
+                        while(pch[q] >= p.Cg)
+                        {
+                            pch[q] -= p.Cg;
+                            if(++ptx[q] == ntx)
+                            {
+                                ptx[q] = 0;
+                                ++pty[q];
+                            }
+                        }
                         const bf16* src = p.x;
                         uint32_t bytes = 0;
-                        if(valid && t < taps)
+                        if(valid && pty[q] < nty)
                         {
-                            const int ty = t / p.ks, tx = t - ty * p.ks;
+                            const int ty = ty0 + step * pty[q], tx = tx0 + step * ptx[q];
                             int iy, ix;
                             bool ok;
                             if(!p.transposed)
@@ -198,12 +233,14 @@ namespace isaacb
                             }
                             if(ok)
                             {
-                                src = p.x + ((size_t(b) * p.H + iy) * p.W + ix) * p.Cg + c;
+                                src = p.x + ((size_t(b) * p.H + iy) * p.W + ix) * p.Cg + pch[q];
                                 bytes = 16;
                             }
                         }
+                        const int j = jBase + 2 * q;
                         const uint32_t dst = stage + uint32_t(m >> 3) * 1024u + uint32_t(j) * 128u + uint32_t(m & 7) * 16u;
                         tc::cp_async16(dst, src, bytes);
+                        pch[q] += kChunkK;
                     }
                 };
 
@@ -214,7 +251,7 @@ namespace isaacb
                         const uint32_t G = G0 + c;
                         if(G >= kStages && !tc::mbar_wait(&sEmpty[G % kStages], ((G / kStages) - 1) & 1))
                             raise_error(p.errorFlag, abortLocal);
-                        load_chunk(c, G);
+                        load_chunk(G);
                     }
                     tc::cp_async_commit();
                 }
@@ -226,7 +263,7 @@ namespace isaacb
                         const uint32_t G = G0 + kn;
                         if(G >= kStages && !tc::mbar_wait(&sEmpty[G % kStages], ((G / kStages) - 1) & 1))
                             raise_error(p.errorFlag, abortLocal);
-                        load_chunk(kn, G);
+                        load_chunk(G);
                     }
                     tc::cp_async_commit();
                     tc::cp_async_wait<kStages - 1>();
@@ -244,8 +281,18 @@ namespace isaacb
 #pragma unroll
                         for(int j = 0; j < kChunkK / 16; ++j)
                         {
+                            // this step's place among the packed weights (a class of several
+                            // takes whole taps of a multiple of 16 channels)
+                            int kw = kc * kChunkK + j * 16;
+                            if(kw >= kTotal)
+                                break;
+                            if(step > 1)
+                            {
+                                const int t = kw / p.Cg, tr = t / ntx;
+                                kw += ((ty0 + step * tr) * p.ks + tx0 + step * (t - tr * ntx) - t) * p.Cg;
+                            }
                             const uint64_t ad = tc::smem_desc(stage + uint32_t(j) * 256u, 128u, 1024u);
-                            const uint64_t bd = tc::smem_desc(sB + uint32_t(kc * 8 + 2 * j) * 128u, 128u, sboB);
+                            const uint64_t bd = tc::smem_desc(sB + uint32_t(kw / 8) * 128u, 128u, sboB);
                             tc::mma_bf16(tmem, ad, bd, idesc, (kc | j) != 0 ? 1u : 0u);
                         }
                         tc::mma_commit(&sEmpty[G % kStages]);
@@ -273,9 +320,12 @@ namespace isaacb
                     const int cpw = p.Npad / 2;
                     for(int c0 = half * cpw; c0 < (half + 1) * cpw; c0 += 8)
                     {
-                        float v[8];
-                        tc::tmem_ld8(tmem + (lane0 << 16) + uint32_t(c0), v);
-                        tc::tmem_wait_ld();
+                        float v[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+                        if(nk > 0) // a class without a tap has no accumulator
+                        {
+                            tc::tmem_ld8(tmem + (lane0 << 16) + uint32_t(c0), v);
+                            tc::tmem_wait_ld();
+                        }
                         if(!valid || c0 >= p.Cout)
                             continue;
                         const size_t o = size_t(pix) * p.Cout + c0;
@@ -883,56 +933,60 @@ namespace isaacb
             const int nk = c1 - c0;
             const int mTile = blockIdx.x;
             const uint32_t idesc = tc::idesc_bf16(kTileM, p.Npad, true, true);
-            const int bPieces = (p.Npad / 8) * kChunkK;
 
-            auto load_chunk = [&](int kc, uint32_t G) {
+            // A thread copies, for pixel px of every chunk, the row blocks (8 channels of one
+            // tap) mb0 + 4 q and the column blocks mb0 + 4 i of dY.  The chunks are taken in
+            // order, so the pixel's place in the image and the blocks' taps need no division
+            // inside the loop.
+            const int px = tid & (kChunkK - 1), mb0 = tid >> 6;
+            int ty[4], tx[4], tc0[4];
+#pragma unroll
+            for(int q = 0; q < 4; ++q)
+            {
+                const int r0 = mTile * kTileM + (mb0 + 4 * q) * 8;
+                const int t = r0 / p.Cin;
+                ty[q] = t / p.ks - p.pad;
+                tx[q] = t % p.ks - p.pad;
+                tc0[q] = r0 < p.Mtot ? r0 - t * p.Cin : -1;
+            }
+            int pix = c0 * kChunkK + px;
+            int ox = pix % p.Wo, oy = (pix / p.Wo) % p.Ho, b = pix / p.Wo / p.Ho;
+            auto load_chunk = [&](uint32_t G) {
                 const uint32_t stA = s0 + (G % kStages) * stageBytes;
                 const uint32_t stB = stA + uint32_t(kStageBytesA);
-                // A: 16 row blocks (8 channels of one tap) x 64 pixels
+                const uint32_t at = uint32_t(px >> 3) * 128u + uint32_t(px & 7) * 16u;
 #pragma unroll
                 for(int q = 0; q < 4; ++q)
                 {
-                    const int id = q * kThreads + tid;
-                    const int px = id & (kChunkK - 1), mb = id >> 6;
-                    const int r0 = mTile * kTileM + mb * 8;
-                    const int pix = kc * kChunkK + px;
-                    const bf16* src = p.x;
-                    uint32_t bytes = 0;
-                    if(r0 < p.Mtot && pix < P)
-                    {
-                        const int t = r0 / p.Cin, c = r0 - t * p.Cin;
-                        const int ty = t / p.ks, tx = t - ty * p.ks;
-                        const int ox = pix % p.Wo, tt = pix / p.Wo;
-                        const int oy = tt % p.Ho, b = tt / p.Ho;
-                        const int iy = oy * p.stride - p.pad + ty, ix = ox * p.stride - p.pad + tx;
-                        if(iy >= 0 && ix >= 0 && iy < p.H && ix < p.W)
-                        {
-                            src = p.x + ((size_t(b) * p.H + iy) * p.W + ix) * p.Cin + c;
-                            bytes = 16;
-                        }
-                    }
-                    tc::cp_async16(stA + uint32_t(mb) * 1024u + uint32_t(px >> 3) * 128u + uint32_t(px & 7) * 16u, src, bytes);
+                    const int iy = oy * p.stride + ty[q], ix = ox * p.stride + tx[q];
+                    const bool ok = tc0[q] >= 0 && pix < P && iy >= 0 && ix >= 0 && iy < p.H && ix < p.W;
+                    const bf16* src = ok ? p.x + ((size_t(b) * p.H + iy) * p.W + ix) * p.Cin + tc0[q] : p.x;
+                    tc::cp_async16(stA + uint32_t(mb0 + 4 * q) * 1024u + at, src, ok ? 16u : 0u);
                 }
                 // B: Npad/8 column blocks x 64 pixels of dY
-                for(int id = tid; id < bPieces; id += kThreads)
+                for(int nb = mb0; nb < p.Npad / 8; nb += 4)
                 {
-                    const int px = id & (kChunkK - 1), nb = id >> 6;
-                    const int pix = kc * kChunkK + px;
-                    const bf16* src = p.dy;
-                    uint32_t bytes = 0;
-                    if(pix < P && nb * 8 < p.Cout)
+                    const bool ok = pix < P && nb * 8 < p.Cout;
+                    const bf16* src = ok ? p.dy + size_t(pix) * p.Cout + nb * 8 : p.dy;
+                    tc::cp_async16(stB + uint32_t(nb) * 1024u + at, src, ok ? 16u : 0u);
+                }
+                pix += kChunkK;
+                ox += kChunkK;
+                while(ox >= p.Wo)
+                {
+                    ox -= p.Wo;
+                    if(++oy == p.Ho)
                     {
-                        src = p.dy + size_t(pix) * p.Cout + nb * 8;
-                        bytes = 16;
+                        oy = 0;
+                        ++b;
                     }
-                    tc::cp_async16(stB + uint32_t(nb) * 1024u + uint32_t(px >> 3) * 128u + uint32_t(px & 7) * 16u, src, bytes);
                 }
             };
 
             for(int c = 0; c < kStages - 1; ++c)
             {
                 if(c < nk)
-                    load_chunk(c0 + c, uint32_t(c));
+                    load_chunk(uint32_t(c));
                 tc::cp_async_commit();
             }
             for(int kc = 0; kc < nk; ++kc)
@@ -943,7 +997,7 @@ namespace isaacb
                     const uint32_t G = uint32_t(kn);
                     if(G >= kStages && !tc::mbar_wait(&sEmpty[G % kStages], ((G / kStages) - 1) & 1))
                         raise_error(p.errorFlag, abortLocal);
-                    load_chunk(c0 + kn, G);
+                    load_chunk(G);
                 }
                 tc::cp_async_commit();
                 tc::cp_async_wait<kStages - 1>();
@@ -989,6 +1043,7 @@ namespace isaacb
                 const int half = warp >> 2;
                 const int cpw = p.Npad / 2;
                 const int row = mTile * kTileM + (tid & (kTileM - 1));
+                const bool vec4 = (reinterpret_cast<uintptr_t>(p.dw) & 15u) == 0; // rows are multiples of 16 floats
                 for(int cc = half * cpw; cc < (half + 1) * cpw; cc += 8)
                 {
                     float v[8];
@@ -996,10 +1051,18 @@ namespace isaacb
                     tc::tmem_wait_ld();
                     if(row >= p.Mtot)
                         continue;
+                    if(cc >= p.Cout) // channel counts are multiples of 8
+                        continue;
+                    float* dst = p.dw + size_t(row) * p.Npad + cc;
+                    if(vec4)
+                    {
+                        atomicAdd(reinterpret_cast<float4*>(dst), make_float4(v[0], v[1], v[2], v[3]));
+                        atomicAdd(reinterpret_cast<float4*>(dst) + 1, make_float4(v[4], v[5], v[6], v[7]));
+                    }
+                    else
 #pragma unroll
-                    for(int i = 0; i < 8; ++i)
-                        if(cc + i < p.Cout)
-                            atomicAdd(p.dw + size_t(row) * p.Npad + cc + i, v[i]);
+                        for(int i = 0; i < 8; ++i)
+                            atomicAdd(dst + i, v[i]);
                 }
             }
             tc::fence_before_sync();
@@ -1212,7 +1275,7 @@ namespace isaacb
     } // namespace
 
     bool g_rowTma = true; // the TMA producer where the input allows it
-    bool launch_conv_gemm(const ConvGemmParams& p, cudaStream_t s)
+    bool launch_conv_gemm(ConvGemmParams p, cudaStream_t s)
     {
         if(row_tiles_apply(p))
         {
@@ -1239,8 +1302,16 @@ namespace isaacb
             return false;
         cudaFuncSetAttribute(k_conv_gemm, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
         cudaFuncSetAttribute(k_conv_gemm, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-        const int P = p.B * p.Ho * p.Wo;
-        const int tiles = (P + kTileM - 1) / kTileM;
+        // output pixels by residue class: whole taps of 16-channel steps only, so that an MMA
+        // step never crosses from one tap to the next of its class
+        p.step = p.transposed && p.Cg % 16 == 0 ? p.stride : 1;
+        p.tiles = 0;
+        for(int c = 0; c < p.step * p.step; ++c)
+        {
+            const int hc = (p.Ho - c / p.step + p.step - 1) / p.step, wc = (p.Wo - c % p.step + p.step - 1) / p.step;
+            p.tiles += (p.B * hc * wc + kTileM - 1) / kTileM;
+        }
+        const int tiles = p.tiles;
         // as many persistent CTAs as fit on an SM (shared memory and TMEM permitting), so one
         // CTA's epilogue and gathers overlap another's MMAs
         int perSm = ctas_per_sm(k_conv_gemm, kThreads, smem);

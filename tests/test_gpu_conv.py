@@ -137,3 +137,33 @@ def test_tma_and_cp_async_producers_agree(case):
         _lib.check(lib.isaacb_conv_set_producer(1))
     assert torch.equal(outs[0][0], outs[1][0])
     assert torch.equal(outs[0][1], outs[1][1])
+
+
+@pytest.mark.parametrize("case", [
+    # B, H, W, Ci, Co, ks, s, pad: the input gradient's residue classes (y mod s, x mod s)
+    (1, 9, 7, 8, 16, 2, 3, 0),  # fewer taps than classes: some have none
+    (2, 8, 9, 16, 24, 3, 2, 1),  # channels not a multiple of 16: one class of all taps
+    (1, 6, 5, 16, 48, 5, 4, 2),  # classes of 1, 2 and 4 taps; fewer pixels than a tile
+    (2, 33, 47, 32, 96, 3, 2, 0),  # tap boundaries inside 64-wide chunks
+    (1, 61, 64, 32, 16, 7, 2, 3),
+])
+def test_dgrad_residue_classes_and_unaligned_dw(case):
+    """Strided input gradients walk each residue class's own taps; a weight gradient that
+    starts off a 16-byte boundary takes scalar atomics."""
+    B, H, W, Ci, Co, ks, s, pad = case
+    rng = np.random.default_rng(11)
+    Ho, Wo = R.out_size(H, ks, s, pad), R.out_size(W, ks, s, pad)
+    x = R.round_bf16(rng.standard_normal((B, H, W, Ci)).astype(np.float32))
+    w = R.round_bf16((rng.standard_normal((Co, ks, ks, Ci)) / np.sqrt(ks * ks * Ci)).astype(np.float32))
+    dy = R.round_bf16(rng.standard_normal((B, Ho, Wo, Co)).astype(np.float32))
+    xd, dyd, wt = _bf16(x), _bf16(dy), _bf16(R.pack_weights_transposed(w))
+    dx = torch.full((B, H, W, Ci), 7.0, dtype=torch.float32, device="cuda")
+    _run("isaacb_conv_forward", x=dyd.data_ptr(), w=wt.data_ptr(), y_f32=dx.data_ptr(), batch=B, in_h=Ho, in_w=Wo,
+         c_in=Co, out_h=H, out_w=W, c_out=Ci, ksize=ks, stride=s, pad=pad, transposed=1)
+    _close(dx.cpu().numpy(), R.conv_dgrad(dy, w, (H, W), s, pad), 2e-3, "dgrad")
+    npad = (Co + 15) // 16 * 16
+    buf = torch.zeros(ks * ks * Ci * npad + 1, dtype=torch.float32, device="cuda")
+    _run("isaacb_conv_wgrad", x=xd.data_ptr(), dy=dyd.data_ptr(), dw=buf.data_ptr() + 4, batch=B, in_h=H, in_w=W, c_in=Ci,
+         out_h=Ho, out_w=Wo, c_out=Co, ksize=ks, stride=s, pad=pad)
+    got = buf.cpu().numpy()[1:].reshape(ks * ks * Ci, npad)[:, :Co]
+    _close(got, np.transpose(R.conv_wgrad(x, dy, ks, s, pad), (1, 2, 3, 0)).reshape(ks * ks * Ci, Co), 2e-3, "wgrad")
