@@ -307,7 +307,6 @@ struct isaacb_ctx
     double proj[16]{}, mv[16]{};
     bool cameraSet = false;
     const float* src[kMaxSources]{};
-    float* compact[kMaxSources]{}; // compact interior copies of guarded sources
     ParticleSrc part[kMaxSources]{};
     bool partSet[kMaxSources]{};
     bool counting = false;
@@ -332,7 +331,8 @@ struct isaacb_ctx
     float* ao = nullptr;
     unsigned long long* counters = nullptr;
     float* mmPartial = nullptr;
-    float* mmResult = nullptr;
+    float* mmResult = nullptr; // min and max of each source
+    unsigned int* mmTicket = nullptr;
     unsigned long long* mmKeys = nullptr;
     int32_t* errorFlag = nullptr;
     // count of all-zero bricks of the last merge (device memory); the march reads it and
@@ -607,31 +607,17 @@ namespace
         return ISAACB_OK;
     }
 
-    // A source with guard cells is read through a compact copy of its interior: the
-    // combined renderer and min/max read only the interior (MergeToCombinedTextureKernel
-    // and MinMaxKernel iterate over the local size, lib/isaac/isaac_common_kernel.hpp:
-    // 716-719, lib/isaac/isaac_min_max_kernel.hpp:35-38), which is what every kernel
-    // here indexes.
-    const float* source_data(const isaacb_ctx* c, int s)
+    // A source's interior, the only part the combined renderer and min/max read
+    // (MergeToCombinedTextureKernel and MinMaxKernel iterate over the local size,
+    // lib/isaac/isaac_common_kernel.hpp:716-719, lib/isaac/isaac_min_max_kernel.hpp:35-38):
+    // its first voxel and the row and plane pitches in voxels, ghost cells included.  The
+    // kernels read guarded sources in place.
+    const float* source_interior(const isaacb_ctx* c, int s, size_t& pitchY, size_t& pitchZ)
     {
-        return c->desc.guard_size[s] != 0 ? c->compact[s] : c->src[s];
-    }
-    isaacb_status compact_guarded(isaacb_ctx* c, cudaStream_t st)
-    {
-        for(int s = 0; s < c->nVol; ++s)
-        {
-            const int g = int(c->desc.guard_size[s]);
-            if(g == 0 || !c->src[s])
-                continue;
-            const int fd = int(c->desc.feature_dim[s]);
-            if(!c->compact[s])
-                ISAACB_CUDA(c, cudaMalloc(&c->compact[s], size_t(c->g.ls[0]) * c->g.ls[1] * c->g.ls[2] * fd * sizeof(float)),
-                            "compact source allocation");
-            launch_compact_guarded(c->src[s], c->compact[s], c->g.ls[0], c->g.ls[1], c->g.ls[2], g, fd, st);
-            ISAACB_CUDA(c, cudaGetLastError(), "compact guarded source");
-            c->updateLaunches++;
-        }
-        return ISAACB_OK;
+        const size_t g = c->desc.guard_size[s];
+        pitchY = size_t(c->g.ls[0]) + 2 * g;
+        pitchZ = pitchY * (size_t(c->g.ls[1]) + 2 * g);
+        return c->src[s] ? c->src[s] + (g * pitchZ + g * pitchY + g) * c->desc.feature_dim[s] : nullptr;
     }
 
     // Slot order of the combined textures for the camera of the merge about to run
@@ -674,7 +660,7 @@ namespace
         p.totalWeight = 0.0f;
         for(int s = 0; s < c->nVol; ++s)
         {
-            p.src[s] = source_data(c, s);
+            p.src[s] = source_interior(c, s, p.pitchY[s], p.pitchZ[s]);
             p.fdim[s] = int32_t(c->desc.feature_dim[s]);
             p.chain[s] = c->chain[s];
             p.chainIdem[s] = (c->chain[s].op[0] == OP_IDEM && c->chain[s].op[1] == OP_IDEM && c->chain[s].op[2] == OP_IDEM) ? 1 : 0;
@@ -834,13 +820,16 @@ extern "C"
         alloc((void**) &c->normal, npix * 3 * sizeof(float));
         alloc((void**) &c->ao, npix * sizeof(float));
         alloc((void**) &c->counters, 2 * sizeof(unsigned long long));
-        alloc((void**) &c->mmPartial, 2 * 148 * 8 * sizeof(float));
-        alloc((void**) &c->mmResult, 2 * sizeof(float));
+        alloc((void**) &c->mmPartial, 2 * kMinMaxBlocks * sizeof(float));
+        alloc((void**) &c->mmResult, 2 * kMaxSources * sizeof(float));
+        alloc((void**) &c->mmTicket, sizeof(unsigned int));
         alloc((void**) &c->mmKeys, 2 * sizeof(unsigned long long));
         alloc((void**) &c->errorFlag, sizeof(int32_t));
         alloc((void**) &c->emptyDev, sizeof(unsigned int));
         if(e == cudaSuccess)
             e = cudaMemset(c->emptyDev, 0, sizeof(unsigned int));
+        if(e == cudaSuccess)
+            e = cudaMemset(c->mmTicket, 0, sizeof(unsigned int));
         if(e == cudaSuccess)
             e = cudaMemset(c->errorFlag, 0, sizeof(int32_t));
         if(e == cudaSuccess)
@@ -864,8 +853,6 @@ extern "C"
     {
         if(!c)
             return ISAACB_OK;
-        for(float* q : c->compact)
-            cudaFree(q);
         cudaFree(c->lutDev);
         cudaFree(c->lutPre);
         cudaFree(c->psPre);
@@ -888,6 +875,7 @@ extern "C"
         cudaFree(c->counters);
         cudaFree(c->mmPartial);
         cudaFree(c->mmResult);
+        cudaFree(c->mmTicket);
         cudaFree(c->mmKeys);
         cudaFree(c->errorFlag);
         for(int s = 0; s < kMaxSources; ++s)
@@ -1286,9 +1274,6 @@ extern "C"
         c->updateLaunches = 0;
         if(c->renderer == ISAACB_RENDERER_COMBINED)
         {
-            r = compact_guarded(c, st);
-            if(r != ISAACB_OK)
-                return r;
             if(!c->advectedThisFrame)
             {
                 r = advect_fields(c, st);
@@ -1299,7 +1284,6 @@ extern "C"
             c->g.yfast = slot_order_for_camera(c);
             MergeParams p{};
             prepare_merge(c, p);
-            ISAACB_CUDA(c, cudaMemsetAsync(c->emptyDev, 0, sizeof(unsigned int), st), "empty brick counter");
             {
                 for(int k = 0; k < ISAACB_TIMING_SLOTS; ++k)
                     c->evUsed[k] = false;
@@ -1536,56 +1520,56 @@ extern "C"
         if(!c || !mn || !mx)
             return fail(c, ISAACB_INVALID_ARG, "isaacb_minmax: null argument");
         cudaStream_t st = (cudaStream_t) stream;
-        {
-            const isaacb_status r = compact_guarded(c, st);
-            if(r != ISAACB_OK)
-                return r;
-        }
         for(int s = 0; s < c->nTotal; ++s)
-        {
+            if(s < c->nVol ? !c->src[s] : !c->partSet[s - c->nVol])
+                return fail(c, ISAACB_NOT_READY, s < c->nVol ? "isaacb_minmax: source without memory"
+                                                             : "isaacb_minmax: particle source without memory");
+        auto params = [&](int s) {
             MinMaxParams p{};
             p.g = c->g;
             p.chain = c->chain[s];
             p.fdim = int32_t(c->desc.feature_dim[s]);
             p.partial = c->mmPartial;
+            p.ticket = c->mmTicket;
+            p.result = c->mmResult + 2 * s;
             p.keys = c->mmKeys;
             if(s < c->nVol)
-            {
-                if(!c->src[s])
-                    return fail(c, ISAACB_NOT_READY, "isaacb_minmax: source without memory");
-                p.src = source_data(c, s);
-                p.particle = 0;
-            }
+                p.src = source_interior(c, s, p.pitchY, p.pitchZ);
             else
             {
                 const ParticleSrc& P = c->part[s - c->nVol];
-                if(!c->partSet[s - c->nVol])
-                    return fail(c, ISAACB_NOT_READY, "isaacb_minmax: particle source without memory");
                 p.offsets = P.offsets;
                 p.attr = P.attr;
                 p.particle = 1;
             }
-            launch_minmax(p, minmax_blocks(p), c->mmResult, st);
-            float res[2];
-            ISAACB_CUDA(c, cudaMemcpyAsync(res, c->mmResult, sizeof(res), cudaMemcpyDeviceToHost, st), "minmax read");
-            ISAACB_CUDA(c, cudaStreamSynchronize(st), "minmax");
-            if(res[0] == 0.0f || res[1] == 0.0f)
+            return p;
+        };
+        // every source's reduction, then one read of all results
+        for(int s = 0; s < c->nTotal; ++s)
+            launch_minmax(params(s), st);
+        float res[2 * kMaxSources];
+        ISAACB_CUDA(c, cudaMemcpyAsync(res, c->mmResult, 2 * c->nTotal * sizeof(float), cudaMemcpyDeviceToHost, st), "minmax read");
+        ISAACB_CUDA(c, cudaStreamSynchronize(st), "minmax");
+        for(int s = 0; s < c->nTotal; ++s)
+        {
+            float* r = res + 2 * s;
+            if(r[0] == 0.0f || r[1] == 0.0f)
             {
                 // +0 and -0 compare equal: the reference keeps the first in its scan order
                 const unsigned long long init[2] = {ULLONG_MAX, ULLONG_MAX};
                 ISAACB_CUDA(c, cudaMemcpyAsync(c->mmKeys, init, sizeof(init), cudaMemcpyHostToDevice, st), "keys");
-                launch_minmax_zero_keys(p, st);
+                launch_minmax_zero_keys(params(s), st);
                 unsigned long long keys[2];
                 ISAACB_CUDA(c, cudaMemcpyAsync(keys, c->mmKeys, sizeof(keys), cudaMemcpyDeviceToHost, st), "keys");
                 ISAACB_CUDA(c, cudaStreamSynchronize(st), "minmax zero order");
                 const float firstZero = keys[1] < keys[0] ? -0.0f : 0.0f;
-                if(res[0] == 0.0f)
-                    res[0] = firstZero;
-                if(res[1] == 0.0f)
-                    res[1] = firstZero;
+                if(r[0] == 0.0f)
+                    r[0] = firstZero;
+                if(r[1] == 0.0f)
+                    r[1] = firstZero;
             }
-            mn[s] = res[0];
-            mx[s] = res[1];
+            mn[s] = r[0];
+            mx[s] = r[1];
         }
         ISAACB_CUDA(c, cudaGetLastError(), "isaacb_minmax");
         return ISAACB_OK;
@@ -1841,14 +1825,10 @@ namespace
                 for(int s = 0; s < c->nVol; ++s)
                     if(!c->src[s] && (c->weight[s] != 0.0f || c->iso[s] != 0.0f))
                         return batch_fail(ISAACB_NOT_READY, "isaacb_batch: a source has no memory");
-                if(compact_guarded(c, st) != ISAACB_OK)
-                    return batch_fail(ISAACB_CUDA_ERROR, std::string("isaacb_batch: ") + c->lastError);
                 MergeParams p{};
                 prepare_merge(c, p);
                 if(capture)
                     b->graphMerges.push_back(p);
-                if(cudaMemsetAsync(c->emptyDev, 0, sizeof(unsigned int), st) != cudaSuccess)
-                    return batch_fail(ISAACB_CUDA_ERROR, "isaacb_batch: empty brick counter");
                 b->launches += uint32_t(launch_merge(p, st));
             }
         }

@@ -230,6 +230,81 @@ namespace isaacb
         return v[0];
     }
 
+    // A chain without pow and with at most one reduction (length or sum), as multiply-adds:
+    // functor k is v * m[k] + a[k] with (p, -0) for mul, (1, p) for add and (1, -0) for idem,
+    // which round like the functor alone (x + -0 is x for every x).  reduce: 0 none, 1 length,
+    // 2 sum, in place of functor `at`.
+    struct LineChain
+    {
+        int32_t reduce, at, idem; // idem: nothing to do
+        float m[kMaxFunctors][4], a[kMaxFunctors][4];
+    };
+    inline bool line_chain_of(const Chain& ch, LineChain& L)
+    {
+        L = LineChain{};
+        L.at = kMaxFunctors;
+        L.idem = 1;
+        for(int k = 0; k < kMaxFunctors; ++k)
+        {
+            const int op = ch.op[k];
+            if(op == OP_POW || ((op == OP_LENGTH || op == OP_SUM) && L.reduce))
+                return false;
+            if(op == OP_LENGTH || op == OP_SUM)
+            {
+                L.reduce = op == OP_LENGTH ? 1 : 2;
+                L.at = k;
+            }
+            if(op != OP_IDEM)
+                L.idem = 0;
+            for(int i = 0; i < 4; ++i)
+            {
+                L.m[k][i] = op == OP_MUL ? ch.p[4 * k + i] : 1.0f;
+                L.a[k][i] = op == OP_ADD ? ch.p[4 * k + i] : -0.0f;
+            }
+        }
+        return true;
+    }
+    // the chain's value of V voxels into v[j][0]; FD components are loaded (1: no source
+    // with more takes a reduction)
+    template<int V, int FD>
+    __device__ __forceinline__ void line_chain(float (&v)[V][FD], int dim, const LineChain& L)
+    {
+        if(L.idem)
+            return;
+#pragma unroll
+        for(int k = 0; k < kMaxFunctors; ++k)
+        {
+            if(k < L.at)
+            {
+                // before a reduction every component, else only the first matters
+#pragma unroll
+                for(int c = 0; c < FD; ++c)
+                    if(c == 0 || (L.reduce && c < dim))
+#pragma unroll
+                        for(int j = 0; j < V; ++j)
+                            v[j][c] = fmaf(v[j][c], L.m[k][c], L.a[k][c]);
+            }
+            else if(k == L.at)
+            {
+                // components past the source's are +0 here and add nothing to either
+#pragma unroll
+                for(int j = 0; j < V; ++j)
+                {
+                    float w[4];
+#pragma unroll
+                    for(int c = 0; c < 4; ++c)
+                        w[c] = c < FD ? v[j][c < FD ? c : 0] : 0.0f;
+                    v[j][0] = L.reduce == 1 ? sqrtf((w[0] * w[0] + w[1] * w[1]) + (w[2] * w[2] + w[3] * w[3]))
+                                            : (((0.0f + w[0]) + w[1]) + w[2]) + w[3];
+                }
+            }
+            else
+#pragma unroll
+                for(int j = 0; j < V; ++j)
+                    v[j][0] = fmaf(v[j][0], L.m[k][0], L.a[k][0]);
+        }
+    }
+
     // transfer-function index round(v*TS) clamped to [0,TS-1], NaN -> 0
     // (lib/isaac/isaac_common_kernel.hpp:589-591)
     __device__ __forceinline__ int lut_index(float v, int ts)

@@ -19,7 +19,8 @@ namespace isaacb
         int32_t ts;
         int32_t ditherMode;
         int32_t writeIso;
-        const float* src[kMaxSources];
+        const float* src[kMaxSources]; // voxel (0, 0, 0) of the interior
+        size_t pitchY[kMaxSources], pitchZ[kMaxSources]; // voxels from a row / plane to the next, ghost cells included
         int32_t fdim[kMaxSources];
         Chain chain[kMaxSources];
         int32_t chainIdem[kMaxSources]; // 1: every functor is idem, the value is the x component
@@ -38,7 +39,7 @@ namespace isaacb
         uint32_t* isoLin; // combined iso RGBA8, linear
         uint8_t* volFlag; // per brick: 1 if any texel (apron included) is non-zero
         uint8_t* isoFlag; // per brick: max alpha byte (apron included)
-        unsigned int* emptyBricks; // count of all-zero bricks (zeroed by the host before the merge)
+        unsigned int* emptyBricks; // count of all-zero bricks (pass 1 zeroes it, pass 2 counts)
     };
     // CTAs of `kernel` that fit on one SM with `threads` threads and `dynSmem` bytes of
     // dynamic shared memory (registers, threads, shared memory; at most 4)
@@ -116,10 +117,6 @@ namespace isaacb
         void* out; // slots of ncomp*4 elements, component major
     };
     void launch_source_bricks(const SourceBrickParams& p, cudaStream_t s);
-    // interior of a source with `guard` cells per side ((X+2g)(Y+2g)(Z+2g) voxels, x fastest)
-    // into a compact X*Y*Z copy, fdim floats per voxel
-    void launch_compact_guarded(const float* src, float* dst, int X, int Y, int Z, int guard, int fdim, cudaStream_t s);
-
     // quad bricks -> linear RGBA8 (diagnostics)
     void launch_unbrick(const Geom& g, const uint4* volQ, uint32_t* out, cudaStream_t s);
 
@@ -127,18 +124,21 @@ namespace isaacb
     struct MinMaxParams
     {
         Geom g;
-        const float* src;
+        const float* src; // voxel (0, 0, 0) of the interior
+        size_t pitchY, pitchZ; // voxels from a row / plane to the next, ghost cells included
         int32_t fdim;
         Chain chain;
         // particles
         const uint32_t* offsets;
         const float* attr;
         int32_t particle;
-        float* partial; // 2 floats per block
-        unsigned long long* keys; // 4 keys: first +0 / -0 for min and max
+        float* partial; // 2 floats per block, kMinMaxBlocks blocks at most
+        unsigned int* ticket; // zero between launches
+        float* result; // min, max
+        unsigned long long* keys; // 2 keys: first +0, first -0
     };
-    int minmax_blocks(const MinMaxParams& p);
-    void launch_minmax(const MinMaxParams& p, int blocks, float* result, cudaStream_t s);
+    constexpr size_t kMinMaxBlocks = 148 * 8;
+    void launch_minmax(const MinMaxParams& p, cudaStream_t s);
     void launch_minmax_zero_keys(const MinMaxParams& p, cudaStream_t s);
 
     // -------------------------------------------------------------- frame

@@ -197,49 +197,20 @@ namespace isaacb
         }
     }
 
-    // NS (1..4) scalar sources whose chains are all idem, none advected: the sources'
-    // pointers, tables and weights live in registers and all values load up front
-    template<bool ISO, int NS>
-    __global__ void __launch_bounds__(256) k_merge_voxels_n(const __grid_constant__ MergeParams p, const __grid_constant__ MergeActive act)
-    {
-        __shared__ uint8_t sMask[64];
-        if(threadIdx.x < 64)
-            sMask[threadIdx.x] = p.ditherMode == 2 ? c_dither2[threadIdx.x] : c_dither1[threadIdx.x];
-        __syncthreads();
-        const Geom& g = p.g;
-        const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y, z = blockIdx.z;
-        if(x >= g.ls[0])
-            return;
-        const size_t i = (size_t(z) * g.ls[1] + y) * g.ls[0] + x;
-        float val[NS];
-#pragma unroll
-        for(int k = 0; k < NS; ++k)
-            val[k] = __ldg(act.src[k] + i);
-        float4 vc = make_float4(0, 0, 0, 0), ic = make_float4(0, 0, 0, 0);
-#pragma unroll
-        for(int k = 0; k < NS; ++k)
-            merge_accumulate(__ldg(act.lut[k] + lut_index_fast(val[k], p.ts)), act.weight[k], act.iso[k], ISO, vc, ic);
-        merge_store<ISO>(p, sMask, i, x, y, z, vc, ic);
-    }
-
     // the largest float below 1: a threshold of exactly 1 behaves as this one below
     constexpr float kDitherMax = 0x1.fffffep-1f;
 
     // the non-negative dither with threshold d (already capped at kDitherMax):
     // floor(s) + (fract(s) > d) == ceil(s - d) for 0 <= d < 1 and s >= 0, and the
-    // round-up subtraction keeps the ceiling exact; ceil by an exact magic-number add
+    // round-up subtraction keeps the ceiling exact; ceil by an exact magic-number add.  s is
+    // cut at 255, where ceil(255 - d) is 255 as for every larger s, so the low byte of the
+    // sum's bits is the result.
     __device__ __forceinline__ uint32_t dither_rgba_ceil(float4 c, float d)
     {
-        const float v[4] = {c.x, c.y, c.z, c.w};
-        uint32_t out = 0;
-#pragma unroll
-        for(int i = 0; i < 4; ++i)
-        {
-            const float s = fminf(v[i] * 255.0f, 257.0f);
-            const float t = __fadd_ru(__fsub_ru(s, d), 12582912.0f);
-            out |= uint32_t(min(__float_as_int(t) - 0x4B400000, 255)) << (8 * i);
-        }
-        return out;
+        auto bits = [&](float v) {
+            return __float_as_uint(__fadd_ru(__fsub_ru(fminf(v * 255.0f, 255.0f), d), 12582912.0f));
+        };
+        return __byte_perm(__byte_perm(bits(c.x), bits(c.y), 0x0040u), __byte_perm(bits(c.z), bits(c.w), 0x0040u), 0x5410u);
     }
 
     // Four x-adjacent voxels (the quad q of rows of rowQuads) of the scalar merge: one
@@ -306,9 +277,10 @@ namespace isaacb
             reinterpret_cast<uint4*>(p.isoLin)[q] = make_uint4(io[0], io[1], io[2], io[3]);
     }
 
-    // As k_merge_voxels_n, four x-adjacent voxels per thread (rows a multiple of 4 voxels,
-    // 16-byte aligned sources, fewer than 2^32 groups of four); table entries from global
-    // memory through a pointer biased so that the floor's bits address them
+    // Scalar sources whose chains are all idem, none advected, four x-adjacent voxels per
+    // thread (rows a multiple of 4 voxels, 16-byte aligned sources, fewer than 2^32 groups of
+    // four); table entries from global memory through a pointer biased so that the floor's
+    // bits address them
     template<bool ISO, int NS>
     __global__ void __launch_bounds__(256) k_merge_voxels_x4(const __grid_constant__ MergeParams p, const __grid_constant__ MergeActive act)
     {
@@ -318,6 +290,8 @@ namespace isaacb
         __syncthreads();
         const uint32_t rowQuads = uint32_t(p.g.ls[0]) >> 2;
         const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;
+        if(q == 0)
+            *p.emptyBricks = 0u; // pass 2 counts
         if(q >= rowQuads * uint32_t(p.g.ls[1]) * uint32_t(p.g.ls[2]))
             return;
         merge_quad<ISO, NS>(p, act, sMask, q, rowQuads, [&](int k, uint32_t bits) {
@@ -337,6 +311,8 @@ namespace isaacb
         __shared__ __align__(4) uint8_t sMask[64];
         if(threadIdx.x < 64)
             sMask[threadIdx.x] = p.ditherMode == 2 ? c_dither2[threadIdx.x] : c_dither1[threadIdx.x];
+        if(blockIdx.x == 0 && threadIdx.x == 0)
+            *p.emptyBricks = 0u; // pass 2 counts
         const int ts = p.ts;
         for(int i = threadIdx.x; i < NS * ts; i += blockDim.x)
             sLut[i] = __ldg(p.lutPre + i);
@@ -349,6 +325,349 @@ namespace isaacb
             });
     }
 
+    // ---------------------------------------------------------------- merge, pass 1: any sources
+    // Up to 4 active sources of any kind but a pow chain: functor chains, vector and field
+    // sources, ghost cells, rows of any length, iso output.  Persistent 512-thread CTAs keep
+    // every table that the sources need in shared memory, formed once per CTA: the weighted
+    // premultiplied entry (c.rgb a, a), a = c.w * weight; for an iso source c.w / iso * 0.5
+    // and the entry's texel; for an advected source the entry itself, its alpha changing per
+    // voxel.  A thread evaluates kRowsPer voxels 32 apart, all their loads issued first.  The
+    // kernel is bound by instructions, so that every functor is one multiply-add (LineChain)
+    // and no voxel divides: the iso threshold, 64 and 255 are in tables, the total weight is
+    // a reciprocal with exact corrections.
+    // One voxel a thread, tables in global memory and a division per channel took 424 us on
+    // the full-feature scene (256^3, 5 floats a voxel, iso output) and 250 us on a scalar
+    // with an advected vector field; this form takes 193 and 137 (one voxel a thread at three
+    // CTAs per SM 221 and 161, four a thread 290 and 138).
+        constexpr int kRowsThreads = 512, kRowsPer = 2, kRowsMaxSources = 4;
+    // tables of one CTA, so that two fit on an SM (6 tables of 1024 entries)
+    constexpr size_t kRowsSmem = 96 * 1024;
+
+    struct FastDiv
+    {
+        uint32_t d, m, s; // n / d == umulhi(n, m) >> s for n < 2^31 (d > 1)
+        __device__ __forceinline__ uint32_t operator()(uint32_t n) const
+        {
+            return d == 1u ? n : __umulhi(n, m) >> s;
+        }
+    };
+    FastDiv fast_div(uint32_t d)
+    {
+        FastDiv f{d, 0u, 0u};
+        if(d > 1u)
+        {
+            uint32_t l = 1;
+            while((uint64_t(1) << l) < d)
+                ++l;
+            f.m = uint32_t((uint64_t(1) << (31 + l)) / d + 1);
+            f.s = l - 1;
+        }
+        return f;
+    }
+
+    struct MergeRows
+    {
+        int n, volTables, isoTables;
+        uint32_t voxels;
+        FastDiv rowOf, planeOf; // voxel index -> row, row -> plane
+        float rcpTotal; // 1 / totalWeight, rounded
+        uint32_t advRow, advPlane; // the advection textures' pitches, guard band included
+        struct Source
+        {
+            const float* base; // interior voxel (0, 0, 0)
+            uint32_t pitchY, pitchZ; // voxels
+            int32_t fdim;
+            LineChain chain;
+            float weight, iso;
+            int32_t volTable, isoTable; // -1: none
+            const uint8_t* adv; // advection texture at voxel (0, 0, 0), null: none
+        } src[kRowsMaxSources];
+        struct Table
+        {
+            const float4* lut;
+            float scale; // weight (0: entries as they are) or iso threshold
+        } vol[kRowsMaxSources], iso[kRowsMaxSources];
+    };
+
+    // x / d for d in [kDivMin, kDivMax], r = 1 / d rounded and x = 0 or >= kDivTiny: the
+    // product and two exact-residual corrections.  The first leaves less than an ulp of
+    // error, the second rounds correctly (Markstein's division); from kDivTiny on no
+    // residual loses bits.
+    constexpr float kDivMin = 0x1p-20f, kDivMax = 0x1p20f, kDivTiny = 0x1p-100f;
+    __device__ __forceinline__ float div_rcp(float x, float d, float r)
+    {
+        float q = x * r;
+        q = fmaf(fmaf(-q, d, x), r, q);
+        return fmaf(fmaf(-q, d, x), r, q);
+    }
+    __device__ __forceinline__ bool div_tiny(float x)
+    {
+        return __float_as_uint(x) - 1u < 0x0D800000u - 1u; // 0 < x < 2^-100
+    }
+
+    // the rare texels: a colour sum so small that div_rcp does not take it, dither mode 0, or
+    // sums that can be negative or not finite
+    __device__ __noinline__ uint32_t merge_volume_texel_any(const MergeParams& p, int x, int y, int z, float4 vc)
+    {
+        return merge_volume_texel(p, p.ditherMode == 2 ? c_dither2 : c_dither1, x, y, z, vc);
+    }
+
+    // FD: 4 where a source reduces a vector or is advected, else 1; NS: sources
+    template<bool ISO, int NS, int FD>
+    __global__ void __launch_bounds__(kRowsThreads, 2) k_merge_rows(const __grid_constant__ MergeParams p, const __grid_constant__ MergeRows act)
+    {
+        extern __shared__ float4 sVol[];
+        __shared__ float sMask[64], sUnit[FD > 1 ? 256 : 1];
+        constexpr int V = kRowsPer;
+        // iso entries: (c.w / iso * 0.5, the entry's texel), as the iso texture takes whole
+        // entries and never a sum
+        float2* sIso = reinterpret_cast<float2*>(sVol + act.volTables * p.ts);
+        if(blockIdx.x == 0 && threadIdx.x == 0)
+            *p.emptyBricks = 0u; // pass 2 counts
+        if(threadIdx.x < 64)
+            sMask[threadIdx.x]
+                = fminf(float(p.ditherMode == 2 ? c_dither2[threadIdx.x] : c_dither1[threadIdx.x]) / 64.0f, kDitherMax);
+        if(FD > 1 && threadIdx.x < 256)
+            sUnit[threadIdx.x] = float(threadIdx.x) / 255.0f;
+        for(int t = 0; t < act.volTables; ++t)
+            for(int i = threadIdx.x; i < p.ts; i += kRowsThreads)
+            {
+                const float w = act.vol[t].scale;
+                float4 c = __ldg(act.vol[t].lut + i);
+                if(w > 0.0f)
+                {
+                    const float a = c.w * w;
+                    c = make_float4(c.x * a, c.y * a, c.z * a, a);
+                }
+                sVol[t * p.ts + i] = c;
+            }
+        if(ISO)
+            for(int t = 0; t < act.isoTables; ++t)
+                for(int i = threadIdx.x; i < p.ts; i += kRowsThreads)
+                {
+                    float4 c = __ldg(act.iso[t].lut + i);
+                    c.w = c.w / act.iso[t].scale * 0.5f;
+                    sIso[t * p.ts + i] = make_float2(c.w, __uint_as_float(merge_iso_texel(c)));
+                }
+        __syncthreads();
+        const float tsf = float(p.ts), tsMax = float(p.ts - 1);
+        const uint32_t lane = threadIdx.x & 31u, warps = gridDim.x * (kRowsThreads / 32);
+        const bool ceilDither = p.nonNegative && p.ditherMode != 0;
+        for(uint32_t w = blockIdx.x * (kRowsThreads / 32) + (threadIdx.x >> 5); w * (32u * V) < act.voxels; w += warps)
+        {
+            uint32_t idx[V];
+            int x[V], y[V], z[V];
+#pragma unroll
+            for(int j = 0; j < V; ++j)
+            {
+                // voxels past the end repeat the last one and are not stored
+                idx[j] = w * (32u * V) + 32u * j + lane;
+                const uint32_t i = min(idx[j], act.voxels - 1u), row = act.rowOf(i), pl = act.planeOf(row);
+                x[j] = int(i - row * act.rowOf.d);
+                y[j] = int(row - pl * act.planeOf.d);
+                z[j] = int(pl);
+            }
+            float v[NS][V][FD];
+            uint32_t adv[NS][V];
+#pragma unroll
+            for(int k = 0; k < NS; ++k)
+            {
+                const auto& S = act.src[k];
+#pragma unroll
+                for(int j = 0; j < V; ++j)
+                {
+                    const uint32_t o = uint32_t(z[j]) * S.pitchZ + uint32_t(y[j]) * S.pitchY + uint32_t(x[j]);
+                    const float* at = S.base + size_t(o) * uint32_t(S.fdim);
+                    v[k][j][0] = __ldg(at);
+#pragma unroll
+                    for(int c = 1; c < FD; ++c)
+                        v[k][j][c] = S.chain.reduce != 0 && S.fdim > c ? __ldg(at + c) : 0.0f;
+                    if(FD > 1) // field sources are vectors
+                        adv[k][j] = !S.adv ? 255u : __ldg(S.adv + (uint32_t(z[j]) * act.advPlane + uint32_t(y[j]) * act.advRow + uint32_t(x[j])));
+                }
+            }
+            float4 vc[V];
+            float isoA[V];
+            uint32_t isoT[V];
+#pragma unroll
+            for(int j = 0; j < V; ++j)
+            {
+                vc[j] = make_float4(0, 0, 0, 0);
+                isoA[j] = 0.0f;
+                isoT[j] = 0u;
+            }
+#pragma unroll
+            for(int k = 0; k < NS; ++k)
+            {
+                const auto& S = act.src[k];
+                line_chain<V, FD>(v[k], S.fdim, S.chain);
+#pragma unroll
+                for(int j = 0; j < V; ++j)
+                {
+                    // round(clamp(value * ts, 0, ts - 1)): a round-down add of 0.5 and an exact floor
+                    const float xi = fminf(fmaxf(v[k][j][0] * tsf, 0.0f), tsMax);
+                    const int e = __float_as_int(__fadd_rd(__fadd_rd(xi, 0.5f), 12582912.0f)) - 0x4B400000;
+                    if(FD > 1 && S.adv)
+                    {
+                        // field source: alpha blended with the advection texture
+                        // (MergeAdvectionToCombinedTextureIterator, isaac_common_kernel.hpp:664-665)
+                        float4 c = sVol[S.volTable * p.ts + e];
+                        c.w *= sUnit[adv[k][j]];
+                        if(S.weight > 0.0f)
+                        {
+                            const float a = c.w * S.weight;
+                            vc[j].x += c.x * a;
+                            vc[j].y += c.y * a;
+                            vc[j].z += c.z * a;
+                            vc[j].w += a;
+                        }
+                        if(ISO && S.iso > 0.0f)
+                        {
+                            c.w = c.w / S.iso * 0.5f;
+                            if(isoA[j] < c.w)
+                            {
+                                isoA[j] = c.w;
+                                isoT[j] = merge_iso_texel(c);
+                            }
+                        }
+                        continue;
+                    }
+                    if(S.volTable >= 0)
+                    {
+                        const float4 c = sVol[S.volTable * p.ts + e];
+                        vc[j].x += c.x;
+                        vc[j].y += c.y;
+                        vc[j].z += c.z;
+                        vc[j].w += c.w;
+                    }
+                    if(ISO && S.isoTable >= 0)
+                    {
+                        const float2 c = sIso[S.isoTable * p.ts + e];
+                        if(isoA[j] < c.x)
+                        {
+                            isoA[j] = c.x;
+                            isoT[j] = __float_as_uint(c.y);
+                        }
+                    }
+                }
+            }
+#pragma unroll
+            for(int j = 0; j < V; ++j)
+            {
+                if(idx[j] >= act.voxels)
+                    continue;
+                uint32_t texel;
+                float4 c = vc[j];
+                if(ceilDither && !(div_tiny(c.x) || div_tiny(c.y) || div_tiny(c.z) || div_tiny(c.w)))
+                {
+                    if(p.invTotalWeight != 0.0f)
+                        c = make_float4(c.x * p.invTotalWeight, c.y * p.invTotalWeight, c.z * p.invTotalWeight, c.w * p.invTotalWeight);
+                    else
+                        c = make_float4(div_rcp(c.x, p.totalWeight, act.rcpTotal), div_rcp(c.y, p.totalWeight, act.rcpTotal),
+                                        div_rcp(c.z, p.totalWeight, act.rcpTotal), div_rcp(c.w, p.totalWeight, act.rcpTotal));
+                    const float d = p.ditherMode <= 2 ? sMask[(x[j] & 3) + (y[j] & 3) * 4 + (z[j] & 3) * 16]
+                                                      : fminf(dither_threshold(p.ditherMode, nullptr, x[j], y[j], z[j]), kDitherMax);
+                    texel = dither_rgba_ceil(c, d);
+                }
+                else
+                    texel = merge_volume_texel_any(p, x[j], y[j], z[j], c);
+                p.volLin[idx[j]] = texel;
+                if(ISO)
+                    p.isoLin[idx[j]] = isoT[j];
+            }
+        }
+    }
+
+    size_t rows_table_bytes(const MergeRows& act, int ts)
+    {
+        return (size_t(act.volTables) * sizeof(float4) + size_t(act.isoTables) * sizeof(float2)) * ts;
+    }
+
+    template<bool ISO, int NS, int FD>
+    void launch_rows(const MergeParams& p, const MergeRows& act, cudaStream_t s)
+    {
+        const size_t bytes = rows_table_bytes(act, p.ts);
+        // the opt-in to more than 48 KiB of dynamic shared memory, once per device
+        static uint64_t configured = 0;
+        int dev = 0, sms = 148;
+        cudaGetDevice(&dev);
+        if(dev < 64 && !((configured >> dev) & 1u)
+           && cudaFuncSetAttribute(k_merge_rows<ISO, NS, FD>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kRowsSmem)) == cudaSuccess)
+            configured |= uint64_t(1) << dev;
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        const size_t resident = size_t(sms) * ctas_per_sm(k_merge_rows<ISO, NS, FD>, kRowsThreads, bytes);
+        const size_t wanted = (size_t(act.voxels) + kRowsThreads * kRowsPer - 1) / (kRowsThreads * kRowsPer);
+        k_merge_rows<ISO, NS, FD><<<unsigned(std::max<size_t>(1, std::min(resident, wanted))), kRowsThreads, bytes, s>>>(p, act);
+    }
+
+    // The parameters of k_merge_rows; false where it does not apply: no or more than 4 active
+    // sources, a pow chain or one of two reductions, tables beyond kRowsSmem, a total weight that
+    // div_rcp does not take, or 2^31 voxels and more
+    bool merge_rows(const MergeParams& p, MergeRows& r)
+    {
+        const size_t voxels = size_t(p.g.ls[0]) * p.g.ls[1] * p.g.ls[2];
+        if(voxels >= (size_t(1) << 31) || (p.nonNegative && !(p.totalWeight >= kDivMin && p.totalWeight <= kDivMax)))
+            return false;
+        r.voxels = uint32_t(voxels);
+        r.rowOf = fast_div(uint32_t(p.g.ls[0]));
+        r.planeOf = fast_div(uint32_t(p.g.ls[1]));
+        r.rcpTotal = 1.0f / p.totalWeight;
+        const size_t advRow = size_t(p.g.ls[0]) + 2 * size_t(p.advG[0]), advPlane = advRow * (size_t(p.g.ls[1]) + 2 * size_t(p.advG[1]));
+        r.advRow = uint32_t(advRow);
+        r.advPlane = uint32_t(advPlane);
+        for(int k = 0; k < p.nVol; ++k)
+        {
+            if(!(p.weight[k] + p.iso[k] > 0.0f))
+                continue;
+            if(r.n == kRowsMaxSources)
+                return false;
+            auto& S = r.src[r.n++];
+            S.base = p.src[k];
+            if(!line_chain_of(p.chain[k], S.chain) || p.pitchZ[k] * (size_t(p.g.ls[2]) + 1) >= (size_t(1) << 31))
+                return false;
+            S.pitchY = uint32_t(p.pitchY[k]);
+            S.pitchZ = uint32_t(p.pitchZ[k]);
+            S.fdim = p.fdim[k];
+            S.weight = p.weight[k];
+            S.iso = p.writeIso ? p.iso[k] : 0.0f;
+            S.adv = p.adv[k] ? p.adv[k] + (size_t(p.advG[2]) * advPlane + size_t(p.advG[1]) * advRow + size_t(p.advG[0])) : nullptr;
+            if(S.adv && advPlane * (size_t(p.g.ls[2]) + 1) >= (size_t(1) << 31))
+                return false;
+            S.volTable = S.isoTable = -1;
+            const float4* lut = p.lut + size_t(k) * p.ts;
+            if(S.adv || S.weight > 0.0f)
+            {
+                S.volTable = r.volTables;
+                r.vol[r.volTables++] = {lut, S.adv ? 0.0f : S.weight};
+            }
+            if(!S.adv && S.iso > 0.0f)
+            {
+                S.isoTable = r.isoTables;
+                r.iso[r.isoTables++] = {lut, S.iso};
+            }
+        }
+        return r.n > 0 && rows_table_bytes(r, p.ts) <= kRowsSmem;
+    }
+
+    template<bool ISO>
+    bool launch_rows_any(const MergeParams& p, cudaStream_t s)
+    {
+        MergeRows r{};
+        if(!merge_rows(p, r))
+            return false;
+        bool vec = false;
+        for(int k = 0; k < r.n; ++k)
+            vec = vec || (r.src[k].chain.reduce && r.src[k].fdim > 1) || r.src[k].adv;
+        switch(r.n)
+        {
+        case 1: vec ? launch_rows<ISO, 1, 4>(p, r, s) : launch_rows<ISO, 1, 1>(p, r, s); break;
+        case 2: vec ? launch_rows<ISO, 2, 4>(p, r, s) : launch_rows<ISO, 2, 1>(p, r, s); break;
+        case 3: vec ? launch_rows<ISO, 3, 4>(p, r, s) : launch_rows<ISO, 3, 1>(p, r, s); break;
+        default: vec ? launch_rows<ISO, 4, 4>(p, r, s) : launch_rows<ISO, 4, 1>(p, r, s); break;
+        }
+        return true;
+    }
+
     template<bool ISO>
     __global__ void __launch_bounds__(256) k_merge_voxels(const __grid_constant__ MergeParams p)
     {
@@ -358,6 +677,8 @@ namespace isaacb
         __syncthreads();
         const Geom& g = p.g;
         const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y, z = blockIdx.z;
+        if(x == 0 && y == 0 && z == 0)
+            *p.emptyBricks = 0u; // pass 2 counts
         if(x >= g.ls[0])
             return;
         const size_t i = (size_t(z) * g.ls[1] + y) * g.ls[0] + x;
@@ -369,12 +690,13 @@ namespace isaacb
             if(!(vw + it > 0.0f))
                 continue;
             float val;
+            const size_t si = size_t(z) * p.pitchZ[s] + size_t(y) * p.pitchY[s] + x;
             if(p.chainIdem[s] != 0)
-                val = __ldg(p.src[s] + i * p.fdim[s]); // every functor idem: the x component
+                val = __ldg(p.src[s] + si * p.fdim[s]); // every functor idem: the x component
             else
             {
                 float v[4];
-                read_voxel(p.src[s], p.fdim[s], i, v);
+                read_voxel(p.src[s], p.fdim[s], si, v);
                 val = apply_chain(v, p.fdim[s], p.chain[s]);
             }
             float4 c = __ldg(p.lut + size_t(s) * p.ts + lut_index_fast(val, p.ts));
@@ -557,73 +879,65 @@ namespace isaacb
         k_merge_voxels_x4_smem<NS><<<unsigned(grid), 512, tableBytes, s>>>(p, act);
     }
 
-    // returns the number of kernels launched
+    // Pass 1 by the sources: scalar ones without chains over aligned rows, no iso output and
+    // tables that fit take four voxels per thread from premultiplied tables; other sets of up
+    // to 4 sources k_merge_rows; scalar ones with tables beyond shared memory four voxels per
+    // thread from global tables; the rest (more sources, pow, huge tables) one voxel per thread.
+    // Returns the number of kernels launched.
     template<bool ISO>
     int launch_merge_iso(const MergeParams& p, cudaStream_t s)
     {
-        const dim3 vgrid((p.g.ls[0] + 255) / 256, p.g.ls[1], p.g.ls[2]);
         MergeActive act{};
         bool scalar = true;
         for(int k = 0; k < p.nVol; ++k)
         {
             if(!(p.weight[k] + p.iso[k] > 0.0f))
                 continue;
-            scalar = scalar && p.chainIdem[k] && p.fdim[k] == 1 && !p.adv[k];
+            scalar = scalar && p.chainIdem[k] && p.fdim[k] == 1 && !p.adv[k] && p.pitchY[k] == size_t(p.g.ls[0]);
             act.src[act.n] = p.src[k];
             act.lut[act.n] = p.lut + size_t(k) * p.ts;
             act.weight[act.n] = p.weight[k];
             act.iso[act.n] = p.iso[k];
             act.n++;
         }
-        bool x4 = (p.g.ls[0] & 3) == 0 && size_t(p.g.ls[0] / 4) * p.g.ls[1] * p.g.ls[2] < (size_t(1) << 32);
+        const size_t quads = size_t(p.g.ls[0] / 4) * p.g.ls[1] * p.g.ls[2];
+        bool x4 = scalar && act.n >= 1 && act.n <= 4 && (p.g.ls[0] & 3) == 0 && quads < (size_t(1) << 32);
         for(int k = 0; k < act.n; ++k)
             x4 = x4 && (reinterpret_cast<uintptr_t>(act.src[k]) & 15u) == 0;
+        const size_t tableBytes = size_t(act.n) * p.ts * sizeof(float4);
         int launches = 2;
-        if(scalar && x4 && act.n >= 1 && act.n <= 4)
+        if((x4 && !ISO && tableBytes <= kMergeSmemTables) || !launch_rows_any<ISO>(p, s))
         {
-            const size_t quads = size_t(p.g.ls[0] / 4) * p.g.ls[1] * p.g.ls[2];
-            const unsigned blocks = unsigned((quads + 255) / 256);
-            if(!ISO)
+            if(x4)
             {
-                for(int k = 0; k < act.n; ++k)
-                    act.pre[k] = p.lutPre + size_t(k) * p.ts;
-                k_merge_premultiply<<<dim3((p.ts + 255) / 256, act.n), 256, 0, s>>>(act, p.lutPre, p.ts);
-                launches++;
-            }
-            const size_t tableBytes = size_t(act.n) * p.ts * sizeof(float4);
-            if(!ISO && tableBytes <= kMergeSmemTables)
-            {
-                switch(act.n)
+                if(!ISO)
                 {
-                case 1: launch_x4_smem<1>(p, act, quads, tableBytes, s); break;
-                case 2: launch_x4_smem<2>(p, act, quads, tableBytes, s); break;
-                case 3: launch_x4_smem<3>(p, act, quads, tableBytes, s); break;
-                default: launch_x4_smem<4>(p, act, quads, tableBytes, s); break;
+                    for(int k = 0; k < act.n; ++k)
+                        act.pre[k] = p.lutPre + size_t(k) * p.ts;
+                    k_merge_premultiply<<<dim3((p.ts + 255) / 256, act.n), 256, 0, s>>>(act, p.lutPre, p.ts);
+                    launches++;
                 }
+                const unsigned blocks = unsigned((quads + 255) / 256);
+                if(!ISO && tableBytes <= kMergeSmemTables)
+                    switch(act.n)
+                    {
+                    case 1: launch_x4_smem<1>(p, act, quads, tableBytes, s); break;
+                    case 2: launch_x4_smem<2>(p, act, quads, tableBytes, s); break;
+                    case 3: launch_x4_smem<3>(p, act, quads, tableBytes, s); break;
+                    default: launch_x4_smem<4>(p, act, quads, tableBytes, s); break;
+                    }
+                else
+                    switch(act.n)
+                    {
+                    case 1: k_merge_voxels_x4<ISO, 1><<<blocks, 256, 0, s>>>(p, act); break;
+                    case 2: k_merge_voxels_x4<ISO, 2><<<blocks, 256, 0, s>>>(p, act); break;
+                    case 3: k_merge_voxels_x4<ISO, 3><<<blocks, 256, 0, s>>>(p, act); break;
+                    default: k_merge_voxels_x4<ISO, 4><<<blocks, 256, 0, s>>>(p, act); break;
+                    }
             }
             else
-            {
-                switch(act.n)
-                {
-                case 1: k_merge_voxels_x4<ISO, 1><<<blocks, 256, 0, s>>>(p, act); break;
-                case 2: k_merge_voxels_x4<ISO, 2><<<blocks, 256, 0, s>>>(p, act); break;
-                case 3: k_merge_voxels_x4<ISO, 3><<<blocks, 256, 0, s>>>(p, act); break;
-                default: k_merge_voxels_x4<ISO, 4><<<blocks, 256, 0, s>>>(p, act); break;
-                }
-            }
+                k_merge_voxels<ISO><<<dim3((p.g.ls[0] + 255) / 256, p.g.ls[1], p.g.ls[2]), 256, 0, s>>>(p);
         }
-        else if(scalar && act.n >= 1 && act.n <= 4)
-        {
-            switch(act.n)
-            {
-            case 1: k_merge_voxels_n<ISO, 1><<<vgrid, 256, 0, s>>>(p, act); break;
-            case 2: k_merge_voxels_n<ISO, 2><<<vgrid, 256, 0, s>>>(p, act); break;
-            case 3: k_merge_voxels_n<ISO, 3><<<vgrid, 256, 0, s>>>(p, act); break;
-            default: k_merge_voxels_n<ISO, 4><<<vgrid, 256, 0, s>>>(p, act); break;
-            }
-        }
-        else
-            k_merge_voxels<ISO><<<vgrid, 256, 0, s>>>(p);
         const dim3 pgrid((p.g.nb[0] + kPackRow - 1) / kPackRow, p.g.nb[1], p.g.nb[2]);
         if(p.g.yfast)
             k_merge_pack<ISO, true><<<pgrid, 256, 0, s>>>(p);
@@ -727,29 +1041,6 @@ namespace isaacb
     {
         for(size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x; i < n; i += size_t(gridDim.x) * blockDim.x)
             dst[i] = gclamp(src[i] * 30.0f, 0.0f, 1.0f);
-    }
-
-    // one thread per float of the compact copy: consecutive threads read consecutive
-    // floats of one guarded row
-    __global__ void __launch_bounds__(256)
-        k_compact_guarded(const float* __restrict__ src, float* __restrict__ dst, int X, int Y, int Z, int g, int fd)
-    {
-        const size_t rowF = size_t(X) * fd;
-        const size_t n = rowF * Y * Z;
-        const size_t gx = size_t(X + 2 * g), gy = size_t(Y + 2 * g);
-        for(size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x; i < n; i += size_t(gridDim.x) * blockDim.x)
-        {
-            const size_t row = i / rowF, k = i - row * rowF;
-            const size_t y = row % Y, z = row / Y;
-            dst[i] = __ldg(src + (((z + g) * gy + (y + g)) * gx + g) * fd + k);
-        }
-    }
-
-    void launch_compact_guarded(const float* src, float* dst, int X, int Y, int Z, int guard, int fdim, cudaStream_t s)
-    {
-        const size_t n = size_t(X) * Y * Z * fdim;
-        const size_t blocks = std::min<size_t>((n + 255) / 256, size_t(148) * 32);
-        k_compact_guarded<<<unsigned(blocks), 256, 0, s>>>(src, dst, X, Y, Z, guard, fdim);
     }
 
     void launch_noise(const NoiseParams& p, float* noise, float* tmp, cudaStream_t s)

@@ -11,16 +11,23 @@
 // scan order (column x + y*X, then z, then particle index).
 #include "isaacb_internal.h"
 
+#include <algorithm>
 #include <cfloat>
 
 namespace isaacb
 {
     constexpr int kMMThreads = 256;
 
-    __device__ __forceinline__ float mm_value(const MinMaxParams& p, size_t idx)
+    // voxel i of the interior in x, y, z order
+    __device__ __forceinline__ float mm_value(const MinMaxParams& p, size_t i)
     {
         float v[4];
-        const float* sp = p.src + idx * p.fdim;
+        if(p.pitchY != size_t(p.g.ls[0]))
+        {
+            const size_t row = i / size_t(p.g.ls[0]), z = row / size_t(p.g.ls[1]);
+            i = z * p.pitchZ + (row - z * size_t(p.g.ls[1])) * p.pitchY + (i - row * size_t(p.g.ls[0]));
+        }
+        const float* sp = p.src + i * p.fdim;
         v[0] = __ldg(sp);
         v[1] = p.fdim > 1 ? __ldg(sp + 1) : 0.0f;
         v[2] = p.fdim > 2 ? __ldg(sp + 2) : 0.0f;
@@ -67,7 +74,35 @@ namespace isaacb
         }
     }
 
-    __global__ void __launch_bounds__(kMMThreads) k_minmax_partial(const __grid_constant__ MinMaxParams p)
+    // The block's result joins the others': the last block to arrive reduces them all and
+    // leaves the ticket at zero for the next launch.
+    __device__ __forceinline__ void mm_finish(const MinMaxParams& p, float lo, float hi)
+    {
+        __shared__ bool last;
+        block_reduce(lo, hi, p.partial + 2 * blockIdx.x);
+        if(threadIdx.x == 0)
+        {
+            __threadfence();
+            last = atomicAdd(p.ticket, 1u) == gridDim.x - 1;
+        }
+        __syncthreads();
+        if(!last)
+            return;
+        __threadfence();
+        lo = FLT_MAX;
+        hi = -FLT_MAX;
+        for(unsigned i = threadIdx.x; i < gridDim.x; i += blockDim.x)
+        {
+            lo = gmin(lo, __ldcg(p.partial + 2 * i));
+            hi = gmax(hi, __ldcg(p.partial + 2 * i + 1));
+        }
+        block_reduce(lo, hi, p.result);
+        if(threadIdx.x == 0)
+            *p.ticket = 0u;
+    }
+
+    // any source or particle source, one value at a time
+    __global__ void __launch_bounds__(kMMThreads) k_minmax(const __grid_constant__ MinMaxParams p)
     {
         float lo = FLT_MAX, hi = -FLT_MAX;
         if(!p.particle)
@@ -93,37 +128,90 @@ namespace isaacb
                 }
             }
         }
-        block_reduce(lo, hi, p.partial + 2 * blockIdx.x);
+        mm_finish(p, lo, hi);
     }
 
-    __global__ void __launch_bounds__(kMMThreads) k_minmax_final(const float* __restrict__ partial, int n, float* result)
+    // A source without ghost cells, 16-byte aligned, its chain a LineChain: 4 voxels are FD
+    // 16-byte loads, and a thread issues those of UNROLL groups before it uses one, 64 bytes
+    // or more in flight each.  Bound by memory: one value at a time took 0.54 ms for a 512^3
+    // scalar and 0.66 ms for a vector field, both together 1.26 ms with their reads; this takes
+    // 0.36 ms for both, 5.9 TB/s.
+    template<int FD, bool CHAIN>
+    __global__ void __launch_bounds__(kMMThreads) k_minmax_vec(const __grid_constant__ MinMaxParams p, const __grid_constant__ LineChain chain)
     {
+        constexpr int UNROLL = FD == 1 ? 4 : 2;
         float lo = FLT_MAX, hi = -FLT_MAX;
-        for(int i = threadIdx.x; i < n; i += blockDim.x)
+        const size_t n = size_t(p.g.ls[0]) * p.g.ls[1] * p.g.ls[2], groups = n / 4;
+        const float4* src = reinterpret_cast<const float4*>(p.src);
+        auto take = [&](float (&v)[4][FD]) {
+            if(CHAIN)
+                line_chain<4, FD>(v, FD, chain);
+#pragma unroll
+            for(int j = 0; j < 4; ++j)
+            {
+                lo = gmin(lo, v[j][0]);
+                hi = gmax(hi, v[j][0]);
+            }
+        };
+        const size_t stride = size_t(gridDim.x) * kMMThreads;
+        for(size_t q = blockIdx.x * size_t(kMMThreads) + threadIdx.x; q < groups; q += UNROLL * stride)
         {
-            lo = gmin(lo, partial[2 * i]);
-            hi = gmax(hi, partial[2 * i + 1]);
+            float4 raw[UNROLL][FD];
+#pragma unroll
+            for(int u = 0; u < UNROLL; ++u)
+#pragma unroll
+                for(int c = 0; c < FD; ++c) // a group past the end repeats the first
+                    raw[u][c] = __ldg(src + (q + u * stride < groups ? q + u * stride : q) * FD + c);
+#pragma unroll
+            for(int u = 0; u < UNROLL; ++u)
+            {
+                float f[4 * FD], v[4][FD];
+#pragma unroll
+                for(int c = 0; c < FD; ++c)
+                    f[4 * c] = raw[u][c].x, f[4 * c + 1] = raw[u][c].y, f[4 * c + 2] = raw[u][c].z, f[4 * c + 3] = raw[u][c].w;
+#pragma unroll
+                for(int j = 0; j < 4; ++j)
+#pragma unroll
+                    for(int c = 0; c < FD; ++c)
+                        v[j][c] = f[j * FD + c];
+                take(v);
+            }
         }
-        block_reduce(lo, hi, result);
+        if(blockIdx.x == 0 && threadIdx.x < n - 4 * groups)
+        {
+            const float v = mm_value(p, 4 * groups + threadIdx.x);
+            lo = gmin(lo, v);
+            hi = gmax(hi, v);
+        }
+        mm_finish(p, lo, hi);
     }
 
-    int minmax_blocks(const MinMaxParams& p)
+    int minmax_blocks(const MinMaxParams& p, size_t perThread = 1)
     {
         const size_t n = p.particle ? size_t(p.g.lps[0]) * p.g.lps[1] * p.g.lps[2]
                                     : size_t(p.g.ls[0]) * p.g.ls[1] * p.g.ls[2];
-        size_t b = (n + kMMThreads - 1) / kMMThreads;
-        const size_t cap = 148 * 8;
-        if(b > cap)
-            b = cap;
-        if(b < 1)
-            b = 1;
-        return int(b);
+        const size_t per = kMMThreads * perThread;
+        return int(std::max<size_t>(1, std::min<size_t>((n + per - 1) / per, kMinMaxBlocks)));
     }
 
-    void launch_minmax(const MinMaxParams& p, int blocks, float* result, cudaStream_t s)
+    void launch_minmax(const MinMaxParams& p, cudaStream_t s)
     {
-        k_minmax_partial<<<blocks, kMMThreads, 0, s>>>(p);
-        k_minmax_final<<<1, kMMThreads, 0, s>>>(p.partial, blocks, result);
+        LineChain line;
+        const bool vec = !p.particle && p.pitchY == size_t(p.g.ls[0]) && (reinterpret_cast<uintptr_t>(p.src) & 15u) == 0
+            && line_chain_of(p.chain, line);
+        if(!vec)
+        {
+            k_minmax<<<minmax_blocks(p), kMMThreads, 0, s>>>(p);
+            return;
+        }
+        const int blocks = minmax_blocks(p, 4);
+        switch(p.fdim)
+        {
+        case 1: line.idem ? k_minmax_vec<1, false><<<blocks, kMMThreads, 0, s>>>(p, line) : k_minmax_vec<1, true><<<blocks, kMMThreads, 0, s>>>(p, line); break;
+        case 2: line.idem ? k_minmax_vec<2, false><<<blocks, kMMThreads, 0, s>>>(p, line) : k_minmax_vec<2, true><<<blocks, kMMThreads, 0, s>>>(p, line); break;
+        case 3: line.idem ? k_minmax_vec<3, false><<<blocks, kMMThreads, 0, s>>>(p, line) : k_minmax_vec<3, true><<<blocks, kMMThreads, 0, s>>>(p, line); break;
+        default: line.idem ? k_minmax_vec<4, false><<<blocks, kMMThreads, 0, s>>>(p, line) : k_minmax_vec<4, true><<<blocks, kMMThreads, 0, s>>>(p, line); break;
+        }
     }
 
     // Reference scan-order key of the first +0 and the first -0:
