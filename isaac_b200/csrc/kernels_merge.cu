@@ -1037,6 +1037,69 @@ namespace isaacb
         }
     }
 
+    // The same for voxels of unit scale, where every sample lies half way between texels: the
+    // 7 samples along the axis read 8 x 2 x 2 texels (x-1, x on the other axes), 32 loads
+    // instead of 56 with six remainders each.  The lerps keep sample_linear's order (z, y, x)
+    // and its operations at offset 1/2, so the results are the same bits.  256^3: 1.21 ms a
+    // pass before, 0.23 now.
+    template<int AXIS>
+    __global__ void __launch_bounds__(256) k_noise_blur_unit(NoiseParams p, FastDiv rowOf, FastDiv planeOf, uint32_t n,
+                                                             const float* __restrict__ src, float* __restrict__ dst)
+    {
+        const float g7[4] = {64.0f, 40.5f, 10.0f, 1.0f};
+        auto half = [](float a, float b) { return a * 0.5f + b * 0.5f; }; // lin(0.5, a, b)
+        for(uint32_t i = blockIdx.x * 256u + threadIdx.x; i < n; i += gridDim.x * 256u)
+        {
+            const uint32_t row = rowOf(i), pl = planeOf(row);
+            const int c[3] = {int(i - row * rowOf.d), int(row - pl * planeOf.d), int(pl)};
+            const int L[3] = {p.LX, p.LY, p.LZ};
+            const uint32_t pitch[3] = {1u, uint32_t(p.LX), uint32_t(p.LX) * uint32_t(p.LY)};
+            uint32_t at[8]; // along the axis: c - 4 .. c + 3, REPEAT border (at least 4 voxels)
+#pragma unroll
+            for(int k = 0; k < 8; ++k)
+            {
+                int a = c[AXIS] + k - 4;
+                a += a < 0 ? L[AXIS] : 0;
+                a -= a >= L[AXIS] ? L[AXIS] : 0;
+                at[k] = uint32_t(a) * pitch[AXIS];
+            }
+            uint32_t side[3][2];
+#pragma unroll
+            for(int a = 0; a < 3; ++a)
+            {
+                side[a][0] = uint32_t(c[a] > 0 ? c[a] - 1 : L[a] - 1) * pitch[a];
+                side[a][1] = uint32_t(c[a]) * pitch[a];
+            }
+            constexpr int U = AXIS == 0 ? 1 : 0, W = AXIS == 2 ? 1 : 2; // the other axes, U before W
+            // v[k][w][u]
+            float v[8][2][2];
+#pragma unroll
+            for(int k = 0; k < 8; ++k)
+#pragma unroll
+                for(int w = 0; w < 2; ++w)
+#pragma unroll
+                    for(int u = 0; u < 2; ++u)
+                        v[k][w][u] = __ldg(src + (at[k] + side[W][w] + side[U][u]));
+            float r = 0.0f;
+#pragma unroll
+            for(int k = 0; k < 7; ++k)
+            {
+                float s;
+                if(AXIS == 0) // U = y, W = z
+                    s = half(half(half(v[k][0][0], v[k][1][0]), half(v[k][0][1], v[k][1][1])),
+                             half(half(v[k + 1][0][0], v[k + 1][1][0]), half(v[k + 1][0][1], v[k + 1][1][1])));
+                else if(AXIS == 1) // U = x, W = z
+                    s = half(half(half(v[k][0][0], v[k][1][0]), half(v[k + 1][0][0], v[k + 1][1][0])),
+                             half(half(v[k][0][1], v[k][1][1]), half(v[k + 1][0][1], v[k + 1][1][1])));
+                else // U = x, W = y
+                    s = half(half(half(v[k][0][0], v[k + 1][0][0]), half(v[k][1][0], v[k + 1][1][0])),
+                             half(half(v[k][0][1], v[k + 1][0][1]), half(v[k][1][1], v[k + 1][1][1])));
+                r += s * g7[k < 3 ? 3 - k : k - 3];
+            }
+            dst[i] = r / 167.0f;
+        }
+    }
+
     __global__ void k_noise_clamp(size_t n, const float* __restrict__ src, float* __restrict__ dst)
     {
         for(size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x; i < n; i += size_t(gridDim.x) * blockDim.x)
@@ -1050,15 +1113,31 @@ namespace isaacb
         if(p.seedPoints > 0)
             k_noise_seed<<<(p.seedPoints + 255) / 256, 256, 0, s>>>(p, noise);
         const int blocks = int(std::min<size_t>((n + 255) / 256, 148 * 16));
-        k_noise_blur<<<blocks, 256, 0, s>>>(p, noise, tmp, 0);
-        k_noise_blur<<<blocks, 256, 0, s>>>(p, tmp, noise, 1);
-        k_noise_blur<<<blocks, 256, 0, s>>>(p, noise, tmp, 2);
+        if(p.scale[0] == 1.0f && p.scale[1] == 1.0f && p.scale[2] == 1.0f && std::min(p.LX, std::min(p.LY, p.LZ)) >= 4
+           && n < (size_t(1) << 31))
+        {
+            const FastDiv rows = fast_div(uint32_t(p.LX)), planes = fast_div(uint32_t(p.LY));
+            k_noise_blur_unit<0><<<blocks, 256, 0, s>>>(p, rows, planes, uint32_t(n), noise, tmp);
+            k_noise_blur_unit<1><<<blocks, 256, 0, s>>>(p, rows, planes, uint32_t(n), tmp, noise);
+            k_noise_blur_unit<2><<<blocks, 256, 0, s>>>(p, rows, planes, uint32_t(n), noise, tmp);
+        }
+        else
+        {
+            k_noise_blur<<<blocks, 256, 0, s>>>(p, noise, tmp, 0);
+            k_noise_blur<<<blocks, 256, 0, s>>>(p, tmp, noise, 1);
+            k_noise_blur<<<blocks, 256, 0, s>>>(p, noise, tmp, 2);
+        }
         k_noise_clamp<<<blocks, 256, 0, s>>>(n, tmp, noise);
     }
 
-    __global__ void k_advect(const __grid_constant__ AdvectParams p)
+    // One thread per voxel: the direction's back-traced history sample, the noise, the dither.
+    // Bound by instructions, so that the index takes no 64-bit remainders, the three
+    // components share one reciprocal with exact corrections (div_rcp) as the division by 255
+    // does, a scale of 1 divides nothing, and the 8 taps are bounds-checked once for all.  The
+    // rare voxels outside those cases (a vanishing or huge vector, a tap beyond the guard
+    // band) take the general operations.  256^3: 327 us before, 171 now.
+    __global__ void __launch_bounds__(256) k_advect(const __grid_constant__ AdvectParams p, FastDiv rowOf, FastDiv planeOf, size_t n)
     {
-        const size_t n = size_t(p.LX) * p.LY * p.LZ;
         const int SX = p.LX + 2 * p.G[0], SY = p.LY + 2 * p.G[1];
         auto at = [&](int x, int y, int z) {
             return (size_t(z + p.G[2]) * SY + (y + p.G[1])) * SX + (x + p.G[0]);
@@ -1070,21 +1149,56 @@ namespace isaacb
                 return 0.0f;
             return float(__ldg(p.back + at(x, y, z)));
         };
-        for(size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x; i < n; i += size_t(gridDim.x) * blockDim.x)
+        const bool unit = p.scale[0] == 1.0f && p.scale[1] == 1.0f && p.scale[2] == 1.0f;
+        for(size_t i = blockIdx.x * size_t(256) + threadIdx.x; i < n; i += size_t(gridDim.x) * 256)
         {
-            const int x = int(i % p.LX);
-            const size_t t = i / p.LX;
-            const int y = int(t % p.LY), z = int(t / p.LY);
+            const uint32_t row = n < (size_t(1) << 31) ? rowOf(uint32_t(i)) : uint32_t(i / rowOf.d), pl = planeOf(row);
+            const int x = int(i - size_t(row) * rowOf.d), y = int(row - pl * planeOf.d), z = int(pl);
             float vx = __ldg(p.field + 3 * i), vy = __ldg(p.field + 3 * i + 1), vz = __ldg(p.field + 3 * i + 2);
             // glm::length: sqrt((x*x + y*y) + z*z); at least FLT_MIN
             const float len = gmax(sqrtf((vx * vx + vy * vy) + vz * vz), 1.17549435e-38f);
-            vx = vx / len;
-            vy = vy / len;
-            vz = vz / len;
-            const float cx = (float(x) + 0.5f) - vx * p.stepSize / p.scale[0];
-            const float cy = (float(y) + 0.5f) - vy * p.stepSize / p.scale[1];
-            const float cz = (float(z) + 0.5f) - vz * p.stepSize / p.scale[2];
-            const float history = sample_linear(cx, cy, cz, fetch) / 255.0f;
+            // components that div_rcp takes: 0, or not below 2^-100 in size
+            auto small = [](float v) { return div_tiny(fabsf(v)); };
+            if(len >= kDivMin && len <= kDivMax && !(small(vx) || small(vy) || small(vz)))
+            {
+                const float r = __frcp_rn(len);
+                vx = div_rcp(vx, len, r);
+                vy = div_rcp(vy, len, r);
+                vz = div_rcp(vz, len, r);
+            }
+            else
+            {
+                vx = vx / len;
+                vy = vy / len;
+                vz = vz / len;
+            }
+            float dx = vx * p.stepSize, dy = vy * p.stepSize, dz = vz * p.stepSize;
+            if(!unit)
+            {
+                dx = dx / p.scale[0];
+                dy = dy / p.scale[1];
+                dz = dz / p.scale[2];
+            }
+            const float cx = (float(x) + 0.5f) - dx, cy = (float(y) + 0.5f) - dy, cz = (float(z) + 0.5f) - dz;
+            float history;
+            {
+                const float ux = cx - 0.5f, uy = cy - 0.5f, uz = cz - 0.5f;
+                const float flx = floorf(ux), fly = floorf(uy), flz = floorf(uz);
+                const int bx = int(flx) + p.G[0], by = int(fly) + p.G[1], bz = int(flz) + p.G[2];
+                // texels b and b + 1 of every axis inside the guarded texture
+                if(uint32_t(bx) < uint32_t(SX - 1) && uint32_t(by) < uint32_t(SY - 1) && uint32_t(bz) < uint32_t(p.LZ + 2 * p.G[2] - 1))
+                {
+                    const uint8_t* q = p.back + ((size_t(bz) * SY + by) * SX + bx);
+                    const uint8_t* q2 = q + size_t(SX) * SY;
+                    history = tri_q(ux - flx, uy - fly, uz - flz, float(__ldg(q)), float(__ldg(q + 1)), float(__ldg(q + SX)),
+                                    float(__ldg(q + SX + 1)), float(__ldg(q2)), float(__ldg(q2 + 1)), float(__ldg(q2 + SX)),
+                                    float(__ldg(q2 + SX + 1)));
+                }
+                else
+                    history = sample_linear(cx, cy, cz, fetch);
+            }
+            // a trilinear of bytes is 0 or at least (2^-25)^3
+            history = div_rcp(history, 255.0f, 1.0f / 255.0f);
             const float nv = p.seedNoise ? __ldg(p.noise + i) : 0.0f;
             const float v = nv + history * p.historyWeight * (1.0f - nv);
             // applyDither3D(5, coord, v): the 16^3 blue-noise mask, int(s) + (fract(s) > d), clamped
@@ -1104,7 +1218,7 @@ namespace isaacb
     void launch_advect(const AdvectParams& p, cudaStream_t s)
     {
         const size_t n = size_t(p.LX) * p.LY * p.LZ;
-        k_advect<<<int(std::min<size_t>((n + 255) / 256, 148 * 16)), 256, 0, s>>>(p);
+        k_advect<<<int(std::min<size_t>((n + 255) / 256, 148 * 16)), 256, 0, s>>>(p, fast_div(uint32_t(p.LX)), fast_div(uint32_t(p.LY)), n);
     }
 
     // guard slab voxel c <-> texture voxel, per axis (the reference's index arithmetic,

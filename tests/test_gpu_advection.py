@@ -61,3 +61,34 @@ def test_field_source_rules():
     viz.setRenderOptimization(False)
     with pytest.raises(_lib.IsaacError):
         viz.update()  # the per-source renderer does not merge field sources
+
+
+@pytest.mark.parametrize("size", [(4, 4, 4), (3, 9, 5), (33, 5, 4), (17, 40, 6)])
+@pytest.mark.parametrize("scale", [(1.0, 1.0, 1.0), (1.0, 0.75, 1.5)])
+@pytest.mark.parametrize("step", [0.4, 3.0])
+def test_noise_and_advection_edges(size, scale, step):
+    """Sizes where the blur's window wraps or falls back, scales other than 1, steps past
+    the guard band, and vectors that vanish, overflow or are not numbers: noise and
+    advection textures bit-exact over several frames."""
+    from harness import Scene
+
+    x, y, z = size
+    rng = np.random.default_rng(x * y + z)
+    a = rng.uniform(0.0, 1.0, (z, y, x)).astype(np.float32)
+    f = rng.standard_normal((z, y, x, 3)).astype(np.float32)
+    flat = f.reshape(-1, 3)
+    flat[:8] = [[0, 0, 0], [1e-30, 0, 0], [1e-42, -1e-42, 0], [1, 1e-35, -1e-40], [3e20, -3e20, 1], [1e-7, 2e-7, 0], [0, -0.0, 5e-5], [2e6, 1, 1]]
+    flat[9] = [np.inf, 1, 0]
+    s = Scene(n=size, fb=(32, 24), volumes=[(a, True), (f, True)], functions=["idem", "length"], scale=scale)
+    viz, o = build_gpu(s), build_oracle(s)
+    viz.setFieldSource(1)
+    o.set_field(1)
+    p = dict(step_factor=step, history_weight=0.9, seeding_period=2, seeding_duration=1, seed_points=max(2, x * y * z // 8))
+    viz.setAdvection(**p)
+    o.set_advection(*p.values())
+    assert np.array_equal(viz.noiseTexture(), o.noise())
+    for frame in range(4):
+        viz.update()
+        o.update()
+        assert np.array_equal(viz.advectionTexture(1), o.advection(1)), frame
+    viz.close()
