@@ -1438,27 +1438,44 @@ extern "C"
         c->renderLaunches = 0;
         for(int k = 1; k < ISAACB_TIMING_SLOTS; ++k)
             c->evUsed[k] = false;
+        // the pass that shades also writes the caller's frame, unless that is unaligned or
+        // the framebuffer itself
+        const bool direct = rgba_dev && (reinterpret_cast<uintptr_t>(rgba_dev) & 3u) == 0 && rgba_dev != reinterpret_cast<uint8_t*>(c->color);
+        p.out = direct ? reinterpret_cast<uchar4*>(rgba_dev) : nullptr;
+        p.shadeDepth = c->renderMode == 2 || (c->renderMode >= 4 && c->renderMode <= 8) ? 1 : 0;
+        // the first pass of the frame clears the G-buffer: the particles' where there are
+        // any, else the iso surface's or the shading's; SSAO and the per-source kernels that
+        // read it need it cleared before
+        bool particles = false;
+        for(int s = 0; s < c->nPart; ++s)
+            particles = particles || c->weight[c->nVol + s] != 0.0f;
+        const bool combined = c->renderer == ISAACB_RENDERER_COMBINED;
+        const bool ssao = c->aoEnabled && c->aoWeight > 0.0f;
+        bool iso = any_iso_active(c), clean = true;
+        if(!combined)
+        {
+            iso = false;
+            for(int s = 0; s < c->nVol; ++s)
+                iso = iso || c->iso[s] != 0.0f;
+        }
+        if(particles || (ssao && !(iso && combined)) || (!combined && (iso || !per_source_specialised(p))))
         {
             PhaseTimer t(c, 1, st);
             launch_clear_particles(p, st);
+            c->renderLaunches++;
+            clean = false;
         }
-        c->renderLaunches++;
-        if(c->renderer == ISAACB_RENDERER_COMBINED)
-        {
-            if(any_iso_active(c))
-            {
-                PhaseTimer t(c, 2, st);
-                launch_iso(p, st);
-                c->renderLaunches++;
-            }
-        }
-        else
+        if(iso)
         {
             PhaseTimer t(c, 2, st);
-            launch_iso_per_source(p, st);
+            if(combined)
+                launch_iso(p, clean, st);
+            else
+                launch_iso_per_source(p, st);
             c->renderLaunches++;
+            clean = false;
         }
-        if(c->aoEnabled && c->aoWeight > 0.0f)
+        if(ssao)
         {
             PhaseTimer t(c, 3, st);
             launch_ssao(p, st);
@@ -1466,16 +1483,16 @@ extern "C"
         }
         {
             PhaseTimer t(c, 4, st);
-            if(c->renderer == ISAACB_RENDERER_COMBINED)
+            if(combined)
             {
-                launch_shade_volume(p, p.totalWeightAll > 0.0f, st);
+                launch_shade_volume(p, p.totalWeightAll > 0.0f, clean, st);
                 c->renderLaunches++;
             }
             else
-                c->renderLaunches += uint32_t(launch_shade_volume_per_source(p, st));
+                c->renderLaunches += uint32_t(launch_shade_volume_per_source(p, clean, st));
         }
         ISAACB_CUDA(c, cudaGetLastError(), "isaacb_render launch");
-        if(rgba_dev)
+        if(rgba_dev && !direct && rgba_dev != reinterpret_cast<uint8_t*>(c->color))
         {
             const size_t bytes = size_t(c->desc.framebuffer[0]) * c->desc.framebuffer[1] * 4;
             ISAACB_CUDA(c, cudaMemcpyAsync(rgba_dev, c->color, bytes, cudaMemcpyDeviceToDevice, st), "frame copy");

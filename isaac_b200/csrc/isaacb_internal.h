@@ -206,6 +206,8 @@ namespace isaacb
         float negZero; // -0.0f, the addend of packed products that must round on their own (f2p_mul_exact)
         // G-buffer
         uchar4* color;
+        uchar4* out; // the caller's frame, null: none
+        int32_t shadeDepth; // the shading changes the depth (render modes 2 and 4 to 8)
         float* depth;
         float* normal; // 3 floats per pixel
         float* ao;
@@ -259,10 +261,13 @@ namespace isaacb
     int batch_max_blocks_per_sm();
 
     void launch_clear_particles(const FrameParams& p, cudaStream_t s);
-    void launch_iso(const FrameParams& p, cudaStream_t s);
+    // clean: no pass has written the G-buffer of this frame yet, so that this one also clears it
+    void launch_iso(const FrameParams& p, bool clean, cudaStream_t s);
     void launch_iso_per_source(const FrameParams& p, cudaStream_t s);
     void launch_ssao(const FrameParams& p, cudaStream_t s);
-    void launch_shade_volume(const FrameParams& p, bool volume, cudaStream_t s);
+    void launch_shade_volume(const FrameParams& p, bool volume, bool clean, cudaStream_t s);
+    // the per-source volume pass can be a frame's only one (clean)
+    bool per_source_specialised(const FrameParams& p);
     // returns the number of kernels it launched
-    int launch_shade_volume_per_source(const FrameParams& p, cudaStream_t s);
+    int launch_shade_volume_per_source(const FrameParams& p, bool clean, cudaStream_t s);
 } // namespace isaacb

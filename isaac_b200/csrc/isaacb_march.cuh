@@ -46,6 +46,24 @@ namespace isaacb
         return make_float4(tri(A.x, B.x), tri(A.y, B.y), tri(A.z, B.z), tri(A.w, B.w));
     }
 
+    // the last step index, at least fi and at most fe, whose position c0 + sv * i stays inside
+    // the sample region [8b-1, 8b+7) of the brick of apron-shifted texel (ax, ay, az)
+    __device__ __forceinline__ float last_step_in_brick(int ax, int ay, int az, const float (&c0)[3], const float (&sv)[3], float fi, float fe)
+    {
+        float tEnd = 3.0e38f;
+        const float bl[3] = {float(ax & ~7) - 1.0f, float(ay & ~7) - 1.0f, float(az & ~7) - 1.0f};
+#pragma unroll
+        for(int a = 0; a < 3; ++a)
+        {
+            if(sv[a] > 0.0f)
+                tEnd = fminf(tEnd, (bl[a] + 8.0f - c0[a]) / sv[a]);
+            else if(sv[a] < 0.0f)
+                tEnd = fminf(tEnd, (bl[a] - c0[a]) / sv[a]);
+        }
+        // margin: 1e-3 steps plus the float rounding of tEnd itself
+        return fminf(fmaxf(floorf(tEnd - (1.0e-3f + 1.0e-6f * fabsf(tEnd))), fi), fe);
+    }
+
     // Front-to-back march of CombinedVolumeRenderKernel (lib/isaac/isaac_volume_kernel.hpp:61-87)
     // at the reference's sample positions.  Differences from the exact form, all far
     // below one output LSB and covered by the parity tests:
@@ -114,22 +132,9 @@ namespace isaacb
             }
             if(SKIP && empty)
             {
-                // last step index whose position stays inside this brick's sample region
-                // [8b-1, 8b+7) per axis, with a 1e-3-step margin against rounding
-                float tEnd = 3.0e38f;
-                const float bl[3] = {float(ax & ~7) - 1.0f, float(ay & ~7) - 1.0f, float(az & ~7) - 1.0f};
                 const float sv[3] = {svx, svy, svz};
                 const float c0[3] = {c0x, c0y, c0z};
-#pragma unroll
-                for(int a = 0; a < 3; ++a)
-                {
-                    if(sv[a] > 0.0f)
-                        tEnd = fminf(tEnd, (bl[a] + 8.0f - c0[a]) / sv[a]);
-                    else if(sv[a] < 0.0f)
-                        tEnd = fminf(tEnd, (bl[a] - c0[a]) / sv[a]);
-                }
-                // margin: 1e-3 steps plus the float rounding of tEnd itself
-                const float last = fminf(fmaxf(floorf(tEnd - (1.0e-3f + 1.0e-6f * fabsf(tEnd))), fi), fe);
+                const float last = last_step_in_brick(ax, ay, az, c0, sv, fi, fe);
                 fi = last + 1.0f;
                 continue;
             }

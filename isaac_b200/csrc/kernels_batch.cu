@@ -21,11 +21,11 @@ namespace isaacb
     {
         uchar4 col = to_byte4(c.bgSwizzled);
         float depth = FLT_MAX;
+        Ray ray = pixel_to_ray(v, c.g, px, py);
         const ShadeParams sp{c.renderMode, c.aoWeight, c.bg};
-        shade_values(sp, v, c.g, px, py, col, f3(0, 0, 0), 0.0f, depth);
+        shade_values(sp, c.g, ray.dir, col, f3(0, 0, 0), 0.0f, depth);
         if(!c.volume)
             return col;
-        Ray ray = pixel_to_ray(v, c.g, px, py);
         if(!clip_ray(ray, v, c.g))
             return col;
         ray.endDepth = gmin(ray.endDepth, depth);
@@ -39,10 +39,7 @@ namespace isaacb
             color = march_combined<LINEAR, false, SKIP, YFAST>(tex, m, factor, n);
         else
             color = march_combined<LINEAR, true, SKIP, YFAST>(tex, m, factor, n);
-        const float4 solid = from_byte4(col);
-        const float r = 1.0f - color.w;
-        color = make_float4(color.x + r * solid.x, color.y + r * solid.y, color.z + r * solid.z, color.w + r * solid.w);
-        return to_byte4(color);
+        return over_surface(color, col);
     }
 
     // 5 CTAs per SM (48 registers; the spills are outside the march): the march waits on

@@ -244,14 +244,14 @@ namespace isaacb
         if(px < p.v.W && py < p.v.H)
         {
             const size_t o = size_t(py) * p.v.W + px;
-            shade_pixel(p, px, py, o);
+            Ray ray = pixel_to_ray(p.v, p.g, px, py);
+            const float depth = shade_surface<false>(p, ray.dir, o);
             bool any = false;
             for(int s = 0; s < p.nVol; ++s)
                 any |= p.ps[s].weight != 0.0f;
-            Ray ray = pixel_to_ray(p.v, p.g, px, py);
             if(any && clip_ray(ray, p.v, p.g))
             {
-                ray.endDepth = gmin(ray.endDepth, p.depth[o]);
+                ray.endDepth = gmin(ray.endDepth, depth);
                 if(!(ray.endDepth <= ray.startDepth))
                 {
                     March m = march_setup(ray, p.g, p.v.scale, p.step);
@@ -283,12 +283,11 @@ namespace isaacb
                         if(color.w > 0.99f)
                             break;
                     }
-                    const float4 solid = from_byte4(p.color[o]);
-                    const float r = 1.0f - color.w;
-                    color = make_float4(color.x + r * solid.x, color.y + r * solid.y, color.z + r * solid.z, color.w + r * solid.w);
-                    p.color[o] = to_byte4(color);
+                    p.color[o] = over_surface(color, p.color[o]);
                 }
             }
+            if(p.out)
+                p.out[o] = p.color[o];
         }
         if(p.counters)
             count_warp(p.counters, n);
@@ -336,14 +335,14 @@ namespace isaacb
         if(px < p.v.W && py < p.v.H)
         {
             const size_t o = size_t(py) * p.v.W + px;
-            shade_pixel(p, px, py, o);
+            Ray ray = pixel_to_ray(p.v, p.g, px, py);
+            const float depth = shade_surface<false>(p, ray.dir, o);
             bool any = false;
             for(int s = 0; s < p.nVol; ++s)
                 any |= p.ps[s].weight != 0.0f;
-            Ray ray = pixel_to_ray(p.v, p.g, px, py);
             if(any && clip_ray(ray, p.v, p.g))
             {
-                ray.endDepth = gmin(ray.endDepth, p.depth[o]);
+                ray.endDepth = gmin(ray.endDepth, depth);
                 if(!(ray.endDepth <= ray.startDepth))
                 {
                     March m = march_setup(ray, p.g, p.v.scale, p.step);
@@ -409,12 +408,11 @@ namespace isaacb
                         if(color.w > 0.99f)
                             break;
                     }
-                    const float4 solid = from_byte4(p.color[o]);
-                    const float r = 1.0f - color.w;
-                    color = make_float4(color.x + r * solid.x, color.y + r * solid.y, color.z + r * solid.z, color.w + r * solid.w);
-                    p.color[o] = to_byte4(color);
+                    p.color[o] = over_surface(color, p.color[o]);
                 }
             }
+            if(p.out)
+                p.out[o] = p.color[o];
         }
         if(p.counters)
             count_warp(p.counters, n);
@@ -477,7 +475,8 @@ namespace isaacb
     // FP32 pairs.  Same operations in the same order per source, so the frame is
     // bit-identical to the general kernels'.
     // (4 CTAs per SM: 58 registers without spills, twice the warps of the unbounded 88)
-    template<int DT, bool LINEAR, int NS, bool IDEM>
+    // CLEAN: the frame's only pass; it clears the G-buffer instead of reading it
+    template<int DT, bool LINEAR, int NS, bool IDEM, bool CLEAN>
     __global__ void __launch_bounds__(256, 4) k_shade_volume_per_source_n(
         const __grid_constant__ FrameParams p,
         const __grid_constant__ ActiveSources act)
@@ -488,11 +487,11 @@ namespace isaacb
         if(px < p.v.W && py < p.v.H)
         {
             const size_t o = size_t(py) * p.v.W + px;
-            shade_pixel(p, px, py, o);
             Ray ray = pixel_to_ray(p.v, p.g, px, py);
+            const float depth = shade_surface<CLEAN>(p, ray.dir, o);
             if(clip_ray(ray, p.v, p.g))
             {
-                ray.endDepth = gmin(ray.endDepth, p.depth[o]);
+                ray.endDepth = gmin(ray.endDepth, depth);
                 if(!(ray.endDepth <= ray.startDepth))
                 {
                     March m = march_setup(ray, p.g, p.v.scale, p.step);
@@ -611,39 +610,61 @@ namespace isaacb
                     float4 color;
                     f2p_split(crg, color.x, color.y);
                     f2p_split(cba, color.z, color.w);
-                    const float4 solid = from_byte4(p.color[o]);
-                    const float r = 1.0f - color.w;
-                    color = make_float4(color.x + r * solid.x, color.y + r * solid.y, color.z + r * solid.z, color.w + r * solid.w);
-                    p.color[o] = to_byte4(color);
+                    p.color[o] = over_surface(color, p.color[o]);
                 }
             }
+            if(p.out)
+                p.out[o] = p.color[o];
         }
         if(p.counters)
             count_warp(p.counters, n);
     }
 
-    template<int DT, bool LINEAR, bool IDEM>
+    template<int DT, bool LINEAR, bool IDEM, bool CLEAN>
     void launch_ps_n(const FrameParams& p, const ActiveSources& act, dim3 grid, cudaStream_t s)
     {
         k_ps_premultiply<<<dim3((p.ts + 255) / 256, act.n), 256, 0, s>>>(p.lut, act, p.psPre, p.ts);
         switch(act.n)
         {
-        case 1: k_shade_volume_per_source_n<DT, LINEAR, 1, IDEM><<<grid, 256, 0, s>>>(p, act); break;
-        case 2: k_shade_volume_per_source_n<DT, LINEAR, 2, IDEM><<<grid, 256, 0, s>>>(p, act); break;
-        case 3: k_shade_volume_per_source_n<DT, LINEAR, 3, IDEM><<<grid, 256, 0, s>>>(p, act); break;
-        default: k_shade_volume_per_source_n<DT, LINEAR, 4, IDEM><<<grid, 256, 0, s>>>(p, act); break;
+        case 1: k_shade_volume_per_source_n<DT, LINEAR, 1, IDEM, CLEAN><<<grid, 256, 0, s>>>(p, act); break;
+        case 2: k_shade_volume_per_source_n<DT, LINEAR, 2, IDEM, CLEAN><<<grid, 256, 0, s>>>(p, act); break;
+        case 3: k_shade_volume_per_source_n<DT, LINEAR, 3, IDEM, CLEAN><<<grid, 256, 0, s>>>(p, act); break;
+        default: k_shade_volume_per_source_n<DT, LINEAR, 4, IDEM, CLEAN><<<grid, 256, 0, s>>>(p, act); break;
         }
     }
-    template<int DT>
+    template<int DT, bool CLEAN>
     void launch_ps_dt(const FrameParams& p, const ActiveSources& act, bool lin, bool idem, dim3 grid, cudaStream_t s)
     {
         if(lin)
-            idem ? launch_ps_n<DT, true, true>(p, act, grid, s) : launch_ps_n<DT, true, false>(p, act, grid, s);
+            idem ? launch_ps_n<DT, true, true, CLEAN>(p, act, grid, s) : launch_ps_n<DT, true, false, CLEAN>(p, act, grid, s);
         else
-            idem ? launch_ps_n<DT, false, true>(p, act, grid, s) : launch_ps_n<DT, false, false>(p, act, grid, s);
+            idem ? launch_ps_n<DT, false, true, CLEAN>(p, act, grid, s) : launch_ps_n<DT, false, false, CLEAN>(p, act, grid, s);
+    }
+    template<int DT>
+    void launch_ps_clean(const FrameParams& p, const ActiveSources& act, bool lin, bool idem, bool clean, dim3 grid, cudaStream_t s)
+    {
+        clean ? launch_ps_dt<DT, true>(p, act, lin, idem, grid, s) : launch_ps_dt<DT, false>(p, act, lin, idem, grid, s);
     }
 
-    int launch_shade_volume_per_source(const FrameParams& p, cudaStream_t s)
+    // whether launch_shade_volume_per_source takes the specialised kernel, which can clear:
+    // 1 to 4 weighted sources, all scalar, persistent and of one type, 32-bit slots
+    bool per_source_specialised(const FrameParams& p)
+    {
+        int dt = -1, n = 0;
+        for(int k = 0; k < p.nVol; ++k)
+        {
+            const PerSourceSrc& S = p.ps[k];
+            if(S.weight == 0.0f)
+                continue;
+            if(S.fdim != 1 || S.ncomp != 1 || !S.persistent || (dt >= 0 && dt != S.dtype))
+                return false;
+            dt = S.dtype;
+            ++n;
+        }
+        return n >= 1 && n <= 4 && size_t(p.g.nb[0]) * p.g.nb[1] * p.g.nb[2] * kSlotsPerBrick < (1ull << 31);
+    }
+
+    int launch_shade_volume_per_source(const FrameParams& p, bool clean, cudaStream_t s)
     {
         dim3 grid((p.v.W + 31) / 32, (p.v.H + 7) / 8);
         // the scalar kernel serves frames whose weighted sources are all scalar, persistent and of one type
@@ -675,16 +696,14 @@ namespace isaacb
                 act.n++;
                 idem = idem && S.chain.op[0] == OP_IDEM && S.chain.op[1] == OP_IDEM && S.chain.op[2] == OP_IDEM;
             }
-            // slot indices of the specialised kernel are 32-bit
-            const bool fits = size_t(p.g.nb[0]) * p.g.nb[1] * p.g.nb[2] * kSlotsPerBrick < (1ull << 31);
-            if(act.n >= 1 && act.n <= 4 && fits)
+            if(per_source_specialised(p))
             {
                 if(dt == 0)
-                    launch_ps_dt<0>(p, act, lin, idem, grid, s);
+                    launch_ps_clean<0>(p, act, lin, idem, clean, grid, s);
                 else if(dt == 1)
-                    launch_ps_dt<1>(p, act, lin, idem, grid, s);
+                    launch_ps_clean<1>(p, act, lin, idem, clean, grid, s);
                 else
-                    launch_ps_dt<2>(p, act, lin, idem, grid, s);
+                    launch_ps_clean<2>(p, act, lin, idem, clean, grid, s);
                 return 2;
             }
             if(dt == 0)

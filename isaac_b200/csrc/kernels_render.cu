@@ -12,8 +12,9 @@
 //                       lib/isaac/isaac_volume_kernel.hpp:23-88)
 //
 // The reference launches these six passes with a blocking wait after each;
-// here the per-pixel passes that need no neighbour are fused, so a frame is
-// two launches (four with iso surfaces and SSAO).
+// here the per-pixel passes that need no neighbour are fused and the first
+// one clears: a frame is one launch, and one more each with particles, iso
+// surfaces and SSAO.
 #include "isaacb_frame.cuh"
 #include "isaacb_march.cuh"
 
@@ -150,11 +151,7 @@ namespace isaacb
             return;
         const size_t o = pix(p, px, py);
         p.color[o] = to_byte4(p.bgSwizzled);
-        p.normal[3 * o] = 0.0f;
-        p.normal[3 * o + 1] = 0.0f;
-        p.normal[3 * o + 2] = 0.0f;
-        p.depth[o] = FLT_MAX;
-        p.ao[o] = 0.0f;
+        store_clear(p, o, FLT_MAX);
         if(p.nPart > 0)
             particle_pixel(p, px, py);
     }
@@ -253,7 +250,8 @@ namespace isaacb
     // in the reference.  So hit, depth, colour and normal follow the reference's float
     // operations exactly.
     constexpr float kIsoMargin = 0.125f; // alpha bytes
-    template<bool LINEAR, bool YFAST>
+    // CLEAN: the first pass of its frame, which clears the G-buffer where nothing is hit.
+    template<bool LINEAR, bool YFAST, bool CLEAN>
     __global__ void __launch_bounds__(256) k_iso(const __grid_constant__ FrameParams p)
     {
         int px, py;
@@ -263,9 +261,14 @@ namespace isaacb
         {
             Ray ray = pixel_to_ray(p.v, p.g, px, py);
             const size_t o = pix(p, px, py);
+            if(CLEAN)
+            {
+                p.color[o] = to_byte4(p.bgSwizzled);
+                store_clear(p, o, FLT_MAX);
+            }
             if(clip_ray(ray, p.v, p.g))
             {
-                ray.endDepth = gmin(ray.endDepth, p.depth[o]);
+                ray.endDepth = gmin(ray.endDepth, CLEAN ? FLT_MAX : p.depth[o]);
                 if(!(ray.endDepth <= ray.startDepth))
                 {
                     const March m = march_setup(ray, p.g, p.v.scale, p.step);
@@ -341,13 +344,18 @@ namespace isaacb
             count_samples(p.counters + 1, n);
     }
 
-    void launch_iso(const FrameParams& p, cudaStream_t s)
+    template<bool LINEAR, bool YFAST>
+    void launch_iso_as(const FrameParams& p, bool clean, cudaStream_t s)
     {
-        dim3 grid((p.v.W + 31) / 32, (p.v.H + 7) / 8);
+        const dim3 grid((p.v.W + 31) / 32, (p.v.H + 7) / 8);
+        clean ? k_iso<LINEAR, YFAST, true><<<grid, 256, 0, s>>>(p) : k_iso<LINEAR, YFAST, false><<<grid, 256, 0, s>>>(p);
+    }
+    void launch_iso(const FrameParams& p, bool clean, cudaStream_t s)
+    {
         if(p.interpolation)
-            p.g.yfast ? k_iso<true, true><<<grid, 256, 0, s>>>(p) : k_iso<true, false><<<grid, 256, 0, s>>>(p);
+            p.g.yfast ? launch_iso_as<true, true>(p, clean, s) : launch_iso_as<true, false>(p, clean, s);
         else
-            p.g.yfast ? k_iso<false, true><<<grid, 256, 0, s>>>(p) : k_iso<false, false><<<grid, 256, 0, s>>>(p);
+            p.g.yfast ? launch_iso_as<false, true>(p, clean, s) : launch_iso_as<false, false>(p, clean, s);
     }
 
     // ------------------------------------------------------------------ SSAO
@@ -445,7 +453,8 @@ namespace isaacb
     // axis keep along y.  Against rows of 4 lanes for y-fastest slots that is 5.9 instead of
     // 10.7 cycles a load (a count over sampled warps that gives the 10.6 ncu showed), and
     // the 4 x 512^3 march at 1920x1080 3.46 -> 3.24 ms, at 960x540 0.73 -> 0.63 ms.
-    template<bool VOLUME, bool LINEAR, bool FULL, bool YFAST>
+    // CLEAN: the frame's only pass; it clears the G-buffer instead of reading it
+    template<bool VOLUME, bool LINEAR, bool FULL, bool YFAST, bool CLEAN>
     __global__ void __launch_bounds__(kShadeThreads, FULL ? 2048 / kShadeThreads : kLongMinBlocks) k_shade_volume(const __grid_constant__ FrameParams p)
     {
         // empty-space skipping only pays when the texture has empty bricks; the merge that
@@ -460,54 +469,55 @@ namespace isaacb
         if(px < p.v.W && py < p.v.H)
         {
             const size_t o = pix(p, px, py);
-            shade_pixel(p, px, py, o);
-            if(VOLUME)
+            Ray ray = pixel_to_ray(p.v, p.g, px, py);
+            const float depth = shade_surface<CLEAN>(p, ray.dir, o);
+            if(VOLUME && clip_ray(ray, p.v, p.g))
             {
-                Ray ray = pixel_to_ray(p.v, p.g, px, py);
-                if(clip_ray(ray, p.v, p.g))
+                ray.endDepth = gmin(ray.endDepth, depth);
+                if(!(ray.endDepth <= ray.startDepth))
                 {
-                    ray.endDepth = gmin(ray.endDepth, p.depth[o]);
-                    if(!(ray.endDepth <= ray.startDepth))
-                    {
-                        const March m = march_setup(ray, p.g, p.v.scale, p.step);
-                        const float factor = m.factor * p.totalWeightAll;
-                        float4 color;
-                        const VolTexRef tex{p.g, p.volQ, p.volFlag};
-                        if(LINEAR && march_in_range(p.g, m))
-                            color = skip ? march_combined<LINEAR, false, true, YFAST>(tex, m, factor, n)
-                                         : march_combined<LINEAR, false, false, YFAST>(tex, m, factor, n);
-                        else
-                            color = skip ? march_combined<LINEAR, true, true, YFAST>(tex, m, factor, n)
-                                         : march_combined<LINEAR, true, false, YFAST>(tex, m, factor, n);
-                        const float4 solid = from_byte4(p.color[o]);
-                        const float r = 1.0f - color.w;
-                        color = make_float4(color.x + r * solid.x, color.y + r * solid.y, color.z + r * solid.z, color.w + r * solid.w);
-                        p.color[o] = to_byte4(color);
-                    }
+                    const March m = march_setup(ray, p.g, p.v.scale, p.step);
+                    const float factor = m.factor * p.totalWeightAll;
+                    float4 color;
+                    const VolTexRef tex{p.g, p.volQ, p.volFlag};
+                    if(LINEAR && march_in_range(p.g, m))
+                        color = skip ? march_combined<LINEAR, false, true, YFAST>(tex, m, factor, n)
+                                     : march_combined<LINEAR, false, false, YFAST>(tex, m, factor, n);
+                    else
+                        color = skip ? march_combined<LINEAR, true, true, YFAST>(tex, m, factor, n)
+                                     : march_combined<LINEAR, true, false, YFAST>(tex, m, factor, n);
+                    p.color[o] = over_surface(color, p.color[o]);
                 }
             }
+            if(p.out)
+                p.out[o] = p.color[o];
         }
         if(VOLUME && p.counters)
             count_samples(p.counters, n);
     }
 
-    template<bool FULL, bool YFAST>
+    template<bool FULL, bool YFAST, bool CLEAN>
     void launch_shade_volume_as(const FrameParams& p, bool volume, cudaStream_t s)
     {
         constexpr int TW = shade_tile_w(FULL, YFAST), TH = shade_tile_h(FULL, YFAST);
         const dim3 grid((p.v.W + TW - 1) / TW, (p.v.H + TH - 1) / TH);
         if(!volume)
-            k_shade_volume<false, false, FULL, YFAST><<<grid, kShadeThreads, 0, s>>>(p);
+            k_shade_volume<false, false, FULL, YFAST, CLEAN><<<grid, kShadeThreads, 0, s>>>(p);
         else if(p.interpolation)
-            k_shade_volume<true, true, FULL, YFAST><<<grid, kShadeThreads, 0, s>>>(p);
+            k_shade_volume<true, true, FULL, YFAST, CLEAN><<<grid, kShadeThreads, 0, s>>>(p);
         else
-            k_shade_volume<true, false, FULL, YFAST><<<grid, kShadeThreads, 0, s>>>(p);
+            k_shade_volume<true, false, FULL, YFAST, CLEAN><<<grid, kShadeThreads, 0, s>>>(p);
+    }
+    template<bool FULL, bool YFAST>
+    void launch_shade_volume_clean(const FrameParams& p, bool volume, bool clean, cudaStream_t s)
+    {
+        clean ? launch_shade_volume_as<FULL, YFAST, true>(p, volume, s) : launch_shade_volume_as<FULL, YFAST, false>(p, volume, s);
     }
 
     // launches of fewer than this many waves of the uncapped form take the FULL form
     constexpr int kShadeShortWaves = 4;
 
-    void launch_shade_volume(const FrameParams& p, bool volume, cudaStream_t s)
+    void launch_shade_volume(const FrameParams& p, bool volume, bool clean, cudaStream_t s)
     {
         const long long blocks = (long long) ((p.v.W + shade_tile_w(false) - 1) / shade_tile_w(false))
             * ((p.v.H + shade_tile_h(false) - 1) / shade_tile_h(false));
@@ -520,14 +530,14 @@ namespace isaacb
         {
             int sms = 0, perSm = 0;
             cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, k_shade_volume<true, true, false, false>, kShadeThreads, 0);
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, k_shade_volume<true, true, false, false, false>, kShadeThreads, 0);
             resident[dev] = std::max(1, sms * perSm);
         }
         const long long waves = blocks / std::max(1, dev >= 0 && dev < 64 ? resident[dev] : 1);
         const bool full = volume && waves < kShadeShortWaves;
         if(p.g.yfast)
-            full ? launch_shade_volume_as<true, true>(p, volume, s) : launch_shade_volume_as<false, true>(p, volume, s);
+            full ? launch_shade_volume_clean<true, true>(p, volume, clean, s) : launch_shade_volume_clean<false, true>(p, volume, clean, s);
         else
-            full ? launch_shade_volume_as<true, false>(p, volume, s) : launch_shade_volume_as<false, false>(p, volume, s);
+            full ? launch_shade_volume_clean<true, false>(p, volume, clean, s) : launch_shade_volume_clean<false, false>(p, volume, clean, s);
     }
 } // namespace isaacb
