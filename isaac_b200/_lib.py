@@ -246,5 +246,14 @@ def check(status: int, ctx=None) -> int:
     return status
 
 
+def current_stream() -> C.c_void_p:
+    """The current CUDA stream's handle.  The raw query costs a tenth of building the
+    ``torch.cuda.Stream`` object that ``torch.cuda.current_stream()`` returns (4 us, a
+    sixth of what a small frame's host side takes)."""
+    import torch
+
+    return C.c_void_p(torch._C._cuda_getCurrentRawStream(torch.cuda.current_device()))
+
+
 def lib_path() -> Path:
     return _build.LIB

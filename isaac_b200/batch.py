@@ -70,7 +70,7 @@ class IsaacBatch:
 
     @staticmethod
     def _stream():
-        return C.c_void_p(_torch().cuda.current_stream().cuda_stream)
+        return _lib.current_stream()
 
     # ------------------------------------------------------------------ settings
     @property

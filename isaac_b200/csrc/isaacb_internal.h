@@ -3,6 +3,7 @@
 #pragma once
 
 #include <algorithm>
+#include <atomic>
 
 #include "isaacb_device.cuh"
 
@@ -63,6 +64,36 @@ namespace isaacb
         n = std::min(n, thrSm / (warps * 32));
         return std::max(1, std::min(n, 4));
     }
+
+    // What a launcher asks the runtime about one kernel, asked once per device: the SM count
+    // and the CTAs per SM for one amount of dynamic shared memory (the last one asked for),
+    // after the opt-in to `optIn` bytes of it.  One atomic word per device, so that any
+    // thread may launch.  The queries took 10 us of a small frame's 27 us of host time.
+    struct LaunchCache
+    {
+        std::atomic<uint64_t> word[64]{}; // bytes << 16 | CTAs per SM << 12 | SMs, 0: not asked
+        template<class K>
+        void get(K kernel, int threads, size_t dynSmem, size_t optIn, int& sms, int& perSm)
+        {
+            int dev = 0;
+            cudaGetDevice(&dev);
+            std::atomic<uint64_t>* w = dev >= 0 && dev < 64 ? &word[dev] : nullptr;
+            const uint64_t have = w ? w->load(std::memory_order_relaxed) : 0;
+            if(have != 0 && (have >> 16) == dynSmem)
+            {
+                sms = int(have & 0xFFFu);
+                perSm = int((have >> 12) & 15u);
+                return;
+            }
+            if(optIn > 48 * 1024)
+                cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(optIn));
+            sms = 148;
+            cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+            perSm = ctas_per_sm(kernel, threads, dynSmem);
+            if(w && sms > 0 && sms < 0x1000 && perSm < 16)
+                w->store(uint64_t(dynSmem) << 16 | uint64_t(perSm) << 12 | uint64_t(sms), std::memory_order_relaxed);
+        }
+    };
 
     // returns the number of kernels it launched
     int launch_merge(const MergeParams& p, cudaStream_t s);

@@ -587,15 +587,10 @@ namespace isaacb
     void launch_rows(const MergeParams& p, const MergeRows& act, cudaStream_t s)
     {
         const size_t bytes = rows_table_bytes(act, p.ts);
-        // the opt-in to more than 48 KiB of dynamic shared memory, once per device
-        static uint64_t configured = 0;
-        int dev = 0, sms = 148;
-        cudaGetDevice(&dev);
-        if(dev < 64 && !((configured >> dev) & 1u)
-           && cudaFuncSetAttribute(k_merge_rows<ISO, NS, FD>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kRowsSmem)) == cudaSuccess)
-            configured |= uint64_t(1) << dev;
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        const size_t resident = size_t(sms) * ctas_per_sm(k_merge_rows<ISO, NS, FD>, kRowsThreads, bytes);
+        static LaunchCache cache;
+        int sms, perSm;
+        cache.get(k_merge_rows<ISO, NS, FD>, kRowsThreads, bytes, kRowsSmem, sms, perSm);
+        const size_t resident = size_t(sms) * perSm;
         const size_t wanted = (size_t(act.voxels) + kRowsThreads * kRowsPer - 1) / (kRowsThreads * kRowsPer);
         k_merge_rows<ISO, NS, FD><<<unsigned(std::max<size_t>(1, std::min(resident, wanted))), kRowsThreads, bytes, s>>>(p, act);
     }
@@ -865,16 +860,10 @@ namespace isaacb
     template<int NS>
     void launch_x4_smem(const MergeParams& p, const MergeActive& act, size_t quads, size_t tableBytes, cudaStream_t s)
     {
-        // the opt-in to more than 48 KiB of dynamic shared memory, once per device
-        static uint64_t configured = 0;
-        int dev = 0, sms = 148;
-        cudaGetDevice(&dev);
-        if(dev < 64 && !((configured >> dev) & 1u)
-           && cudaFuncSetAttribute(k_merge_voxels_x4_smem<NS>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kMergeSmemTables))
-               == cudaSuccess)
-            configured |= uint64_t(1) << dev;
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        const size_t resident = size_t(sms) * ctas_per_sm(k_merge_voxels_x4_smem<NS>, 512, tableBytes);
+        static LaunchCache cache;
+        int sms, perSm;
+        cache.get(k_merge_voxels_x4_smem<NS>, 512, tableBytes, kMergeSmemTables, sms, perSm);
+        const size_t resident = size_t(sms) * perSm;
         const size_t grid = std::max<size_t>(1, std::min(resident, (quads + 511) / 512));
         k_merge_voxels_x4_smem<NS><<<unsigned(grid), 512, tableBytes, s>>>(p, act);
     }

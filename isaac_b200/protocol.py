@@ -57,9 +57,7 @@ FUNCTORS = [
 
 
 def _stream_ptr():
-    import torch
-
-    return C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    return _lib.current_stream()
 
 
 class FrameEncoder:

@@ -36,7 +36,7 @@ def _torch():
 
 
 def _stream():
-    return C.c_void_p(_torch().cuda.current_stream().cuda_stream)
+    return _lib.current_stream()
 
 
 def psnr_from_sq(sq: float, nbytes: int) -> float:

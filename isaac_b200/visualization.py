@@ -534,7 +534,7 @@ class IsaacVisualization:
                 self._srcPtrs[i] = ptr
 
     def _stream(self):
-        return C.c_void_p(_torch().cuda.current_stream().cuda_stream)
+        return _lib.current_stream()
 
     def doVisualization(self, pointer=None, redraw: bool = True, host: bool = True, out=None, timing: bool = False):
         """One frame: the sources' ``update`` hooks, buffer update, draw and readback
