@@ -643,15 +643,18 @@ namespace
     // than the image x axis to the volume's x.  Counted over sampled warps of a 512^3 volume
     // at 1920x1080 (L1 cycles a load, x / y fastest): pitch 20 degrees 5.7 / 5.9 at yaw 0,
     // 7.5 / 6.1 at 30, 12.8 / 6.2 at 45, 14.5 / 5.9 at 90; pitch 34 degrees 7.0 / 10.9 at yaw
-    // 30, 11.8 / 10.5 at 45.  On textures that L2 holds much of the choice is left at x
-    // fastest: for the full-feature scene (256^3, 0.33 GB) y fastest costs its pixel passes
-    // more than it gains.  Only the speed depends on it: both orders hold the same texels.
+    // 30, 11.8 / 10.5 at 45.  Where L2 holds much of the texture and the frame fills the SMs
+    // the choice is left at x fastest: for the full-feature scene (256^3, 0.33 GB, 1920x1080)
+    // y fastest costs its pixel passes more than it gains (shading and march 236 us against
+    // 252), while small frames gain (500x300 over 128^3: 115 -> 92 us at yaw 60).  Only the
+    // speed depends on it: both orders hold the same texels.
     int32_t slot_order_for_camera(const isaacb_ctx* c)
     {
         if(c->slotOrder >= 0)
             return c->slotOrder;
         const double textureBytes = double(brick_count(c->g)) * kSlotsPerBrick * sizeof(uint4);
-        if(textureBytes < 4.0 * 126.0e6)
+        const long long warps = (long long) ((c->desc.framebuffer[0] + 7) / 8) * ((c->desc.framebuffer[1] + 3) / 4);
+        if(textureBytes < 4.0 * 126.0e6 && warps > 148 * 64)
             return 0;
         // rows 0 and 1 of the column-major modelview: the image axes in volume coordinates
         const double ix[3] = {c->mv[0], c->mv[4], c->mv[8]}, iy[3] = {c->mv[1], c->mv[5], c->mv[9]};
@@ -1886,6 +1889,7 @@ namespace
         bp.tileH = int32_t(b->cfg.tile_h);
         bp.counter = b->counter;
         bp.samples = b->counting ? b->samples : nullptr;
+        bp.negZero = -0.0f;
         if(b->counting && cudaMemsetAsync(b->samples, 0, sizeof(unsigned long long), st) != cudaSuccess)
             return batch_fail(ISAACB_CUDA_ERROR, "isaacb_batch: sample counter reset");
         launch_batch(bp, batch_blocks(b), st);

@@ -690,6 +690,19 @@ namespace isaacb
         asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
         return r;
     }
+    __device__ __forceinline__ f2p f2p_sub(f2p a, f2p b)
+    {
+        f2p r;
+        asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+        return r;
+    }
+    // a + b rounded toward minus infinity per lane (__fadd_rd)
+    __device__ __forceinline__ f2p f2p_add_rd(f2p a, f2p b)
+    {
+        f2p r;
+        asm("add.rm.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+        return r;
+    }
     // a * b rounded once, for a product that feeds an add.  The assembler contracts
     // mul.rn.f32x2 followed by add.rn.f32x2 into one fma.rn.f32x2 (the explicit rounding
     // does not stop it for the packed forms, as it does for mul.rn.f32), which rounds

@@ -126,8 +126,7 @@ namespace isaacb
     // Shades pixel o in place along its ray direction and returns its depth.  CLEAN: no pass
     // has drawn a surface, so that the pixel has the clear values, which are written here
     // instead of by a pass of their own.  The results go to memory rather than stay in
-    // registers, of which the march that follows needs every one (3.24 ms at 46 registers,
-    // 3.40 at 52).
+    // registers, of which the march that follows needs every one.
     template<bool CLEAN>
     __device__ __forceinline__ float shade_surface(const FrameParams& p, float3 dir, size_t o)
     {

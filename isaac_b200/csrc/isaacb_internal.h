@@ -287,6 +287,7 @@ namespace isaacb
         int32_t tileW, tileH; // tileW * tileH == 256, tileW % 8 == 0, tileH % 4 == 0
         int32_t* counter; // work queue head, zero before the launch
         unsigned long long* samples; // optional sample counter
+        float negZero; // -0.0f (f2p_mul_exact)
     };
     void launch_batch(const BatchParams& p, int blocks, cudaStream_t s);
     int batch_max_blocks_per_sm();

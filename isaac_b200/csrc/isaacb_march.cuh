@@ -12,39 +12,8 @@ namespace isaacb
         Geom g;
         const uint4* volQ;
         const uint8_t* volFlag;
+        float negZero; // -0.0f from a kernel parameter (f2p_mul_exact), for march_ahead
     };
-
-    // the trilinear sample of channel-major slots A (plane z0) and B (plane z0 + 1) at the
-    // fractional position (fx, fy, fz), in units of 1/65535 byte: an exact integer sum of
-    // 16-bit fixed-point weights times bytes
-    __device__ __forceinline__ float4 trilinear_dp2a(uint4 A, uint4 B, float fx, float fy, float fz)
-    {
-        constexpr float kUnit = 65535.0f;
-        const float gx = 1.0f - fx, gy = 1.0f - fy;
-        const float fzU = fz * kUnit, gzU = kUnit - fzU;
-        // the xy weights of a texel row as packed pairs (texel x0, texel x0 + 1):
-        // (w00, w10) = (gx, fx) * gy and (w01, w11) = (gx, fx) * fy
-        const f2p X = f2p_make(gx, fx);
-        const f2p R0 = f2p_mul(X, f2p_make(gy, gy)), R1 = f2p_mul(X, f2p_make(fy, fy));
-        // round(w * 65535) lands in the low bits of 2^23 + w * 65535 (one rounding per lane,
-        // to nearest, as the scalar fmaf); <= 65535, so the low 16 bits are the weight
-        const f2p M = f2p_make(8388608.0f, 8388608.0f), GZ = f2p_make(gzU, gzU), FZ = f2p_make(fzU, fzU);
-        auto pack = [](f2p q) {
-            float lo, hi;
-            f2p_split(q, lo, hi);
-            return __byte_perm(__float_as_uint(lo), __float_as_uint(hi), 0x5410u);
-        };
-        // weight pairs (texel (x0,y) | texel (x0+1,y) << 16) for rows y0 and y0+1 of each plane
-        const uint32_t W0a = pack(f2p_fma(R0, GZ, M));
-        const uint32_t W1a = pack(f2p_fma(R1, GZ, M));
-        const uint32_t W0b = pack(f2p_fma(R0, FZ, M));
-        const uint32_t W1b = pack(f2p_fma(R1, FZ, M));
-        // Σ weights <= 65535 + 4, so every channel sum is an exact integer below 2^24
-        auto tri = [&](uint32_t a, uint32_t b) {
-            return __uint2float_rn(dp2a_hi(W1b, b, dp2a_lo(W0b, b, dp2a_hi(W1a, a, dp2a_lo(W0a, a, 0u)))));
-        };
-        return make_float4(tri(A.x, B.x), tri(A.y, B.y), tri(A.z, B.z), tri(A.w, B.w));
-    }
 
     // the last step index, at least fi and at most fe, whose position c0 + sv * i stays inside
     // the sample region [8b-1, 8b+7) of the brick of apron-shifted texel (ax, ay, az)
@@ -64,6 +33,54 @@ namespace isaacb
         return fminf(fmaxf(floorf(tEnd - (1.0e-3f + 1.0e-6f * fabsf(tEnd))), fi), fe);
     }
 
+    // a slot's load that stays where it is written: the compiler moves an ordinary one past
+    // the exits between the samples of a trip, next to its use, and nothing is ahead any more
+    __device__ __forceinline__ uint4 load_slot_here(const uint4* at)
+    {
+        uint4 v;
+        asm volatile("ld.global.nc.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(at));
+        return v;
+    }
+
+    // the weight words of two samples at once, one per packed lane, at the fractional
+    // positions (fx, fy, fz): w[l][0..3] are lane l's 16-bit fixed-point weight pairs
+    // (texel x0 | texel x0 + 1 << 16) of rows y0 and y0 + 1 of plane z0, then of z0 + 1.
+    // With the samples in the lanes every product of the chain is packed and no weight has
+    // to be broadcast into a pair; each lane rounds like the scalar operations.
+    __device__ __forceinline__ void trilinear_weights2(f2p fx, f2p fy, f2p fz, f2p negZero, uint32_t (&w)[2][4])
+    {
+        constexpr float kUnit = 65535.0f;
+        const f2p one = f2p_make(1.0f, 1.0f), unit = f2p_make(kUnit, kUnit);
+        const f2p gx = f2p_sub(one, fx), gy = f2p_sub(one, fy);
+        // a product that feeds a subtraction: rounded on its own (f2p_mul_exact)
+        const f2p fzU = f2p_mul_exact(fz, unit, negZero), gzU = f2p_sub(unit, fzU);
+        const f2p r[4] = {f2p_mul(gx, gy), f2p_mul(fx, gy), f2p_mul(gx, fy), f2p_mul(fx, fy)};
+        // round(w * 65535) lands in the low bits of 2^23 + w * 65535 (one rounding per lane,
+        // to nearest, as the scalar fmaf); <= 65535, so the low 16 bits are the weight
+        const f2p M = f2p_make(8388608.0f, 8388608.0f);
+#pragma unroll
+        for(int q = 0; q < 4; ++q)
+        {
+            const f2p z = q < 2 ? gzU : fzU;
+            float a0, a1, b0, b1;
+            f2p_split(f2p_fma(r[2 * (q & 1)], z, M), a0, a1);
+            f2p_split(f2p_fma(r[2 * (q & 1) + 1], z, M), b0, b1);
+            w[0][q] = __byte_perm(__float_as_uint(a0), __float_as_uint(b0), 0x5410u);
+            w[1][q] = __byte_perm(__float_as_uint(a1), __float_as_uint(b1), 0x5410u);
+        }
+    }
+
+    // the trilinear sample of channel-major slots A (plane z0) and B (plane z0 + 1) with the
+    // weight words w, in units of 1/65535 byte: an exact integer sum of 16-bit fixed-point
+    // weights times bytes (the weights sum to at most 65535 + 4, so it stays below 2^24)
+    __device__ __forceinline__ float4 trilinear_dp2a(uint4 A, uint4 B, const uint32_t (&w)[4])
+    {
+        auto tri = [&](uint32_t a, uint32_t b) {
+            return __uint2float_rn(dp2a_hi(w[3], b, dp2a_lo(w[2], b, dp2a_hi(w[1], a, dp2a_lo(w[0], a, 0u)))));
+        };
+        return make_float4(tri(A.x, B.x), tri(A.y, B.y), tri(A.z, B.z), tri(A.w, B.w));
+    }
+
     // Front-to-back march of CombinedVolumeRenderKernel (lib/isaac/isaac_volume_kernel.hpp:61-87)
     // at the reference's sample positions.  Differences from the exact form, all far
     // below one output LSB and covered by the parity tests:
@@ -81,7 +98,14 @@ namespace isaacb
     // last sample lie strictly inside needs no per-sample clamp (positions are affine
     // in the step index, rounding is far below the 1e-3 margin).
     // YFAST: the texture's slots are y fastest (Geom::yfast), else x fastest.
-    template<bool LINEAR, bool CLAMP, bool SKIP, bool YFAST = false>
+    //
+    // A trip takes 2 * PAIRS samples, all their slots loading before any is weighed.  Two
+    // consecutive samples are the two lanes of every packed position and weight operation
+    // (f32x2); they are composited one after the other, in order, and a sample past the last
+    // step or the opacity limit takes the factor 0 and adds exactly nothing.  There is no
+    // branch between a trip's samples: with one, the compiler moved each sample's loads
+    // behind it and a ray waited for every sample's loads in turn.
+    template<bool LINEAR, bool CLAMP, bool SKIP, bool YFAST, int PAIRS>
     __device__ __forceinline__ float4 march_combined(
         const VolTexRef& p,
         const March& m,
@@ -102,29 +126,64 @@ namespace isaacb
         // the slot of apron-shifted coordinates as a sum over the axes: with b = a >> 3 and
         // l = a & 7 per axis, b * stride + l * step == a * step + b * (stride - 8 * step);
         // the in-brick steps of x and y are (1, 8), or (8, 1) for y-fastest slots
-        constexpr uint32_t stepX = YFAST ? 8u : 1u, stepY = YFAST ? 1u : 8u;
+        constexpr uint32_t stepX = YFAST ? 8u : 1u, stepY = YFAST ? 1u : 8u, kx = 576u - 8u * stepX;
         const uint32_t sy = uint32_t(nb0) * uint32_t(kSlotsPerBrick) - 8u * stepY;
         const uint32_t sz = uint32_t(nb1) * uint32_t(nb0) * uint32_t(kSlotsPerBrick) - 512u;
-        // floor(c) + 1 (the apron-shifted coordinate) straight from the magic-number add
-        const int magic = 0x4B400000 - 1;
-        float4 color = make_float4(0, 0, 0, 0);
+        // floor(c) + 1, the apron-shifted coordinate a, by a round-down add of 1.5 * 2^23 + 1:
+        // the sum's bits are kBits + a, and kBits is a multiple of 8, so bits >> 3 is
+        // (kBits >> 3) + (a >> 3) and the constants leave the slot as one offset (mod 2^32)
+        constexpr float kFloor = 12582913.0f;
+        constexpr uint32_t kBits = 0x4B400000u;
+        const uint32_t slot0 = 0u - (stepX + stepY + 64u) * kBits - (kx + sy + sz) * (kBits >> 3);
+        const f2p sv2[3] = {f2p_make(svx, svx), f2p_make(svy, svy), f2p_make(svz, svz)};
+        const f2p c02[3] = {f2p_make(c0x, c0x), f2p_make(c0y, c0y), f2p_make(c0z, c0z)};
+        const f2p floor2 = f2p_make(kFloor, kFloor), nz = f2p_make(p.negZero, p.negZero);
+        f2p rg = f2p_make(0.0f, 0.0f), ba = rg; // colour so far: (red, green), (blue, alpha)
+        float alpha = 0.0f;
         int curBrick = -1;
         bool empty = false;
         const float fs = float(m.startSteps), fe = float(m.endSteps);
         float fi = fs;
         while(fi <= fe)
         {
-            float cx = fmaf(svx, fi, c0x), cy = fmaf(svy, fi, c0y), cz = fmaf(svz, fi, c0z);
-            if(CLAMP)
+            f2p fr[PAIRS][3];
+            uint32_t slot[2 * PAIRS];
+            int brick = 0, ax = 0, ay = 0, az = 0; // of the first sample
+#pragma unroll
+            for(int q = 0; q < PAIRS; ++q)
             {
-                cx = fminf(fmaxf(cx, lo), hx);
-                cy = fminf(fmaxf(cy, lo), hy);
-                cz = fminf(fmaxf(cz, lo), hz);
+                const f2p fq = f2p_make(q == 0 ? fi : fminf(fi + float(2 * q), fe), fminf(fi + float(2 * q + 1), fe));
+                uint32_t tb[3][2];
+#pragma unroll
+                for(int a = 0; a < 3; ++a)
+                {
+                    f2p c = f2p_fma(sv2[a], fq, c02[a]);
+                    if(CLAMP)
+                    {
+                        const float h = a == 0 ? hx : a == 1 ? hy : hz;
+                        float u, v;
+                        f2p_split(c, u, v);
+                        c = f2p_make(fminf(fmaxf(u, lo), h), fminf(fmaxf(v, lo), h));
+                    }
+                    const f2p t = f2p_add_rd(c, floor2);
+                    fr[q][a] = f2p_sub(c, f2p_sub(t, floor2));
+                    float t0, t1;
+                    f2p_split(t, t0, t1);
+                    tb[a][0] = __float_as_uint(t0);
+                    tb[a][1] = __float_as_uint(t1);
+                }
+#pragma unroll
+                for(int l = 0; l < 2; ++l)
+                    slot[2 * q + l] = (tb[0][l] >> 3) * kx + (tb[0][l] * stepX + slot0) + ((tb[1][l] >> 3) * sy + tb[1][l] * stepY)
+                        + ((tb[2][l] >> 3) * sz + tb[2][l] * 64u);
+                if(SKIP && q == 0)
+                {
+                    ax = int(tb[0][0] - kBits), ay = int(tb[1][0] - kBits), az = int(tb[2][0] - kBits);
+                    brick = ((az >> 3) * nb1 + (ay >> 3)) * nb0 + (ax >> 3);
+                }
             }
-            const float tx = __fadd_rd(cx, 12582912.0f), ty = __fadd_rd(cy, 12582912.0f),
-                        tz = __fadd_rd(cz, 12582912.0f);
-            const int ax = __float_as_int(tx) - magic, ay = __float_as_int(ty) - magic, az = __float_as_int(tz) - magic;
-            const int brick = SKIP ? ((az >> 3) * nb1 + (ay >> 3)) * nb0 + (ax >> 3) : 0;
+            // an empty brick under the first sample of the trip ends it; a later sample of
+            // the trip in one is weighed and adds exactly zero
             if(SKIP && brick != curBrick)
             {
                 curBrick = brick;
@@ -138,33 +197,47 @@ namespace isaacb
                 fi = last + 1.0f;
                 continue;
             }
-            const uint32_t slot = stepX * uint32_t(ax) + (576u - 8u * stepX) * uint32_t(ax >> 3) + stepY * uint32_t(ay)
-                + sy * uint32_t(ay >> 3) + 64u * uint32_t(az) + sz * uint32_t(az >> 3);
-            float r0, r1, r2, r3;
+            // channel-major slots: A.c / B.c = channel c of the 2x2 texels of planes z0 / z0+1
+            uint4 A[2 * PAIRS], B[2 * PAIRS];
+#pragma unroll
+            for(int j = 0; j < 2 * PAIRS; ++j)
+            {
+                A[j] = load_slot_here(p.volQ + slot[j]);
+                if(LINEAR)
+                    B[j] = load_slot_here(p.volQ + slot[j] + 64);
+            }
+            uint32_t w[PAIRS][2][4];
             if(LINEAR)
+#pragma unroll
+                for(int q = 0; q < PAIRS; ++q)
+                    trilinear_weights2(fr[q][0], fr[q][1], fr[q][2], nz, w[q]);
+            // a sample past the last step or the opacity limit takes the factor 0 and adds
+            // exactly nothing: no branch parts the trip's loads from their uses
+            bool done = false;
+#pragma unroll
+            for(int j = 0; j < 2 * PAIRS; ++j)
             {
-                // channel-major slots: A.c / B.c = channel c of the 2x2 texels of planes z0 / z0+1
-                const uint4 A = __ldg(p.volQ + slot);
-                const uint4 B = __ldg(p.volQ + slot + 64);
-                const float4 r = trilinear_dp2a(A, B, cx - (tx - 12582912.0f), cy - (ty - 12582912.0f), cz - (tz - 12582912.0f));
-                r0 = r.x, r1 = r.y, r2 = r.z, r3 = r.w;
+                float4 r;
+                if(LINEAR)
+                    r = trilinear_dp2a(A[j], B[j], w[j >> 1][j & 1]);
+                else // texel (x0, y0) of the slot: byte 0 of each channel word
+                    r = make_float4(ubyte_f(A[j].x, 0), ubyte_f(A[j].y, 0), ubyte_f(A[j].z, 0), ubyte_f(A[j].w, 0));
+                const bool take = j == 0 || (!done && fi <= fe);
+                const float s = take ? (1.0f - alpha) * kS : 0.0f;
+                rg = f2p_fma(f2p_make(s, s), f2p_make(r.x, r.y), rg);
+                ba = f2p_fma(f2p_make(s, s), f2p_make(r.z, r.w), ba);
+                float blue;
+                f2p_split(ba, blue, alpha);
+                fi += take ? 1.0f : 0.0f;
+                done = done || alpha > 0.99f;
             }
-            else
-            {
-                // texel (x0, y0) of the slot: byte 0 of each channel word
-                const uint4 Q = __ldg(p.volQ + slot);
-                r0 = ubyte_f(Q.x, 0), r1 = ubyte_f(Q.y, 0), r2 = ubyte_f(Q.z, 0), r3 = ubyte_f(Q.w, 0);
-            }
-            const float s = (1.0f - color.w) * kS;
-            color.x = fmaf(s, r0, color.x);
-            color.y = fmaf(s, r1, color.y);
-            color.z = fmaf(s, r2, color.z);
-            color.w = fmaf(s, r3, color.w);
-            fi += 1.0f;
-            if(color.w > 0.99f)
+            if(done)
                 break;
         }
         count += (unsigned long long) (fminf(fi, fe + 1.0f) - fs);
+        float4 color;
+        f2p_split(rg, color.x, color.y);
+        f2p_split(ba, color.z, color.w);
         return color;
     }
 

@@ -17,35 +17,34 @@
 namespace isaacb
 {
     template<bool LINEAR, bool SKIP, bool YFAST>
-    __device__ __forceinline__ uchar4 batch_pixel(const BatchCtx& c, const View& v, int px, int py, unsigned long long& n)
+    __device__ __forceinline__ void batch_pixel(
+        const BatchCtx& c, const View& v, float negZero, int px, int py, uchar4* out, unsigned long long& n)
     {
         uchar4 col = to_byte4(c.bgSwizzled);
         float depth = FLT_MAX;
         Ray ray = pixel_to_ray(v, c.g, px, py);
         const ShadeParams sp{c.renderMode, c.aoWeight, c.bg};
         shade_values(sp, c.g, ray.dir, col, f3(0, 0, 0), 0.0f, depth);
-        if(!c.volume)
-            return col;
-        if(!clip_ray(ray, v, c.g))
-            return col;
+        *out = col; // read back after the march, which needs the registers
+        if(!c.volume || !clip_ray(ray, v, c.g))
+            return;
         ray.endDepth = gmin(ray.endDepth, depth);
         if(ray.endDepth <= ray.startDepth)
-            return col;
+            return;
         const March m = march_setup(ray, c.g, v.scale, c.step);
         const float factor = m.factor * c.totalWeightAll;
-        const VolTexRef tex{c.g, c.volQ, c.volFlag};
+        const VolTexRef tex{c.g, c.volQ, c.volFlag, negZero};
         float4 color;
         if(LINEAR && march_in_range(c.g, m))
-            color = march_combined<LINEAR, false, SKIP, YFAST>(tex, m, factor, n);
+            color = march_combined<LINEAR, false, SKIP, YFAST, 1>(tex, m, factor, n);
         else
-            color = march_combined<LINEAR, true, SKIP, YFAST>(tex, m, factor, n);
-        return over_surface(color, col);
+            color = march_combined<LINEAR, true, SKIP, YFAST, 1>(tex, m, factor, n);
+        *out = over_surface(color, *out);
     }
 
-    // 5 CTAs per SM (48 registers; the spills are outside the march): the march waits on
-    // memory, and 40 resident warps instead of 32 took two merges and 8 views of 512^3
-    // textures from 22.3 to 21.2 ms (6 CTAs: 21.4)
-    __global__ void __launch_bounds__(256, 5) k_batch(const __grid_constant__ BatchParams bp)
+    // 4 CTAs per SM (64 registers): two merges and 8 views of 512^3 textures take 20.9 ms; 3
+    // CTAs at 80 registers 21.5, 5 at 48 with spills 22.8
+    __global__ void __launch_bounds__(256, 4) k_batch(const __grid_constant__ BatchParams bp)
     {
         __shared__ View sv;
         __shared__ BatchCtx sc;
@@ -112,20 +111,21 @@ namespace isaacb
             const int py = (local / bv.tilesX) * bp.tileH + oy;
             if(px < sv.W && py < sv.H)
             {
-                uchar4 c;
                 // auto (-1): skip when the context's last merge found empty bricks
                 const bool skip = sc.skipEmpty >= 0 ? sc.skipEmpty != 0 : __ldg(sc.emptyCount) != 0u;
+                uchar4* out = bv.out + (size_t(py) * sv.W + px);
                 auto pixel = [&](auto linear, auto y) {
-                    return skip ? batch_pixel<decltype(linear)::value, true, decltype(y)::value>(sc, sv, px, py, n)
-                                : batch_pixel<decltype(linear)::value, false, decltype(y)::value>(sc, sv, px, py, n);
+                    if(skip)
+                        batch_pixel<decltype(linear)::value, true, decltype(y)::value>(sc, sv, bp.negZero, px, py, out, n);
+                    else
+                        batch_pixel<decltype(linear)::value, false, decltype(y)::value>(sc, sv, bp.negZero, px, py, out, n);
                 };
                 const std::true_type yes;
                 const std::false_type no;
                 if(sc.interpolation)
-                    c = yfast ? pixel(yes, yes) : pixel(yes, no);
+                    yfast ? pixel(yes, yes) : pixel(yes, no);
                 else
-                    c = yfast ? pixel(no, yes) : pixel(no, no);
-                bv.out[size_t(py) * sv.W + px] = c;
+                    yfast ? pixel(no, yes) : pixel(no, no);
             }
             __syncthreads();
         }

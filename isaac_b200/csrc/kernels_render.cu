@@ -412,37 +412,41 @@ namespace isaacb
         k_ssao<<<grid, 256, 0, s>>>(p);
     }
 
-    // A k_shade_volume block is 128 threads, 4 warps of 8 x 4 pixels, covering a tile of
-    // tile_w(FULL) x tile_h(FULL) pixels.
-    constexpr int kShadeThreads = 128;
-    // tile width of the FULL form (the short launches): 16 x 8 pixels keep a block's rays
-    // closer together than 32 x 4 (the 960x540 half-size render: 0.953 -> 0.931 ms)
-    constexpr int kShortTileW = 16;
-    // tile width and minimum blocks per SM of the uncapped form (the long launches)
-    constexpr int kLongTileW = 32;
-    constexpr int kLongMinBlocks = 1;
-    __host__ __device__ constexpr int shade_tile_w(bool full)
+    // How a launch of k_shade_volume is shaped, by the rays that an SM gets.  The march waits
+    // on its loads; with a full SM the other rays cover them, with few only the ray's own
+    // next samples can (march_combined's PAIRS), which cost registers and so rays.
+    //   SHADE_FULL  2 samples a trip, 64 registers: 8 blocks of 4 warps per SM.
+    //   SHADE_MID   4 samples, 100 registers: 5 blocks of 4 warps.
+    //   SHADE_FEW   8 samples, 162 registers, blocks of 2 warps.
+    // Shading and march in us, FULL / MID / FEW, 2 sources at step 0.5:
+    //   12.7 warps per SM (300x200 over 300^3) 283 / 181 / 142 (one sample a trip 471)
+    //   32 (500x300 over 300^3) 281 / 240 / 232, over 128^3 123 / 113 / 113
+    //   59 (700x400 over 300^3) 373 / 322 / 330, over 128^3 160 / 154 / 160
+    //   76 (800x450 over two 200^3 fields with empty space) 140 / 146 / 173
+    //   118 (1000x560 over 128^3) 261 / 254 / 277
+    //   437 (1920x1080 over 4 x 512^3) 3177 / 3189 / 3386
+    enum ShadeShape
     {
-        return full ? kShortTileW : kLongTileW;
+        SHADE_FULL,
+        SHADE_MID,
+        SHADE_FEW
+    };
+    constexpr int kShadeFewWarps = 24, kShadeMidWarps = 64; // most warps per SM of FEW and MID
+    __host__ __device__ constexpr int shade_threads(ShadeShape sh)
+    {
+        return sh == SHADE_FEW ? 64 : 128;
     }
-    __host__ __device__ constexpr int shade_tile_h(bool full)
+    __host__ __device__ constexpr int shade_pairs(ShadeShape sh)
     {
-        return kShadeThreads / shade_tile_w(full);
+        return sh == SHADE_FULL ? 1 : sh == SHADE_MID ? 2 : 4;
     }
-
-    // FULL: registers capped so that a whole SM's threads are resident (16 blocks, 32
-    // registers, a few bytes spilled).  Launches of only a few waves take it: more
-    // resident rays shorten their tail.  Longer launches keep the uncapped form (46
-    // registers, 10 blocks per SM), whose loop runs faster.
-    // tile of a y-fastest texture's blocks (4 warps of 4 x 8 pixels)
-    constexpr int kYTileW = 16;
-    __host__ __device__ constexpr int shade_tile_w(bool full, bool yfast)
+    __host__ __device__ constexpr int shade_tile_w(ShadeShape sh, bool yfast)
     {
-        return yfast ? kYTileW : shade_tile_w(full);
+        return sh == SHADE_FULL && !yfast ? 32 : sh == SHADE_FEW ? 8 : 16;
     }
-    __host__ __device__ constexpr int shade_tile_h(bool full, bool yfast)
+    __host__ __device__ constexpr int shade_tile_h(ShadeShape sh, bool yfast)
     {
-        return kShadeThreads / shade_tile_w(full, yfast);
+        return shade_threads(sh) / shade_tile_w(sh, yfast);
     }
 
     // The march's loads are bound by L1, which serves a 16-byte load 8 lanes at a time, one
@@ -452,15 +456,16 @@ namespace isaacb
     // y-fastest ones (YFAST) 8 lanes down a column (4 x 8 pixels), which views about the y
     // axis keep along y.  Against rows of 4 lanes for y-fastest slots that is 5.9 instead of
     // 10.7 cycles a load (a count over sampled warps that gives the 10.6 ncu showed), and
-    // the 4 x 512^3 march at 1920x1080 3.46 -> 3.24 ms, at 960x540 0.73 -> 0.63 ms.
+    // the 4 x 512^3 march at 1920x1080 3.46 -> 3.24 ms, at 960x540 0.73 -> 0.63 ms (one
+    // sample a trip).
     // CLEAN: the frame's only pass; it clears the G-buffer instead of reading it
-    template<bool VOLUME, bool LINEAR, bool FULL, bool YFAST, bool CLEAN>
-    __global__ void __launch_bounds__(kShadeThreads, FULL ? 2048 / kShadeThreads : kLongMinBlocks) k_shade_volume(const __grid_constant__ FrameParams p)
+    template<bool VOLUME, bool LINEAR, ShadeShape SHAPE, bool YFAST, bool CLEAN>
+    __global__ void __launch_bounds__(shade_threads(SHAPE), SHAPE == SHADE_FULL ? 8 : 1) k_shade_volume(const __grid_constant__ FrameParams p)
     {
         // empty-space skipping only pays when the texture has empty bricks; the merge that
         // wrote it counted them (either choice renders the same image)
         const bool skip = VOLUME && __ldg(p.emptyCount) != 0u;
-        constexpr int TW = shade_tile_w(FULL, YFAST), TH = shade_tile_h(FULL, YFAST);
+        constexpr int TW = shade_tile_w(SHAPE, YFAST), TH = shade_tile_h(SHAPE, YFAST);
         constexpr int WW = YFAST ? 4 : 8, WH = 32 / WW, WX = TW / WW; // warp tile and warps per row
         const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
         const int px = int(blockIdx.x) * TW + (w % WX) * WW + (YFAST ? l / WH : l % WW);
@@ -479,13 +484,15 @@ namespace isaacb
                     const March m = march_setup(ray, p.g, p.v.scale, p.step);
                     const float factor = m.factor * p.totalWeightAll;
                     float4 color;
-                    const VolTexRef tex{p.g, p.volQ, p.volFlag};
-                    if(LINEAR && march_in_range(p.g, m))
-                        color = skip ? march_combined<LINEAR, false, true, YFAST>(tex, m, factor, n)
-                                     : march_combined<LINEAR, false, false, YFAST>(tex, m, factor, n);
+                    const VolTexRef tex{p.g, p.volQ, p.volFlag, p.negZero};
+                    const bool inside = LINEAR && march_in_range(p.g, m);
+                    constexpr int PAIRS = shade_pairs(SHAPE);
+                    if(inside)
+                        color = skip ? march_combined<LINEAR, false, true, YFAST, PAIRS>(tex, m, factor, n)
+                                     : march_combined<LINEAR, false, false, YFAST, PAIRS>(tex, m, factor, n);
                     else
-                        color = skip ? march_combined<LINEAR, true, true, YFAST>(tex, m, factor, n)
-                                     : march_combined<LINEAR, true, false, YFAST>(tex, m, factor, n);
+                        color = skip ? march_combined<LINEAR, true, true, YFAST, PAIRS>(tex, m, factor, n)
+                                     : march_combined<LINEAR, true, false, YFAST, PAIRS>(tex, m, factor, n);
                     p.color[o] = over_surface(color, p.color[o]);
                 }
             }
@@ -496,48 +503,48 @@ namespace isaacb
             count_samples(p.counters, n);
     }
 
-    template<bool FULL, bool YFAST, bool CLEAN>
+    template<ShadeShape SHAPE, bool YFAST, bool CLEAN>
     void launch_shade_volume_as(const FrameParams& p, bool volume, cudaStream_t s)
     {
-        constexpr int TW = shade_tile_w(FULL, YFAST), TH = shade_tile_h(FULL, YFAST);
+        constexpr int TW = shade_tile_w(SHAPE, YFAST), TH = shade_tile_h(SHAPE, YFAST);
         const dim3 grid((p.v.W + TW - 1) / TW, (p.v.H + TH - 1) / TH);
         if(!volume)
-            k_shade_volume<false, false, FULL, YFAST, CLEAN><<<grid, kShadeThreads, 0, s>>>(p);
+            k_shade_volume<false, false, SHAPE, YFAST, CLEAN><<<grid, shade_threads(SHAPE), 0, s>>>(p);
         else if(p.interpolation)
-            k_shade_volume<true, true, FULL, YFAST, CLEAN><<<grid, kShadeThreads, 0, s>>>(p);
+            k_shade_volume<true, true, SHAPE, YFAST, CLEAN><<<grid, shade_threads(SHAPE), 0, s>>>(p);
         else
-            k_shade_volume<true, false, FULL, YFAST, CLEAN><<<grid, kShadeThreads, 0, s>>>(p);
+            k_shade_volume<true, false, SHAPE, YFAST, CLEAN><<<grid, shade_threads(SHAPE), 0, s>>>(p);
     }
-    template<bool FULL, bool YFAST>
-    void launch_shade_volume_clean(const FrameParams& p, bool volume, bool clean, cudaStream_t s)
+    template<ShadeShape SHAPE>
+    void launch_shade_volume_shape(const FrameParams& p, bool volume, bool clean, cudaStream_t s)
     {
-        clean ? launch_shade_volume_as<FULL, YFAST, true>(p, volume, s) : launch_shade_volume_as<FULL, YFAST, false>(p, volume, s);
+        if(p.g.yfast)
+            clean ? launch_shade_volume_as<SHAPE, true, true>(p, volume, s) : launch_shade_volume_as<SHAPE, true, false>(p, volume, s);
+        else
+            clean ? launch_shade_volume_as<SHAPE, false, true>(p, volume, s) : launch_shade_volume_as<SHAPE, false, false>(p, volume, s);
     }
-
-    // launches of fewer than this many waves of the uncapped form take the FULL form
-    constexpr int kShadeShortWaves = 4;
 
     void launch_shade_volume(const FrameParams& p, bool volume, bool clean, cudaStream_t s)
     {
-        const long long blocks = (long long) ((p.v.W + shade_tile_w(false) - 1) / shade_tile_w(false))
-            * ((p.v.H + shade_tile_h(false) - 1) / shade_tile_h(false));
-        // resident blocks of the uncapped form on the whole device, once per device (a
-        // property of the kernel and the device, valid in any context on it)
-        static int resident[64] = {0};
-        int dev = 0;
+        // SMs, once per device
+        static std::atomic<int> smCount[64]{};
+        int dev = 0, sms = 148;
         cudaGetDevice(&dev);
-        if(dev >= 0 && dev < 64 && resident[dev] == 0)
+        if(dev >= 0 && dev < 64)
         {
-            int sms = 0, perSm = 0;
-            cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, k_shade_volume<true, true, false, false, false>, kShadeThreads, 0);
-            resident[dev] = std::max(1, sms * perSm);
+            if(smCount[dev].load() == 0)
+            {
+                cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+                smCount[dev].store(std::max(1, sms));
+            }
+            sms = smCount[dev].load();
         }
-        const long long waves = blocks / std::max(1, dev >= 0 && dev < 64 ? resident[dev] : 1);
-        const bool full = volume && waves < kShadeShortWaves;
-        if(p.g.yfast)
-            full ? launch_shade_volume_clean<true, true>(p, volume, clean, s) : launch_shade_volume_clean<false, true>(p, volume, clean, s);
+        const long long warps = (long long) ((p.v.W + 7) / 8) * ((p.v.H + 3) / 4);
+        if(!volume || warps > (long long) sms * kShadeMidWarps)
+            launch_shade_volume_shape<SHADE_FULL>(p, volume, clean, s);
+        else if(warps > (long long) sms * kShadeFewWarps)
+            launch_shade_volume_shape<SHADE_MID>(p, volume, clean, s);
         else
-            full ? launch_shade_volume_clean<true, false>(p, volume, clean, s) : launch_shade_volume_clean<false, false>(p, volume, clean, s);
+            launch_shade_volume_shape<SHADE_FEW>(p, volume, clean, s);
     }
 } // namespace isaacb
