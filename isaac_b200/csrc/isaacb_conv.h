@@ -73,14 +73,25 @@ namespace isaacb
         int B, H, W, Cin, Ho, Wo, Cout, Npad;
         int ks, stride, pad;
         int Mtot; // ks*ks*Cin
-        int chunksPerSplit; // set by the launcher
+        // implicit concatenation as in ConvGemmParams (1x1): the first upC input channels come
+        // from xUp at the nearest coarse pixel, the other Cin - upC from x; null = off
+        const __nv_bfloat16* xUp;
+        int upC, upInH, upInW;
+        int chunksPerSplit, mTiles, stages; // set by the launcher
         int* errorFlag;
+    };
+    // the layers of one launch; CTA i works on layer l with first[l] <= i < first[l + 1]
+    constexpr int kWgradLayers = 12;
+    struct WgradTable
+    {
+        WgradParams layer[kWgradLayers];
+        int first[kWgradLayers + 1];
     };
 
     size_t conv_gemm_smem(int Npad, int Kpad);
     // the row-tile kernel takes this convolution (and then honours xUp)
     bool row_tiles_apply(const ConvGemmParams& p);
-    size_t conv_wgrad_smem(int Npad);
     bool launch_conv_gemm(ConvGemmParams p, cudaStream_t s);
-    bool launch_conv_wgrad(WgradParams p, cudaStream_t s);
+    // the weight gradients of n layers (at most kWgradLayers) in one launch
+    bool launch_conv_wgrad(const WgradParams* layers, int n, cudaStream_t s);
 } // namespace isaacb

@@ -121,31 +121,7 @@ namespace
         }
     }
 
-    // [up(coarse), fine] along channels, 8 channels per thread step
-    __global__ void k_cat_up(const bf16* __restrict__ coarse, const bf16* __restrict__ fine, bf16* __restrict__ out, int B, int h, int w, int hc, int wc, int c1, int c2)
-    {
-        const int cc = (c1 + c2) / 8;
-        const size_t n = size_t(B) * h * w * cc;
-        for(size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x; i < n; i += size_t(gridDim.x) * blockDim.x)
-        {
-            const int j = int(i % cc);
-            const size_t p = i / cc;
-            uint4 v;
-            if(j * 8 < c1)
-            {
-                const int x = int(p % w);
-                const size_t t = p / w;
-                const int y = int(t % h), b = int(t / h);
-                const int yc = min(y / 2, hc - 1), xc = min(x / 2, wc - 1);
-                v = __ldg(reinterpret_cast<const uint4*>(coarse + ((size_t(b) * hc + yc) * wc + xc) * c1 + j * 8));
-            }
-            else
-                v = __ldg(reinterpret_cast<const uint4*>(fine + p * c2 + (j * 8 - c1)));
-            reinterpret_cast<uint4*>(out)[i] = v;
-        }
-    }
-
-    // gradient of k_cat_up: fine part copied, coarse part summed over its children; both
+    // gradient of the concatenation [up(coarse), fine]: fine part copied, coarse part summed over its children; both
     // multiplied by (activation > 0), the derivative of the producing layer's ReLU
     __global__ void k_cat_up_backward(
         const bf16* __restrict__ dcat,
@@ -501,7 +477,6 @@ struct isaacb_recon
     bf16* wt[kLayers] = {};
     bf16* act[kLayers] = {}; // outputs (OUT: unused, see r)
     bf16* dpre[kLayers] = {}; // gradient with respect to each layer's pre-activation output
-    bf16* cat[kLayers] = {}; // concatenated inputs
     bf16* dcat = nullptr; // gradient of a concatenated input (largest one)
     bf16* x = nullptr;
     float* r = nullptr; // OUT, FP32
@@ -561,22 +536,12 @@ namespace
         return kLevel[d.src];
     }
 
-    const bf16* layer_input(const isaacb_recon* R, int L)
-    {
-        const LayerDef& d = kDefs[L];
-        if(d.src == SRC_X)
-            return R->x;
-        if(d.src == -2)
-            return R->cat[L];
-        return R->act[d.src];
-    }
-
     bool conv_layer(isaacb_recon* R, int L, int B, cudaStream_t s, bool pdl = false)
     {
         const LayerDef& d = kDefs[L];
         const int li = in_level(L), lo = kLevel[L];
         ConvGemmParams p{};
-        p.x = layer_input(R, L);
+        p.x = d.src == SRC_X ? R->x : R->act[d.src];
         p.w = R->wf[L];
         p.bias = R->bias[L];
         p.y = L == kLayers - 1 ? nullptr : R->act[L];
@@ -601,37 +566,48 @@ namespace
         return launch_conv_gemm(p, s);
     }
 
+    // A concatenating 1x1 layer reads its two inputs in place: the row-tile producer gathers
+    // the coarse tensor's channels at the nearest coarse pixel and the fine tensor's after
+    // them, which is [up(coarse), fine] without the concatenated tensor ever being formed
+    // (forming it took 6, 11 and 21 us of a training step of 16 128 x 128 pairs).
+    bool cat_layer(isaacb_recon* R, int L, int B, cudaStream_t s)
+    {
+        const LayerDef& d = kDefs[L];
+        const int lf = kLevel[d.fine], lc = kLevel[d.coarse];
+        ConvGemmParams p{};
+        p.x = R->act[d.fine];
+        p.xUp = R->act[d.coarse];
+        p.upC = kDefs[d.coarse].cout;
+        p.upInH = R->lh[lc];
+        p.upInW = R->lw[lc];
+        p.w = R->wf[L];
+        p.bias = R->bias[L];
+        p.y = R->act[L];
+        p.B = B;
+        p.H = p.Ho = R->lh[lf];
+        p.W = p.Wo = R->lw[lf];
+        p.Cg = R->T.cg[L];
+        p.Cout = d.cout;
+        p.Npad = R->T.Npad[L];
+        p.Kpad = R->T.Kpad[L];
+        p.ks = 1;
+        p.stride = 1;
+        p.relu = d.relu;
+        p.errorFlag = R->errorFlag;
+        p.pdl = 1;
+        return p.Cg == d.cin && row_tiles_apply(p) && launch_conv_gemm(p, s);
+    }
+
+    // each layer follows a row-tile convolution (the first k_input) as its programmatic dependent
     bool forward(isaacb_recon* R, int B, cudaStream_t s)
     {
         for(int L = 0; L < kLayers; ++L)
-        {
-            const LayerDef& d = kDefs[L];
-            if(d.src == -2)
-            {
-                const int lf = kLevel[d.fine], lc = kLevel[d.coarse];
-                const size_t n = size_t(B) * R->lh[lf] * R->lw[lf] * (d.cin / 8);
-                k_cat_up<<<grid_for(n), 256, 0, s>>>(
-                    R->act[d.coarse],
-                    R->act[d.fine],
-                    R->cat[L],
-                    B,
-                    R->lh[lf],
-                    R->lw[lf],
-                    R->lh[lc],
-                    R->lw[lc],
-                    kDefs[d.coarse].cout,
-                    kDefs[d.fine].cout);
-            }
-            if(!conv_layer(R, L, B, s))
+            if(!(kDefs[L].src == -2 ? cat_layer(R, L, B, s) : conv_layer(R, L, B, s, true)))
                 return false;
-        }
         return true;
     }
 
-    // One image, inference only.  A concatenating 1x1 layer reads its two inputs in place:
-    // the row-tile producer gathers the coarse tensor's channels at the nearest coarse
-    // pixel and the fine tensor's after them, which is [up(coarse), fine] without the
-    // concatenated tensor ever being formed.  The sums are the training forward's.
+    // One image, inference only: the training forward's sums, then the frame.
     bool forward_infer(isaacb_recon* R, const uint8_t* low, uint8_t* out, cudaStream_t s)
     {
         for(int L = 0; L < kLayers; ++L)
@@ -639,30 +615,7 @@ namespace
             const LayerDef& d = kDefs[L];
             if(d.src == -2)
             {
-                // [up(coarse), fine] read in place by the producer (implicit concatenation)
-                const int lf = kLevel[d.fine], lc = kLevel[d.coarse];
-                ConvGemmParams p{};
-                p.x = R->act[d.fine];
-                p.xUp = R->act[d.coarse];
-                p.upC = kDefs[d.coarse].cout;
-                p.upInH = R->lh[lc];
-                p.upInW = R->lw[lc];
-                p.w = R->wf[L];
-                p.bias = R->bias[L];
-                p.y = R->act[L];
-                p.B = 1;
-                p.H = p.Ho = R->lh[lf];
-                p.W = p.Wo = R->lw[lf];
-                p.Cg = R->T.cg[L];
-                p.Cout = d.cout;
-                p.Npad = R->T.Npad[L];
-                p.Kpad = R->T.Kpad[L];
-                p.ks = 1;
-                p.stride = 1;
-                p.relu = d.relu;
-                p.errorFlag = R->errorFlag;
-                p.pdl = 1;
-                if(p.Cg != d.cin || !row_tiles_apply(p) || !launch_conv_gemm(p, s))
+                if(!cat_layer(R, L, 1, s))
                     return false;
                 continue;
             }
@@ -711,14 +664,23 @@ namespace
     bool backward(isaacb_recon* R, int B, cudaStream_t s)
     {
         bool has[kLayers] = {};
+        WgradParams grads[kLayers] = {};
         for(int L = kLayers - 1; L >= 0; --L)
         {
             const LayerDef& d = kDefs[L];
             const int li = in_level(L), lo = kLevel[L];
             const bf16* g = R->dpre[L];
-            // weight gradient
-            WgradParams wp{};
-            wp.x = layer_input(R, L);
+            // weight gradient, of all layers at the end
+            WgradParams& wp = grads[L];
+            wp.x = d.src == -2 ? R->act[d.fine] : d.src == SRC_X ? R->x : R->act[d.src];
+            if(d.src == -2)
+            {
+                const int lc = kLevel[d.coarse];
+                wp.xUp = R->act[d.coarse];
+                wp.upC = kDefs[d.coarse].cout;
+                wp.upInH = R->lh[lc];
+                wp.upInW = R->lw[lc];
+            }
             wp.dy = g;
             wp.dw = R->dw[L];
             wp.B = B;
@@ -734,8 +696,6 @@ namespace
             wp.pad = d.pad;
             wp.Mtot = d.ks * d.ks * R->T.cg[L];
             wp.errorFlag = R->errorFlag;
-            if(!launch_conv_wgrad(wp, s))
-                return false;
             if(d.src == SRC_X)
                 continue;
             // input gradient
@@ -756,6 +716,7 @@ namespace
             p.pad = d.pad;
             p.transposed = 1;
             p.errorFlag = R->errorFlag;
+            p.pdl = 1;
             if(d.src == -2)
             {
                 p.y = R->dcat;
@@ -789,6 +750,8 @@ namespace
                 has[d.src] = true;
             }
         }
+        if(!launch_conv_wgrad(grads, kLayers, s))
+            return false;
         BiasGradTable T{};
         for(int L = 0; L < kLayers; ++L)
         {
@@ -883,7 +846,6 @@ extern "C"
                 ok = ok && dalloc(R, R->act[L], pix * d.cout);
             if(d.src == -2)
             {
-                ok = ok && dalloc(R, R->cat[L], pix * d.cin);
                 maxCat = std::max(maxCat, pix * d.cin);
             }
             if(ok && conv_gemm_smem(R->T.Npad[L], R->T.Kpad[L]) > 227 * 1024)

@@ -896,12 +896,21 @@ namespace isaacb
         }
 
         // ------------------------------------------------------------------ weight gradient
-        __global__ void __launch_bounds__(kThreads, 1) k_conv_wgrad(const __grid_constant__ WgradParams p)
+        // All layers of a network in one launch: their CTAs fill the device together, and there
+        // is one tail instead of one per layer (a step of 16 128 x 128 pairs: eleven launches of
+        // 14-55 us, 362 us together, to one of 329 us).
+        __global__ void __launch_bounds__(kThreads, 1) k_conv_wgrad(const __grid_constant__ WgradTable T)
         {
             extern __shared__ unsigned char dsm[];
             __shared__ uint32_t sTmem;
             __shared__ __align__(8) uint64_t sEmpty[kStages];
             __shared__ __align__(8) uint64_t sDone;
+            int layer = 0;
+            while(int(blockIdx.x) >= T.first[layer + 1])
+                ++layer;
+            const WgradParams& p = T.layer[layer];
+            const int local = int(blockIdx.x) - T.first[layer];
+            const uint32_t stages = uint32_t(p.stages);
             unsigned char* base = dsm + ((128u - (tc::smem_addr(dsm) & 127u)) & 127u);
             const uint32_t stageB = uint32_t(p.Npad) * 128u; // Npad/8 core rows x 8 pixel blocks x 128 B
             const uint32_t stageBytes = uint32_t(kStageBytesA) + stageB;
@@ -928,10 +937,11 @@ namespace isaacb
 
             const int P = p.B * p.Ho * p.Wo;
             const int nChunks = (P + kChunkK - 1) / kChunkK;
-            const int c0 = blockIdx.y * p.chunksPerSplit;
+            const int split = local / p.mTiles;
+            const int c0 = split * p.chunksPerSplit;
             const int c1 = min(nChunks, c0 + p.chunksPerSplit);
             const int nk = c1 - c0;
-            const int mTile = blockIdx.x;
+            const int mTile = local - split * p.mTiles;
             const uint32_t idesc = tc::idesc_bf16(kTileM, p.Npad, true, true);
 
             // A thread copies, for pixel px of every chunk, the row blocks (8 channels of one
@@ -952,7 +962,7 @@ namespace isaacb
             int pix = c0 * kChunkK + px;
             int ox = pix % p.Wo, oy = (pix / p.Wo) % p.Ho, b = pix / p.Wo / p.Ho;
             auto load_chunk = [&](uint32_t G) {
-                const uint32_t stA = s0 + (G % kStages) * stageBytes;
+                const uint32_t stA = s0 + (G % stages) * stageBytes;
                 const uint32_t stB = stA + uint32_t(kStageBytesA);
                 const uint32_t at = uint32_t(px >> 3) * 128u + uint32_t(px & 7) * 16u;
 #pragma unroll
@@ -960,7 +970,12 @@ namespace isaacb
                 {
                     const int iy = oy * p.stride + ty[q], ix = ox * p.stride + tx[q];
                     const bool ok = tc0[q] >= 0 && pix < P && iy >= 0 && ix >= 0 && iy < p.H && ix < p.W;
-                    const bf16* src = ok ? p.x + ((size_t(b) * p.H + iy) * p.W + ix) * p.Cin + tc0[q] : p.x;
+                    const bf16* src = p.x;
+                    if(ok && tc0[q] < p.upC) // nearest coarse pixel
+                        src = p.xUp
+                            + ((size_t(b) * p.upInH + min(iy >> 1, p.upInH - 1)) * p.upInW + min(ix >> 1, p.upInW - 1)) * p.upC + tc0[q];
+                    else if(ok)
+                        src += ((size_t(b) * p.H + iy) * p.W + ix) * (p.Cin - p.upC) + (tc0[q] - p.upC);
                     tc::cp_async16(stA + uint32_t(mb0 + 4 * q) * 1024u + at, src, ok ? 16u : 0u);
                 }
                 // B: Npad/8 column blocks x 64 pixels of dY
@@ -983,7 +998,7 @@ namespace isaacb
                 }
             };
 
-            for(int c = 0; c < kStages - 1; ++c)
+            for(int c = 0; c < int(stages) - 1; ++c)
             {
                 if(c < nk)
                     load_chunk(uint32_t(c));
@@ -991,16 +1006,19 @@ namespace isaacb
             }
             for(int kc = 0; kc < nk; ++kc)
             {
-                const int kn = kc + kStages - 1;
+                const int kn = kc + int(stages) - 1;
                 if(kn < nk)
                 {
                     const uint32_t G = uint32_t(kn);
-                    if(G >= kStages && !tc::mbar_wait(&sEmpty[G % kStages], ((G / kStages) - 1) & 1))
+                    if(G >= stages && !tc::mbar_wait(&sEmpty[G % stages], ((G / stages) - 1) & 1))
                         raise_error(p.errorFlag, abortLocal);
                     load_chunk(G);
                 }
                 tc::cp_async_commit();
-                tc::cp_async_wait<kStages - 1>();
+                if(stages == kStages)
+                    tc::cp_async_wait<kStages - 1>();
+                else
+                    tc::cp_async_wait<kStages - 2>();
                 tc::fence_async_smem();
                 if(__syncthreads_or(abortLocal))
                 {
@@ -1010,7 +1028,7 @@ namespace isaacb
                 if(tid == 0)
                 {
                     tc::fence_after_sync();
-                    const uint32_t stA = s0 + (uint32_t(kc) % kStages) * stageBytes;
+                    const uint32_t stA = s0 + (uint32_t(kc) % stages) * stageBytes;
                     const uint32_t stB = stA + uint32_t(kStageBytesA);
 #pragma unroll
                     for(int j = 0; j < kChunkK / 16; ++j)
@@ -1019,7 +1037,7 @@ namespace isaacb
                         const uint64_t bd = tc::smem_desc(stB + uint32_t(j) * 256u, 128u, 1024u);
                         tc::mma_bf16(tmem, ad, bd, idesc, (kc | j) != 0 ? 1u : 0u);
                     }
-                    tc::mma_commit(&sEmpty[uint32_t(kc) % kStages]);
+                    tc::mma_commit(&sEmpty[uint32_t(kc) % stages]);
                 }
             }
             tc::cp_async_wait<0>();
@@ -1090,11 +1108,6 @@ namespace isaacb
     {
         return size_t(Npad) * Kpad * 2 + size_t(kStages) * kStageBytesA + 128;
     }
-    size_t conv_wgrad_smem(int Npad)
-    {
-        return size_t(kStages) * (kStageBytesA + size_t(Npad) * 128) + 128;
-    }
-
     bool row_tiles_apply(const ConvGemmParams& p)
     {
         if(p.xUp && (p.ks != 1 || p.stride != 1 || p.upC % 8 != 0 || p.transposed))
@@ -1323,25 +1336,36 @@ namespace isaacb
         return true;
     }
 
-    bool launch_conv_wgrad(WgradParams p, cudaStream_t s)
+    bool launch_conv_wgrad(const WgradParams* layers, int n, cudaStream_t s)
     {
-        const size_t smem = conv_wgrad_smem(p.Npad);
+        WgradTable T{};
+        size_t smem = 0, work = 0;
+        for(int l = 0; l < n; ++l)
+        {
+            WgradParams& p = T.layer[l];
+            p = layers[l];
+            // three stages where four would leave room for one CTA per SM only
+            p.stages = 4 * (kStageBytesA + p.Npad * 128) <= 112 * 1024 ? kStages : kStages - 1;
+            p.mTiles = (p.Mtot + kTileM - 1) / kTileM;
+            smem = std::max(smem, size_t(p.stages) * (kStageBytesA + size_t(p.Npad) * 128) + 128);
+            work += size_t(p.mTiles) * ((size_t(p.B) * p.Ho * p.Wo + kChunkK - 1) / kChunkK);
+        }
         if(smem > 227 * 1024)
             return false;
         cudaFuncSetAttribute(k_conv_wgrad, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
         cudaFuncSetAttribute(k_conv_wgrad, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-        const int P = p.B * p.Ho * p.Wo;
-        const int nChunks = (P + kChunkK - 1) / kChunkK;
-        const int mTiles = (p.Mtot + kTileM - 1) / kTileM;
-        // about two CTAs' worth of work per SM in total, at least 4 chunks each
-        int splits = (2 * num_sms() + mTiles - 1) / mTiles;
-        int per = (nChunks + splits - 1) / splits;
-        if(per < 4)
-            per = 4;
-        splits = (nChunks + per - 1) / per;
-        p.chunksPerSplit = per;
-        dim3 grid(mTiles, splits);
-        k_conv_wgrad<<<grid, kThreads, smem, s>>>(p);
+        // two CTAs fit on an SM; about two such waves of equal work, at least 4 chunks each
+        const int per = std::max(4, int((work + 4 * num_sms() - 1) / (4 * num_sms())));
+        for(int l = 0; l < n; ++l)
+        {
+            WgradParams& p = T.layer[l];
+            const int chunks = (p.B * p.Ho * p.Wo + kChunkK - 1) / kChunkK;
+            p.chunksPerSplit = per;
+            T.first[l + 1] = T.first[l] + p.mTiles * ((chunks + per - 1) / per);
+        }
+        for(int l = n; l < kWgradLayers; ++l)
+            T.first[l + 1] = T.first[n];
+        k_conv_wgrad<<<T.first[n], kThreads, smem, s>>>(T);
         return true;
     }
 } // namespace isaacb
@@ -1450,7 +1474,7 @@ extern "C"
         p.pad = int(a->pad);
         p.Mtot = int(a->ksize * a->ksize * a->c_in);
         p.errorFlag = a->error_flag;
-        if(!launch_conv_wgrad(p, (cudaStream_t) stream))
+        if(!launch_conv_wgrad(&p, 1, (cudaStream_t) stream))
         {
             set_global_error("isaacb_conv_wgrad: tile does not fit in shared memory");
             return ISAACB_INVALID_ARG;

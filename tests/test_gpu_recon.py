@@ -75,6 +75,28 @@ def test_gradients_match_oracle():
         assert rel < 3e-2 and cos > 0.999, (name, rel, cos)
 
 
+@pytest.mark.parametrize("b,h,w", [(3, 16, 24), (2, 13, 17), (1, 8, 160)])
+def test_gradients_match_oracle_by_size(b, h, w):
+    """The training forward's in-place concatenation over several images: by TMA (every
+    level's width even), gathered with clamped coarse rows and columns (odd levels), and
+    with two tiles a row; the weight gradients of all layers in one launch."""
+    params = _he_params(1)
+    rng = np.random.default_rng(b * h * w)
+    low = rng.integers(0, 256, (b, h, w, 4)).astype(np.uint8)
+    high = rng.integers(0, 256, (b, 2 * h, 2 * w, 4)).astype(np.uint8)
+    net = Reconstructor(b, h, w, seed=1)
+    net.set_params(params)
+    g, loss = net.gradients(torch.from_numpy(low).cuda(), torch.from_numpy(high).cuda())
+    assert net.error_flag() == 0
+    ref_loss, ref = R.UNet(params.astype(np.float64), bf16=True).loss_and_backward(low, high)
+    assert abs(loss - ref_loss) <= 1e-3 * ref_loss
+    for name, sl in _layer_slices():
+        a, r = g[sl].astype(np.float64), ref[sl]
+        rel = np.linalg.norm(a - r) / np.linalg.norm(r)
+        cos = float(a @ r / (np.linalg.norm(a) * np.linalg.norm(r)))
+        assert rel < 3e-2 and cos > 0.999, (name, rel, cos)
+
+
 def test_inference_matches_oracle():
     params = _he_params(3)
     params[-528:] *= 0.1  # OUT weights and bias: a small residual, as after initialisation
