@@ -77,7 +77,7 @@ namespace isaacb
         // from xUp at the nearest coarse pixel, the other Cin - upC from x; null = off
         const __nv_bfloat16* xUp;
         int upC, upInH, upInW;
-        int chunksPerSplit, mTiles, stages; // set by the launcher
+        int chunksPerSplit, mTiles; // set by the launcher
         int* errorFlag;
     };
     // the layers of one launch; CTA i works on layer l with first[l] <= i < first[l + 1]

@@ -895,25 +895,52 @@ namespace isaacb
                 tc::tmem_dealloc(tmem, cols);
         }
 
+        constexpr int kWgradStages = 2;
+        // bytes from one 8-channel block of 64 pixels to the next: 32 more than the block, so
+        // that the 8 lanes of a 16-byte store phase (2 pixels x 4 blocks) meet all banks
+        constexpr uint32_t kBlockPitch = kChunkK * 16 + 32;
+
+        // 16 bytes, or zeros; issued where it stands
+        __device__ __forceinline__ uint4 load_piece(const bf16* src, bool ok)
+        {
+            uint4 v = make_uint4(0, 0, 0, 0);
+            asm volatile(
+                "{\n\t.reg .pred p;\n\tsetp.ne.s32 p, %5, 0;\n\t@p ld.global.nc.v4.u32 {%0, %1, %2, %3}, [%4];\n\t}"
+                : "+r"(v.x), "+r"(v.y), "+r"(v.z), "+r"(v.w)
+                : "l"(src), "r"(int(ok)));
+            return v;
+        }
+        __device__ __forceinline__ void store_piece(uint32_t at, uint4 v)
+        {
+            asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(at), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
+        }
+
         // ------------------------------------------------------------------ weight gradient
         // All layers of a network in one launch: their CTAs fill the device together, and there
         // is one tail instead of one per layer (a step of 16 128 x 128 pairs: eleven launches of
-        // 14-55 us, 362 us together, to one of 329 us).
-        __global__ void __launch_bounds__(kThreads, 1) k_conv_wgrad(const __grid_constant__ WgradTable T)
+        // 14-55 us, 362 us together, to one of 329 us).  What bounds a CTA is bringing the tiles to
+        // shared memory, pixels' channels into 8-channel blocks: cp.async writes each 16-byte
+        // piece of its own line in its own shared-memory cycle (30 a request, half of the time),
+        // so a thread loads its pieces of the next chunk into registers while the MMAs of this
+        // one run, and stores them 8 lanes a cycle: 329 -> 213 us; addresses as 32-bit piece
+        // counts from the pixel's: 177 us.  Three CTAs an SM (two 3533, three 3374, four, with
+        // 62 registers, 3430 us per four steps), twelve an SM in all (three 3410, six 3374,
+        // twelve 3359 us): the layers' CTAs differ in cost and the last ones stay short.
+        template<int NB>
+        __global__ void __launch_bounds__(kThreads, NB == 4 ? 3 : 2) k_conv_wgrad(const __grid_constant__ WgradTable T)
         {
             extern __shared__ unsigned char dsm[];
             __shared__ uint32_t sTmem;
-            __shared__ __align__(8) uint64_t sEmpty[kStages];
+            __shared__ __align__(8) uint64_t sEmpty[kWgradStages];
             __shared__ __align__(8) uint64_t sDone;
             int layer = 0;
             while(int(blockIdx.x) >= T.first[layer + 1])
                 ++layer;
             const WgradParams& p = T.layer[layer];
             const int local = int(blockIdx.x) - T.first[layer];
-            const uint32_t stages = uint32_t(p.stages);
+            constexpr uint32_t stages = kWgradStages;
             unsigned char* base = dsm + ((128u - (tc::smem_addr(dsm) & 127u)) & 127u);
-            const uint32_t stageB = uint32_t(p.Npad) * 128u; // Npad/8 core rows x 8 pixel blocks x 128 B
-            const uint32_t stageBytes = uint32_t(kStageBytesA) + stageB;
+            const uint32_t stageBytes = (16u + uint32_t(p.Npad) / 8u) * kBlockPitch;
             const uint32_t s0 = tc::smem_addr(base);
             const int tid = threadIdx.x;
             const uint32_t cols = tmem_columns(p.Npad);
@@ -924,7 +951,7 @@ namespace isaacb
             }
             if(tid == 0)
             {
-                for(int s = 0; s < kStages; ++s)
+                for(int s = 0; s < kWgradStages; ++s)
                     tc::mbar_init(&sEmpty[s], 1);
                 tc::mbar_init(&sDone, 1);
                 tc::mbar_init_fence();
@@ -944,46 +971,51 @@ namespace isaacb
             const int mTile = local - split * p.mTiles;
             const uint32_t idesc = tc::idesc_bf16(kTileM, p.Npad, true, true);
 
-            // A thread copies, for pixel px of every chunk, the row blocks (8 channels of one
+            // A thread carries, for pixel px of every chunk, the row blocks (8 channels of one
             // tap) mb0 + 4 q and the column blocks mb0 + 4 i of dY.  The chunks are taken in
             // order, so the pixel's place in the image and the blocks' taps need no division
             // inside the loop.
-            const int px = tid & (kChunkK - 1), mb0 = tid >> 6;
-            int ty[4], tx[4], tc0[4];
+            const int px = tid >> 2, mb0 = tid & 3;
+            // Addresses in 16-byte pieces: a tensor's fit 32 bits (2^26 pixels of at most 28).
+            const int cX = (p.Cin - p.upC) / 8, cD = p.Cout / 8, cU = p.upC / 8;
+            int ty[4], tx[4];
+            int inUp = 0; // bit q: row block q is of the coarse tensor
+            uint32_t delta[4]; // the tap's and channel's pieces from the pixel's first
 #pragma unroll
             for(int q = 0; q < 4; ++q)
             {
                 const int r0 = mTile * kTileM + (mb0 + 4 * q) * 8;
-                const int t = r0 / p.Cin;
-                ty[q] = t / p.ks - p.pad;
+                const int t = r0 / p.Cin, ch = (r0 - t * p.Cin) / 8;
+                ty[q] = r0 < p.Mtot ? t / p.ks - p.pad : 1 << 30; // past the last row: outside always (H < 2^28)
                 tx[q] = t % p.ks - p.pad;
-                tc0[q] = r0 < p.Mtot ? r0 - t * p.Cin : -1;
+                // of the coarse tensor (1x1 layers: the tap is the pixel) or of x
+                inUp |= int(ch < cU) << q;
+                delta[q] = ch < cU ? uint32_t(ch) : (uint32_t(ty[q]) * uint32_t(p.W) + uint32_t(tx[q])) * uint32_t(cX) + uint32_t(ch - cU);
             }
+            const bool up = cU > 0;
             int pix = c0 * kChunkK + px;
             int ox = pix % p.Wo, oy = (pix / p.Wo) % p.Ho, b = pix / p.Wo / p.Ho;
-            auto load_chunk = [&](uint32_t G) {
-                const uint32_t stA = s0 + (G % stages) * stageBytes;
-                const uint32_t stB = stA + uint32_t(kStageBytesA);
-                const uint32_t at = uint32_t(px >> 3) * 128u + uint32_t(px & 7) * 16u;
+            uint4 ra[4], rb[NB];
+            auto fetch = [&]() {
+                const int x0 = ox * p.stride, y0 = pix < P ? oy * p.stride : -(1 << 20); // past the last pixel: no row
+                const uint32_t at = (uint32_t(b * p.H + y0) * uint32_t(p.W) + uint32_t(x0)) * uint32_t(cX);
+                uint32_t atUp = 0;
+                if(up) // nearest coarse pixel
+                    atUp = (uint32_t(b * p.upInH + min(y0 >> 1, p.upInH - 1)) * uint32_t(p.upInW)
+                            + uint32_t(min(x0 >> 1, p.upInW - 1))) * uint32_t(cU);
 #pragma unroll
                 for(int q = 0; q < 4; ++q)
                 {
-                    const int iy = oy * p.stride + ty[q], ix = ox * p.stride + tx[q];
-                    const bool ok = tc0[q] >= 0 && pix < P && iy >= 0 && ix >= 0 && iy < p.H && ix < p.W;
-                    const bf16* src = p.x;
-                    if(ok && tc0[q] < p.upC) // nearest coarse pixel
-                        src = p.xUp
-                            + ((size_t(b) * p.upInH + min(iy >> 1, p.upInH - 1)) * p.upInW + min(ix >> 1, p.upInW - 1)) * p.upC + tc0[q];
-                    else if(ok)
-                        src += ((size_t(b) * p.H + iy) * p.W + ix) * (p.Cin - p.upC) + (tc0[q] - p.upC);
-                    tc::cp_async16(stA + uint32_t(mb0 + 4 * q) * 1024u + at, src, ok ? 16u : 0u);
+                    const bool ok = uint32_t(y0 + ty[q]) < uint32_t(p.H) && uint32_t(x0 + tx[q]) < uint32_t(p.W);
+                    const bool coarse = inUp >> q & 1;
+                    ra[q] = load_piece((coarse ? p.xUp : p.x) + size_t((coarse ? atUp : at) + delta[q]) * 8, ok);
                 }
                 // B: Npad/8 column blocks x 64 pixels of dY
-                for(int nb = mb0; nb < p.Npad / 8; nb += 4)
+#pragma unroll
+                for(int i = 0; i < NB; ++i)
                 {
-                    const bool ok = pix < P && nb * 8 < p.Cout;
-                    const bf16* src = ok ? p.dy + size_t(pix) * p.Cout + nb * 8 : p.dy;
-                    tc::cp_async16(stB + uint32_t(nb) * 1024u + at, src, ok ? 16u : 0u);
+                    const int nb = mb0 + 4 * i;
+                    rb[i] = load_piece(p.dy + (size_t(uint32_t(pix) * uint32_t(cD)) + nb) * 8, pix < P && nb < cD);
                 }
                 pix += kChunkK;
                 ox += kChunkK;
@@ -998,28 +1030,25 @@ namespace isaacb
                 }
             };
 
-            for(int c = 0; c < int(stages) - 1; ++c)
-            {
-                if(c < nk)
-                    load_chunk(uint32_t(c));
-                tc::cp_async_commit();
-            }
+            const uint32_t at = uint32_t(mb0) * kBlockPitch + uint32_t(px) * 16u;
+            if(nk > 0)
+                fetch();
             for(int kc = 0; kc < nk; ++kc)
             {
-                const int kn = kc + int(stages) - 1;
-                if(kn < nk)
-                {
-                    const uint32_t G = uint32_t(kn);
-                    if(G >= stages && !tc::mbar_wait(&sEmpty[G % stages], ((G / stages) - 1) & 1))
-                        raise_error(p.errorFlag, abortLocal);
-                    load_chunk(G);
-                }
-                tc::cp_async_commit();
-                if(stages == kStages)
-                    tc::cp_async_wait<kStages - 1>();
-                else
-                    tc::cp_async_wait<kStages - 2>();
+                const uint32_t G = uint32_t(kc);
+                if(G >= stages && !tc::mbar_wait(&sEmpty[G % stages], ((G / stages) - 1) & 1))
+                    raise_error(p.errorFlag, abortLocal);
+                const uint32_t st = s0 + (G % stages) * stageBytes + at;
+#pragma unroll
+                for(int q = 0; q < 4; ++q)
+                    store_piece(st + uint32_t(4 * q) * kBlockPitch, ra[q]);
+#pragma unroll
+                for(int i = 0; i < NB; ++i)
+                    if(mb0 + 4 * i < p.Npad / 8)
+                        store_piece(st + uint32_t(16 + 4 * i) * kBlockPitch, rb[i]);
                 tc::fence_async_smem();
+                if(kc + 1 < nk) // in flight over the barrier and the next wait
+                    fetch();
                 if(__syncthreads_or(abortLocal))
                 {
                     aborted = true;
@@ -1029,18 +1058,17 @@ namespace isaacb
                 {
                     tc::fence_after_sync();
                     const uint32_t stA = s0 + (uint32_t(kc) % stages) * stageBytes;
-                    const uint32_t stB = stA + uint32_t(kStageBytesA);
+                    const uint32_t stB = stA + 16u * kBlockPitch;
 #pragma unroll
                     for(int j = 0; j < kChunkK / 16; ++j)
                     {
-                        const uint64_t ad = tc::smem_desc(stA + uint32_t(j) * 256u, 128u, 1024u);
-                        const uint64_t bd = tc::smem_desc(stB + uint32_t(j) * 256u, 128u, 1024u);
+                        const uint64_t ad = tc::smem_desc(stA + uint32_t(j) * 256u, 128u, kBlockPitch);
+                        const uint64_t bd = tc::smem_desc(stB + uint32_t(j) * 256u, 128u, kBlockPitch);
                         tc::mma_bf16(tmem, ad, bd, idesc, (kc | j) != 0 ? 1u : 0u);
                     }
                     tc::mma_commit(&sEmpty[uint32_t(kc) % stages]);
                 }
             }
-            tc::cp_async_wait<0>();
             if(tid == 0)
                 tc::mma_commit(&sDone);
             if(!aborted && !tc::mbar_wait(&sDone, 0))
@@ -1336,26 +1364,39 @@ namespace isaacb
         return true;
     }
 
+    namespace
+    {
+        template<int NB>
+        void launch_wgrad(const WgradTable& T, int grid, size_t smem, cudaStream_t s)
+        {
+            cudaFuncSetAttribute(k_conv_wgrad<NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+            cudaFuncSetAttribute(k_conv_wgrad<NB>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+            k_conv_wgrad<NB><<<grid, kThreads, smem, s>>>(T);
+        }
+    } // namespace
+
     bool launch_conv_wgrad(const WgradParams* layers, int n, cudaStream_t s)
     {
         WgradTable T{};
         size_t smem = 0, work = 0;
+        int npad = 0;
         for(int l = 0; l < n; ++l)
         {
             WgradParams& p = T.layer[l];
             p = layers[l];
-            // three stages where four would leave room for one CTA per SM only
-            p.stages = 4 * (kStageBytesA + p.Npad * 128) <= 112 * 1024 ? kStages : kStages - 1;
             p.mTiles = (p.Mtot + kTileM - 1) / kTileM;
-            smem = std::max(smem, size_t(p.stages) * (kStageBytesA + size_t(p.Npad) * 128) + 128);
+            npad = std::max(npad, p.Npad);
             work += size_t(p.mTiles) * ((size_t(p.B) * p.Ho * p.Wo + kChunkK - 1) / kChunkK);
         }
-        if(smem > 227 * 1024)
+        if(npad > 256)
             return false;
-        cudaFuncSetAttribute(k_conv_wgrad, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
-        cudaFuncSetAttribute(k_conv_wgrad, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-        // two CTAs fit on an SM; about two such waves of equal work, at least 4 chunks each
-        const int per = std::max(4, int((work + 4 * num_sms() - 1) / (4 * num_sms())));
+        smem = size_t(kWgradStages) * (16 + npad / 8) * kBlockPitch + 128;
+        // beyond 128 columns a CTA holds 256 TMEM columns: no more than two on an SM
+        if(npad > 128)
+            smem = std::max(smem, size_t(80) * 1024);
+        // three CTAs fit on an SM; about four such waves of equal work, at least 4 chunks each
+        const size_t ctas = size_t(12) * num_sms();
+        const int per = std::max(4, int((work + ctas - 1) / ctas));
         for(int l = 0; l < n; ++l)
         {
             WgradParams& p = T.layer[l];
@@ -1365,7 +1406,10 @@ namespace isaacb
         }
         for(int l = n; l < kWgradLayers; ++l)
             T.first[l + 1] = T.first[n];
-        k_conv_wgrad<<<T.first[n], kThreads, smem, s>>>(T);
+        if(npad > 128)
+            launch_wgrad<8>(T, T.first[n], smem, s);
+        else
+            launch_wgrad<4>(T, T.first[n], smem, s);
         return true;
     }
 } // namespace isaacb

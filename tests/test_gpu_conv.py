@@ -167,3 +167,29 @@ def test_dgrad_residue_classes_and_unaligned_dw(case):
          out_h=Ho, out_w=Wo, c_out=Co, ksize=ks, stride=s, pad=pad)
     got = buf.cpu().numpy()[1:].reshape(ks * ks * Ci, npad)[:, :Co]
     _close(got, np.transpose(R.conv_wgrad(x, dy, ks, s, pad), (1, 2, 3, 0)).reshape(ks * ks * Ci, Co), 2e-3, "wgrad")
+
+
+@pytest.mark.parametrize("case", [
+    # B, H, W, Ci, Co, ks, s, pad
+    (1, 5, 3, 8, 8, 1, 1, 0),  # fewer pixels than a chunk, one row block
+    (2, 9, 11, 24, 256, 3, 2, 1),  # the widest output, taps that cross the 128-row tiles
+    (1, 17, 16, 16, 136, 3, 1, 1),  # just past 128 output channels
+    (3, 64, 65, 40, 128, 2, 1, 0),  # many splits, a ragged last chunk
+])
+def test_wgrad_tiles(case):
+    """Weight gradients at the edges of their tiles: rows of channels and taps, columns of
+    output channels, chunks of 64 pixels."""
+    B, H, W, Ci, Co, ks, s, pad = case
+    rng = np.random.default_rng(5)
+    Ho, Wo = R.out_size(H, ks, s, pad), R.out_size(W, ks, s, pad)
+    x = R.round_bf16(rng.standard_normal((B, H, W, Ci)).astype(np.float32))
+    dy = R.round_bf16(rng.standard_normal((B, Ho, Wo, Co)).astype(np.float32))
+    xd, dyd = _bf16(x), _bf16(dy)
+    npad = (Co + 15) // 16 * 16
+    dw = torch.zeros((ks * ks * Ci, npad), dtype=torch.float32, device="cuda")
+    flag = torch.zeros(1, dtype=torch.int32, device="cuda")
+    _run("isaacb_conv_wgrad", x=xd.data_ptr(), dy=dyd.data_ptr(), dw=dw.data_ptr(), batch=B, in_h=H, in_w=W, c_in=Ci,
+         out_h=Ho, out_w=Wo, c_out=Co, ksize=ks, stride=s, pad=pad, error_flag=flag.data_ptr())
+    got = dw.cpu().numpy()[:, :Co]
+    _close(got, np.transpose(R.conv_wgrad(x, dy, ks, s, pad), (1, 2, 3, 0)).reshape(ks * ks * Ci, Co), 2e-3, "wgrad")
+    assert int(flag.item()) == 0
