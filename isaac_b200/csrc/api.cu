@@ -828,7 +828,7 @@ extern "C"
         };
         alloc((void**) &c->lutDev, c->lutHost.size() * sizeof(float));
         alloc((void**) &c->lutPre, c->lutHost.size() * sizeof(float));
-        alloc((void**) &c->psPre, c->lutHost.size() * sizeof(float));
+        alloc((void**) &c->psPre, (c->lutHost.size() + size_t(kMaxSources) * 4) * sizeof(float)); // one entry more each
         if(e == cudaSuccess)
             e = cudaMallocHost((void**) &c->lutPinned, c->lutHost.size() * sizeof(float));
         if(e == cudaSuccess)

@@ -435,26 +435,27 @@ namespace isaacb
     // of once per sample: a = c.w * weight, (c.x * a, c.y * a, c.z * a, a).  These are the
     // products the per-sample loop of PerSourceVolumeRenderKernel forms
     // (lib/isaac/isaac_volume_kernel.hpp:365-377: color.w *= weight; value += color * color.w),
-    // so the sums that use them round the same way.
+    // so the sums that use them round the same way.  A table has ts + 1 entries, the last
+    // two alike, so that an index needs no clamp at the top.
     __global__ void __launch_bounds__(256) k_ps_premultiply(const float4* __restrict__ lut, ActiveSources act, float4* __restrict__ out, int ts)
     {
         const int k = blockIdx.y;
         const int i = blockIdx.x * blockDim.x + threadIdx.x;
-        if(i >= ts)
+        if(i > ts)
             return;
-        const float4 c = __ldg(lut + size_t(act.idx[k]) * ts + i);
+        const float4 c = __ldg(lut + size_t(act.idx[k]) * ts + min(i, ts - 1));
         const float a = c.w * act.weight[k];
-        out[size_t(k) * ts + i] = make_float4(c.x * a, c.y * a, c.z * a, a);
+        out[size_t(k) * (ts + 1) + i] = make_float4(c.x * a, c.y * a, c.z * a, a);
     }
 
-    // the premultiplied entry of lut_index_fast(v, ts) as two FP32 pairs (r, g) and (b, a):
-    // round(clamp(v * ts, 0, ts - 1)) is floor(x + 0.5) with the add rounded down (it never
-    // crosses the next integer), and the floor comes as float bits from a magic-number add
-    // also rounded down; both give lut_index_fast's index for every v, NaN included
-    __device__ __forceinline__ void transfer_entry(const char* biased, float v, float tsf, float tsMax, f2p& rg, f2p& ba)
+    // the premultiplied entry of lut_index_fast(v, ts) as two FP32 pairs (r, g) and (b, a),
+    // v already saturated to [0, 1]: round(clamp(v * ts, 0, ts - 1)) is floor(x + 0.5) with
+    // the add rounded down (it never crosses the next integer), the floor comes as float bits
+    // from a magic-number add also rounded down, and x past ts - 0.5 finds the table's
+    // doubled last entry; both give lut_index_fast's index for every v, NaN included
+    __device__ __forceinline__ void transfer_entry(const char* biased, float v, float tsf, f2p& rg, f2p& ba)
     {
-        const float xi = fminf(fmaxf(v * tsf, 0.0f), tsMax);
-        const float t = __fadd_rd(__fadd_rd(xi, 0.5f), 12582912.0f);
+        const float t = __fadd_rd(__fadd_rd(v * tsf, 0.5f), 12582912.0f);
         const ulonglong2 e = __ldg(reinterpret_cast<const ulonglong2*>(biased + size_t(uint32_t(__float_as_int(t))) * sizeof(float4)));
         rg.v = e.x;
         ba.v = e.y;
@@ -471,10 +472,14 @@ namespace isaacb
     // the sources' quads are all loaded before any is used, pairs of sources share packed
     // FP32 trilinear arithmetic (two lanes, the scalar roundings), and with IDEM the
     // functor chain is skipped.  The weighted premultiplied table entries come from
-    // k_ps_premultiply, found with a 6-instruction index, and value and colour run as
-    // FP32 pairs.  Same operations in the same order per source, so the frame is
-    // bit-identical to the general kernels'.
-    // (4 CTAs per SM: 58 registers without spills, twice the warps of the unbounded 88)
+    // k_ps_premultiply, and value and colour run as FP32 pairs.  Same operations in the same
+    // order per source, so the frame is bit-identical to the general kernels'.
+    // What bounds it is issuing: 212 instructions a sample of four sources, 63 of them packed
+    // ones, which take two issue cycles.  Floors from round-down adds, 32-bit Morton slots,
+    // no clamp at the tables' ends and no counter took 9 % of them out: 512^3, four bf16
+    // sources, 1920 x 1080, 10.47 -> 9.92 ms.  Not issue but loads were spared by keeping the
+    // quads while a ray stays in its slot: 10.18 ms, so that is not done.
+    // (4 CTAs per SM: 55 registers without spills)
     // CLEAN: the frame's only pass; it clears the G-buffer instead of reading it
     template<int DT, bool LINEAR, int NS, bool IDEM, bool CLEAN>
     __global__ void __launch_bounds__(256, 4) k_shade_volume_per_source_n(
@@ -501,7 +506,14 @@ namespace isaacb
 #pragma unroll
                     for(int k = 0; k < NS; ++k)
                         br[k] = act.bricks[k];
-                    const float tsf = float(p.ts), tsMax = float(p.ts - 1);
+                    const float tsf = float(p.ts);
+                    // floor(c) + 1 from the bits of a round-down add, as in march_combined:
+                    // kBits + the apron-shifted coordinate, and kBits is a multiple of 8
+                    constexpr float kFloor = 12582913.0f;
+                    constexpr int kBits = 0x4B400000;
+                    const int hiX = kBits + g.ls[0], hiY = kBits + g.ls[1], hiZ = kBits + g.ls[2];
+                    const uint32_t sy = uint32_t(g.nb[0]) * uint32_t(kSlotsPerBrick), sz = uint32_t(g.nb[1]) * sy;
+                    const uint32_t slot0 = 0u - (uint32_t(kSlotsPerBrick) + sy + sz) * (uint32_t(kBits) >> 3);
                     const f2p fac = f2p_make(m.factor, m.factor);
                     const f2p nz = f2p_make(p.negZero, p.negZero);
                     // value and colour as FP32 pairs (r, g), (b, a); every lane rounds like
@@ -515,34 +527,41 @@ namespace isaacb
                     // entry face is oblique to the view.  Each ray's samples and their
                     // order are unchanged.
                     const int wStart = __reduce_min_sync(__activemask(), m.startSteps);
+                    int last = m.startSteps - 1;
                     for(int i = wStart; i <= m.endSteps; i++)
                     {
                         if(i < m.startSteps)
                             continue;
-                        ++n;
+                        last = i;
                         const float3 pos = march_pos(m, i);
-                        uint32_t q0, q1 = 0;
                         float fx = 0.0f, fy = 0.0f, fz = 0.0f;
-                        size_t above;
+                        int ax, ay, az;
                         if(LINEAR)
                         {
                             const float cx = pos.x - 0.5f, cy = pos.y - 0.5f, cz = pos.z - 0.5f;
-                            fx = cx - floorf(cx);
-                            fy = cy - floorf(cy);
-                            fz = cz - floorf(cz);
-                            const int ix = iclamp(f2i(cx), -1, g.ls[0] - 1);
-                            const int iy = iclamp(f2i(cy), -1, g.ls[1] - 1);
-                            const int iz = iclamp(f2i(cz), -1, g.ls[2] - 1);
-                            q0 = uint32_t(source_slot(g, ix, iy, iz, above));
-                            q1 = uint32_t(above);
+                            const float tx = __fadd_rd(cx, kFloor), ty = __fadd_rd(cy, kFloor), tz = __fadd_rd(cz, kFloor);
+                            fx = cx - (tx - kFloor);
+                            fy = cy - (ty - kFloor);
+                            fz = cz - (tz - kFloor);
+                            // samples lie in [0, size) (legacy_bounds; the positions are
+                            // monotone), so truncation to isaac_int is the floor, but 0 for -1
+                            ax = iclamp(__float_as_int(tx), kBits + 1, hiX);
+                            ay = iclamp(__float_as_int(ty), kBits + 1, hiY);
+                            az = iclamp(__float_as_int(tz), kBits + 1, hiZ);
                         }
                         else
                         {
-                            const int ix = iclamp(f2i(pos.x), 0, g.ls[0] - 1);
-                            const int iy = iclamp(f2i(pos.y), 0, g.ls[1] - 1);
-                            const int iz = iclamp(f2i(pos.z), 0, g.ls[2] - 1);
-                            q0 = uint32_t(source_slot(g, ix, iy, iz, above));
+                            ax = iclamp(__float_as_int(__fadd_rd(pos.x, kFloor)), kBits + 1, hiX);
+                            ay = iclamp(__float_as_int(__fadd_rd(pos.y, kFloor)), kBits + 1, hiY);
+                            az = iclamp(__float_as_int(__fadd_rd(pos.z, kFloor)), kBits + 1, hiZ);
                         }
+                        // source_slot in 32 bits
+                        const uint32_t base = slot0 + (uint32_t(ax) >> 3) * uint32_t(kSlotsPerBrick) + (uint32_t(ay) >> 3) * sy
+                            + (uint32_t(az) >> 3) * sz;
+                        const int lx = ax & 7, ly = ay & 7, lz = az & 7;
+                        const uint32_t xy = base + spread3(lx) + 2u * spread3(ly);
+                        const uint32_t q0 = xy + 4u * spread3(lz);
+                        const uint32_t q1 = lz < 7 ? xy + 4u * spread3(lz + 1) : base + 512u + uint32_t(ly * 8 + lx);
                         float a[NS][4], b[NS][4], val[NS];
 #pragma unroll
                         for(int k = 0; k < NS; ++k)
@@ -566,7 +585,11 @@ namespace isaacb
                                 const f2p z11 = lin2(omz, vz, f2p_make(a[k][3], a[k + 1][3]), f2p_make(b[k][3], b[k + 1][3]), nz);
                                 const f2p A = lin2(omy, vy, z00, z01, nz);
                                 const f2p B = lin2(omy, vy, z10, z11, nz);
-                                f2p_split(lin2(omx, vx, A, B, nz), val[k], val[k + 1]);
+                                float a0, a1, b0, b1;
+                                f2p_split(f2p_mul_exact(A, omx, nz), a0, a1);
+                                f2p_split(f2p_mul_exact(B, vx, nz), b0, b1);
+                                val[k] = __fadd_rn(a0, b0);
+                                val[k + 1] = __fadd_rn(a1, b1);
                             }
                             if(NS & 1)
                             {
@@ -592,7 +615,7 @@ namespace isaacb
                                 result = apply_chain(v, 1, p.ps[act.idx[k]].chain);
                             }
                             f2p erg, eba;
-                            transfer_entry(act.pre[k], result, tsf, tsMax, erg, eba);
+                            transfer_entry(act.pre[k], __saturatef(result), tsf, erg, eba);
                             vrg = f2p_add(vrg, erg);
                             vba = f2p_add(vba, eba);
                         }
@@ -607,6 +630,7 @@ namespace isaacb
                         if(cw > 0.99f)
                             break;
                     }
+                    n = (unsigned long long) (last - m.startSteps + 1);
                     float4 color;
                     f2p_split(crg, color.x, color.y);
                     f2p_split(cba, color.z, color.w);
@@ -623,7 +647,7 @@ namespace isaacb
     template<int DT, bool LINEAR, bool IDEM, bool CLEAN>
     void launch_ps_n(const FrameParams& p, const ActiveSources& act, dim3 grid, cudaStream_t s)
     {
-        k_ps_premultiply<<<dim3((p.ts + 255) / 256, act.n), 256, 0, s>>>(p.lut, act, p.psPre, p.ts);
+        k_ps_premultiply<<<dim3((p.ts + 256) / 256, act.n), 256, 0, s>>>(p.lut, act, p.psPre, p.ts);
         switch(act.n)
         {
         case 1: k_shade_volume_per_source_n<DT, LINEAR, 1, IDEM, CLEAN><<<grid, 256, 0, s>>>(p, act); break;
@@ -691,7 +715,7 @@ namespace isaacb
                 act.idx[act.n] = k;
                 act.bricks[act.n] = S.bricks;
                 act.weight[act.n] = S.weight;
-                act.pre[act.n] = reinterpret_cast<const char*>(p.psPre + size_t(act.n) * p.ts)
+                act.pre[act.n] = reinterpret_cast<const char*>(p.psPre + size_t(act.n) * (p.ts + 1))
                     - size_t(0x4B400000u) * sizeof(float4);
                 act.n++;
                 idem = idem && S.chain.op[0] == OP_IDEM && S.chain.op[1] == OP_IDEM && S.chain.op[2] == OP_IDEM;

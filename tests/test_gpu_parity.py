@@ -299,6 +299,24 @@ def test_per_source_packed_arithmetic_is_exact(dtype, interp, seed):
     assert st["max"] == 0, st
 
 
+@pytest.mark.parametrize("n", [(13, 21, 30), (8, 8, 8), (1, 17, 64)])
+@pytest.mark.parametrize("sources,chain", [(1, "idem"), (2, "idem"), (3, "mul(1.5)|add(-0.25)"), (4, "idem")])
+def test_per_source_edges(n, sources, chain):
+    """The specialised kernel where its indices end: bricks cut by the volume, the first
+    half voxel (floor -1, truncated to 0), values below 0 and above 1, which take the
+    tables' first and doubled last entries.  Equal to the oracle's, pixel for pixel."""
+    rng = np.random.default_rng(sources)
+    fields = [(rng.random(n[::-1]) * 1.6 - 0.3).astype(np.float32) for _ in range(sources)]
+    s = Scene(n=n, fb=(61, 43), volumes=[(f, True) for f in fields], optimized=False)
+    s.transfer = [scenes.transfer_4point(0.7 * i) for i in range(sources)]
+    s.storage = [1] * sources
+    s.functions = [chain] * sources
+    s.weights = [1.5] * sources
+    got, ref, _, _ = _frames(s)
+    st = image_diff(got, ref)
+    assert st["max"] == 0, st
+
+
 @pytest.mark.parametrize("interp", [True, False])
 def test_per_source_iso(interp):
     s = gaussian_pair(n=32, fb=(64, 48), optimized=False, interpolation=interp, iso=[0.3, 0.2])
