@@ -420,7 +420,7 @@ namespace isaacb
         {
             int S; // stride: 1 or 2
             int HWp; // entries between runs (per parity plane for stride 2)
-            int HWn; // entries a run needs (<= HWp; HWp is padded to 8 for TMA destinations)
+            int HWn; // entries a run needs (<= HWp, which holds a full tile's, padded to 8 for TMA destinations)
             int stages; // halo buffers: 1 or 2
             int rowB; // swizzled staging: bytes per staged pixel (Cg * 2 = 32, 64 or 128); 0 = chunked runs
             // implicit concatenation by TMA (1x1, xUp): channel chunks of cwc (coarse) and cwf
@@ -428,36 +428,108 @@ namespace isaacb
             int cwc, cwf;
         };
 
-        __host__ __device__ inline RowGeom row_geom(int stride, int ks, int pad, int stages, bool tma = false)
+        // width: output pixels of a row (of a parity's, for stride-2 input gradients)
+        inline RowGeom row_geom(int stride, int ks, int pad, int width, int stages, bool tma)
         {
             RowGeom g;
             g.S = stride;
-            g.HWn = stride == 1 ? kTileM + 2 * pad : kTileM + (ks - 1) / 2 + 1;
+            const int more = stride == 1 ? 2 * pad : (ks - 1) / 2 + 1;
+            // a row narrower than a tile needs its own columns only; the MMA's other rows read
+            // what the buffer holds, and nothing stores them
+            g.HWn = (width < kTileM ? width : kTileM) + more;
             // a TMA destination starts on a 128-byte boundary: runs of a multiple of 8 entries
-            g.HWp = tma ? (g.HWn + 7) / 8 * 8 : g.HWn;
+            g.HWp = tma ? (kTileM + more + 7) / 8 * 8 : kTileM + more;
             g.stages = stages;
             g.rowB = 0;
             g.cwc = g.cwf = 0;
             return g;
         }
+        // Input gradients of stride 2 go by output parity: output row y takes the tap rows
+        // ty = (y + pad) mod 2, + 2, ... at input rows (y + pad - ty) / 2, and its even and
+        // odd columns x = 2u, 2u + 1 are two stride-1 convolutions in u over the same halo
+        // (taps tx of their parity at input column u + (x mod 2 + pad - tx) / 2, within one
+        // of u), accumulated side by side in TMEM.
+        __host__ __device__ inline bool parity_tiles(const ConvGemmParams& p)
+        {
+            return p.transposed && p.stride == 2;
+        }
+        // input rows of a tile's halo, at most
+        __host__ __device__ inline int halo_rows(const ConvGemmParams& p)
+        {
+            return parity_tiles(p) ? (p.ks + 1) / 2 : p.ks;
+        }
+        __host__ __device__ inline int row_tile_count(const ConvGemmParams& p)
+        {
+            return ((parity_tiles(p) ? (p.Wo + 1) / 2 : p.Wo) + kTileM - 1) / kTileM;
+        }
+        __host__ __device__ inline int accumulator_columns(const ConvGemmParams& p)
+        {
+            return parity_tiles(p) ? 2 * p.Npad : p.Npad;
+        }
+        inline RowGeom row_geom_of(const ConvGemmParams& p, int stages, bool tma)
+        {
+            return parity_tiles(p) ? row_geom(1, p.ks, 1, (p.Wo + 1) / 2, stages, tma) : row_geom(p.stride, p.ks, p.pad, p.Wo, stages, tma);
+        }
 
-        // Epilogue of one 128-pixel output tile (row y of image b, column tile xt): this
-        // thread's pixel px, accumulator columns [cBeg, cBeg + colsPer) of the TMEM tile at
-        // tAcc (this warp's lanes); bias, ReLU, mask, then the bf16 / FP32 store.
-        __device__ __forceinline__ void row_epilogue(
+        // 16 bytes, or zeros; issued where it stands
+        __device__ __forceinline__ uint4 load_piece(const bf16* src, bool ok)
+        {
+            uint4 v = make_uint4(0, 0, 0, 0);
+            asm volatile(
+                "{\n\t.reg .pred p;\n\tsetp.ne.s32 p, %5, 0;\n\t@p ld.global.nc.v4.u32 {%0, %1, %2, %3}, [%4];\n\t}"
+                : "+r"(v.x), "+r"(v.y), "+r"(v.z), "+r"(v.w)
+                : "l"(src), "r"(int(ok)));
+            return v;
+        }
+        // 16 bytes of a tensor that this kernel also writes
+        __device__ __forceinline__ uint4 load_own(const bf16* src)
+        {
+            uint4 v;
+            asm volatile("ld.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(src) : "memory");
+            return v;
+        }
+
+        // Epilogue of one 128-pixel output tile (row y of image b): this thread's column x,
+        // accumulator columns [cBeg, cBeg + colsPer) of the TMEM tile at tAcc (this warp's
+        // lanes), which are complete when `full` reaches `phase`; bias, ReLU, mask, then the
+        // bf16 / FP32 store.  What it reads of a mask or of the tensor it adds to is loaded one
+        // group of columns ahead, the first group's before the wait: with each group's loads
+        // after the last one's stores a tile waited for memory once a group (the three
+        // stride-2 gradients of a step of 16 128 x 128 pairs: 136 -> 92 us).
+        // False when the wait ran out.
+        template<bool READS>
+        __device__ __forceinline__ bool row_epilogue(
             const ConvGemmParams& p,
+            uint64_t* full,
+            uint32_t phase,
             uint32_t tAcc,
-            int xt,
+            int x,
             int b,
             int y,
-            int px,
             int cBeg,
             int colsPer,
             const float* sBias)
         {
-            const int x = xt * kTileM + px;
             const bool valid = x < p.Wo;
             const size_t pix = (size_t(b) * p.Ho + y) * p.Wo + x;
+            const int cEnd = min(cBeg + colsPer, p.Cout);
+            const bool masked = READS && valid && p.mask, added = READS && valid && p.accumulate && !p.yf;
+            uint4 mk[2] = {}, ad[2] = {};
+            auto fetch = [&](int c16) {
+#pragma unroll
+                for(int hh = 0; hh < 2; ++hh)
+                {
+                    const int c0 = c16 + 8 * hh;
+                    if(masked && c0 < cEnd)
+                        mk[hh] = load_piece(p.mask + pix * p.Cout + c0, true);
+                    if(added && c0 < cEnd)
+                        ad[hh] = load_own(p.y + pix * p.Cout + c0);
+                }
+            };
+            fetch(cBeg);
+            if(!tc::mbar_wait(full, phase))
+                return false;
+            tc::fence_after_sync();
             // 16 accumulator columns per TMEM wait (8 where a column group ends)
             for(int c16 = cBeg; c16 < cBeg + colsPer; c16 += 16)
             {
@@ -468,13 +540,15 @@ namespace isaacb
                 if(two)
                     tc::tmem_ld8(ta + 8u, v[1]);
                 tc::tmem_wait_ld();
+                const uint4 mkNow[2] = {mk[0], mk[1]}, adNow[2] = {ad[0], ad[1]};
+                fetch(c16 + 16);
                 if(!valid)
                     continue;
 #pragma unroll
                 for(int hh = 0; hh < 2; ++hh)
                 {
                     const int c0 = c16 + 8 * hh;
-                    if(c0 >= p.Cout || (hh == 1 && !two))
+                    if(c0 >= cEnd)
                         break;
                     float(&w)[8] = v[hh];
                     const size_t o = pix * p.Cout + c0;
@@ -490,18 +564,18 @@ namespace isaacb
                         for(int k = 0; k < 8; ++k)
                             w[k] = fmaxf(w[k], 0.0f);
                     }
-                    if(p.mask)
+                    if(READS && p.mask)
                     {
-                        float mk[8];
-                        unpack_bf16x8(__ldg(reinterpret_cast<const uint4*>(p.mask + o)), mk);
+                        float m8[8];
+                        unpack_bf16x8(mkNow[hh], m8);
 #pragma unroll
                         for(int k = 0; k < 8; ++k)
-                            w[k] = mk[k] > 0.0f ? w[k] : 0.0f;
+                            w[k] = m8[k] > 0.0f ? w[k] : 0.0f;
                     }
                     if(p.yf)
                     {
                         float4* dst = reinterpret_cast<float4*>(p.yf + o);
-                        if(p.accumulate)
+                        if(READS && p.accumulate)
                         {
                             const float4 u = dst[0], t2 = dst[1];
                             w[0] += u.x, w[1] += u.y, w[2] += u.z, w[3] += u.w;
@@ -512,22 +586,24 @@ namespace isaacb
                     }
                     else
                     {
-                        uint4* dst = reinterpret_cast<uint4*>(p.y + o);
-                        if(p.accumulate)
+                        if(READS && p.accumulate)
                         {
                             float u[8];
-                            unpack_bf16x8(*dst, u);
+                            unpack_bf16x8(adNow[hh], u);
 #pragma unroll
                             for(int k = 0; k < 8; ++k)
                                 w[k] += u[k];
                         }
-                        *dst = pack_bf16x8(w);
+                        *reinterpret_cast<uint4*>(p.y + o) = pack_bf16x8(w);
                     }
                 }
             }
+            return true;
         }
 
-        template<bool TMA>
+        // PAR: parity_tiles.  READS: the epilogue reads a mask or the tensor it adds to.  Each is
+        // compiled apart: a plain convolution keeps three blocks an SM by registers.
+        template<bool TMA, bool PAR, bool READS>
         __global__ void __launch_bounds__(row_threads<TMA>(), 1)
             k_conv_row(const __grid_constant__ ConvGemmParams p, const RowGeom rg, const __grid_constant__ CUtensorMap tmap,
                        const __grid_constant__ CUtensorMap tmapUp)
@@ -544,6 +620,8 @@ namespace isaacb
             const uint32_t sB = tc::smem_addr(base);
             const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
             const int pad = p.pad, ks = p.ks, S = rg.S, HWp = rg.HWp, NS = rg.stages;
+            constexpr bool par = PAR;
+            const int rows = halo_rows(p), left = par ? 1 : pad; // columns of the halo before the tile's first
             const int nC = p.Cg / 8;
             const uint32_t runBytes = uint32_t(HWp) * 16u;
             // swizzled staging: each input row is HWp pixels of rowB bytes, the row buffers
@@ -552,10 +630,10 @@ namespace isaacb
             const bool cat = TMA && rg.cwc != 0;
             const uint32_t swSpan = cat ? 1024u : 8u * uint32_t(rowB);
             const uint32_t rowPitch = rowB ? (uint32_t(HWp * rowB) + swSpan - 1u) / swSpan * swSpan : 0u;
-            const uint32_t haloBytes = rowB ? uint32_t(ks * S) * rowPitch : uint32_t(ks * nC * S) * runBytes;
+            const uint32_t haloBytes = rowB ? uint32_t(rows * S) * rowPitch : uint32_t(rows * nC * S) * runBytes;
             const uint32_t wEnd = sB + uint32_t(p.Npad) * uint32_t(p.Kpad) * 2u;
             const uint32_t sH = (rowB || cat) ? (wEnd + swSpan - 1u) / swSpan * swSpan : wEnd;
-            const uint32_t half = tmem_columns(p.Npad);
+            const uint32_t half = tmem_columns(accumulator_columns(p));
             const uint32_t cols = 2 * half;
             if(warp == 0)
             {
@@ -610,7 +688,7 @@ namespace isaacb
                     tc::tmem_dealloc(tmem, cols);
                 return;
             }
-            const int tilesPerRow = (p.Wo + kTileM - 1) / kTileM;
+            const int tilesPerRow = row_tile_count(p);
             const int nTiles = p.B * p.Ho * tilesPerRow;
 
             if(TMA && warp == 9)
@@ -620,14 +698,12 @@ namespace isaacb
                 // (8j, x0 - pad, row, b).  Stride 2: map (C, 2, W/2, H, B), the column split
                 // into its parity and half, box (8, 1, HWn, 1, 1) at (8j, c & 1, c >> 1, row,
                 // b) with c = 2*x0 - pad + q.  Swizzled staging (16-64 channels): one box of
-                // all channels per run, (C, HWp, 1, 1) at (0, x0 - pad, row, b) or
-                // (C, 1, HWp, 1, 1) at (0, c & 1, c >> 1, row, b), written with the map's
+                // all channels per run, (C, HWn, 1, 1) at (0, x0 - pad, row, b) or
+                // (C, 1, HWn, 1, 1) at (0, c & 1, c >> 1, row, b), written with the map's
                 // 32/64/128-byte swizzle.  Rows and columns outside the image read zeros.
                 if(lane == 0)
                 {
-                    const uint32_t txBytes = cat ? uint32_t(kTileM * p.Cg * 2)
-                        : rowB                   ? uint32_t(ks * S * HWp * rowB)
-                                                 : uint32_t(ks * nC * S * rg.HWn) * 16u;
+                    const uint32_t rowTx = rowB ? uint32_t(S * rg.HWn * rowB) : uint32_t(nC * S * rg.HWn) * 16u;
                     int i = 0;
                     for(int tile = blockIdx.x; tile < nTiles; tile += gridDim.x, ++i)
                     {
@@ -643,7 +719,9 @@ namespace isaacb
                         const int y = row % p.Ho, b = row / p.Ho;
                         const int x0 = xt * kTileM;
                         const uint32_t st = sH + uint32_t(s) * haloBytes;
-                        tc::mbar_arrive_expect_tx(&sFull[s], txBytes);
+                        const int ty0 = par ? (y + pad) & 1 : 0;
+                        const int nRows = par ? (ks - ty0 + 1) / 2 : ks;
+                        tc::mbar_arrive_expect_tx(&sFull[s], cat ? uint32_t(kTileM * p.Cg * 2) : uint32_t(nRows) * rowTx);
                         if(cat)
                         {
                             // tile rows in parity order: row m < 64 is pixel x0 + 2m, row 64 + m
@@ -665,13 +743,13 @@ namespace isaacb
                             }
                             continue;
                         }
-                        for(int ty = 0; ty < ks; ++ty)
+                        for(int ty = 0; ty < nRows; ++ty)
                         {
-                            const int iy = p.transposed ? y + pad - ty : S * y - pad + ty;
+                            const int iy = par ? ((y + pad - ty0) >> 1) - ty : p.transposed ? y + pad - ty : S * y - pad + ty;
                             if(rowB)
                             {
                                 if(S == 1)
-                                    tc::tma_load_4d(st + uint32_t(ty) * rowPitch, &tmap, 0, x0 - pad, iy, b, &sFull[s]);
+                                    tc::tma_load_4d(st + uint32_t(ty) * rowPitch, &tmap, 0, x0 - left, iy, b, &sFull[s]);
                                 else
                                     for(int q = 0; q < 2; ++q)
                                     {
@@ -686,7 +764,7 @@ namespace isaacb
                                 {
                                     const uint32_t dst = st + uint32_t((ty * nC + j) * S + q) * runBytes;
                                     if(S == 1)
-                                        tc::tma_load_4d(dst, &tmap, 8 * j, x0 - pad, iy, b, &sFull[s]);
+                                        tc::tma_load_4d(dst, &tmap, 8 * j, x0 - left, iy, b, &sFull[s]);
                                     else
                                     {
                                         const int c = 2 * x0 - pad + q;
@@ -721,9 +799,11 @@ namespace isaacb
                     // offset; consecutive threads take consecutive 16-byte pieces of global memory and
                     // step by 128 pieces, so j and c advance by fixed amounts
                     const int perRow = nC * S * HWp;
-                    for(int ty = 0; ty < ks; ++ty)
+                    const int ty0 = par ? (y + pad) & 1 : 0;
+                    const int nRows = par ? (ks - ty0 + 1) / 2 : ks;
+                    for(int ty = 0; ty < nRows; ++ty)
                     {
-                        const int iy = p.transposed ? y + pad - ty : S * y - pad + ty;
+                        const int iy = par ? ((y + pad - ty0) >> 1) - ty : p.transposed ? y + pad - ty : S * y - pad + ty;
                         const bool rowOk = iy >= 0 && iy < p.H;
                         // implicit concatenation: chunks below nUp come from the coarse tensor at
                         // the nearest coarse pixel, the rest from x, whose pixels hold cX channels
@@ -737,7 +817,7 @@ namespace isaacb
                         int j = pt % nC, c = pt / nC;
                         for(int g = pt; g < perRow; g += 128)
                         {
-                            const int ix = S * x0 - pad + c;
+                            const int ix = S * x0 - left + c;
                             const int q = c & (S - 1), idx = S == 1 ? c : (c >> 1);
                             const bool ok = rowOk && ix >= 0 && ix < p.W;
                             const bf16* src = !ok ? p.x
@@ -779,7 +859,10 @@ namespace isaacb
                         tc::fence_async_smem();
                         tc::fence_after_sync();
                         const uint32_t st = sH + uint32_t(s) * haloBytes;
-                        const uint32_t d = tmem + uint32_t(a) * half;
+                        const uint32_t dTile = tmem + uint32_t(a) * half;
+                        const int y = (tile / tilesPerRow) % p.Ho;
+                        const int ty0 = par ? (y + pad) & 1 : 0, nRows = par ? (ks - ty0 + 1) / 2 : ks;
+                        const int nPar = par ? 2 : 1, tapStep = nPar;
                         // descriptors differ only in their start field (16-byte units), so the
                         // loop adds offsets to two base descriptors
                         const uint64_t aBase = tc::smem_desc(st, lboA, 128u);
@@ -802,7 +885,7 @@ namespace isaacb
                                     for(int jp = 0; jp < cw / 16; ++jp)
                                     {
                                         const uint32_t addr = region + uint32_t(jp) * 32u;
-                                        tc::mma_bf16(d, swDesc | uint64_t((addr >> 4) & 0x3FFFu), bBase + bOff, idesc, acc);
+                                        tc::mma_bf16(dTile, swDesc | uint64_t((addr >> 4) & 0x3FFFu), bBase + bOff, idesc, acc);
                                         acc = 1;
                                         bOff += 16u;
                                     }
@@ -819,13 +902,15 @@ namespace isaacb
                             // copy wrote it, so the base-offset field stays 0.
                             const uint64_t swDesc = (tc::smem_desc(0, 16u, swSpan) & ~uint64_t(0x3FFF))
                                 | (uint64_t(rowB == 32 ? 6 : rowB == 64 ? 4 : 2) << 61);
-                            for(int ty = 0; ty < ks; ++ty)
-                                for(int tx = 0; tx < ks; ++tx)
+                            for(int cx = 0; cx < nPar; ++cx, acc = 0)
+                            for(int ty = 0; ty < nRows; ++ty)
+                                for(int tx = par ? (cx + pad) & 1 : 0; tx < ks; tx += tapStep)
                                 {
-                                    const int col = p.transposed ? 2 * pad - tx : tx;
+                                    const int col = par ? ((cx + pad - tx) >> 1) + 1 : p.transposed ? 2 * pad - tx : tx;
                                     const int q = col & (S - 1), idx0 = S == 1 ? col : (col >> 1);
+                                    const uint32_t d = dTile + uint32_t(cx * p.Npad);
                                     uint32_t addr = st + uint32_t(ty * S + q) * rowPitch + uint32_t(idx0 * rowB);
-                                    uint32_t bOff = uint32_t((ty * ks + tx) * p.Cg);
+                                    uint32_t bOff = uint32_t(((ty0 + tapStep * ty) * ks + tx) * p.Cg);
                                     for(int jp = 0; jp < nC / 2; ++jp)
                                     {
                                         tc::mma_bf16(d, swDesc | uint64_t((addr >> 4) & 0x3FFFu), bBase + bOff, idesc, acc);
@@ -836,13 +921,15 @@ namespace isaacb
                                 }
                         }
                         else
-                        for(int ty = 0; ty < ks; ++ty)
-                            for(int tx = 0; tx < ks; ++tx)
+                        for(int cx = 0; cx < nPar; ++cx, acc = 0)
+                        for(int ty = 0; ty < nRows; ++ty)
+                            for(int tx = par ? (cx + pad) & 1 : 0; tx < ks; tx += tapStep)
                             {
-                                const int col = p.transposed ? 2 * pad - tx : tx;
+                                const int col = par ? ((cx + pad - tx) >> 1) + 1 : p.transposed ? 2 * pad - tx : tx;
                                 const int q = col & (S - 1), idx0 = S == 1 ? col : (col >> 1);
+                                const uint32_t d = dTile + uint32_t(cx * p.Npad);
                                 uint32_t aOff = uint32_t((ty * nC * S + q) * HWp + idx0);
-                                uint32_t bOff = uint32_t((ty * ks + tx) * p.Cg);
+                                uint32_t bOff = uint32_t(((ty0 + tapStep * ty) * ks + tx) * p.Cg);
                                 for(int jp = 0; jp < nC / 2; ++jp)
                                 {
                                     tc::mma_bf16(d, aBase + aOff, bBase + bOff, idesc, acc);
@@ -865,25 +952,31 @@ namespace isaacb
                 // epilogue: thread = TMEM lane = pixel of the tile; with TMA two groups of four
                 // warps split the accumulator columns
                 const uint32_t lane0 = uint32_t(warp & 3) * 32u;
-                const int colsPer = TMA ? p.Npad / 2 : p.Npad; // a multiple of 8
-                const int cBeg = TMA ? (warp >> 2) * colsPer : 0;
+                const int group = TMA ? warp >> 2 : 0;
+                const int colsPer = TMA && !par ? p.Npad / 2 : p.Npad; // a multiple of 8
+                const int cBeg = group * colsPer;
                 int i = 0;
                 for(int tile = blockIdx.x; tile < nTiles; tile += gridDim.x, ++i)
                 {
                     const int a = i & 1;
-                    if(!tc::mbar_wait(&sAccFull[a], uint32_t(i >> 1) & 1u))
+                    const int xt = tile % tilesPerRow;
+                    const int row = tile / tilesPerRow;
+                    const int m = tid & 127;
+                    const int px = cat ? (m < 64 ? 2 * m : 2 * (m - 64) + 1) : m; // parity-ordered rows
+                    const uint32_t tAcc = tmem + uint32_t(a) * half + (lane0 << 16), phase = uint32_t(i >> 1) & 1u;
+                    bool ok = true;
+                    if(par) // a parity's columns each, with TMA a group of warps each
+                        for(int cx = group; cx < 2; cx += TMA ? 2 : 1)
+                            ok = ok && row_epilogue<READS>(p, &sAccFull[a], phase, tAcc + uint32_t(cx * p.Npad), 2 * (xt * kTileM + px) + cx,
+                                                    row / p.Ho, row % p.Ho, 0, p.Npad, sBias);
+                    else
+                        ok = row_epilogue<READS>(p, &sAccFull[a], phase, tAcc, xt * kTileM + px, row / p.Ho, row % p.Ho, cBeg, colsPer, sBias);
+                    if(!ok)
                     {
                         if(p.errorFlag)
                             atomicExch(p.errorFlag, 1);
                         break;
                     }
-                    tc::fence_after_sync();
-                    const int xt = tile % tilesPerRow;
-                    const int row = tile / tilesPerRow;
-                    const int m = tid & 127;
-                    const int px = cat ? (m < 64 ? 2 * m : 2 * (m - 64) + 1) : m; // parity-ordered rows
-                    row_epilogue(p, tmem + uint32_t(a) * half + (lane0 << 16), xt, row / p.Ho, row % p.Ho, px, cBeg,
-                                 colsPer, sBias);
                     tc::fence_before_sync();
                     tc::mbar_arrive(&sAccEmpty[a]);
                 }
@@ -900,16 +993,6 @@ namespace isaacb
         // that the 8 lanes of a 16-byte store phase (2 pixels x 4 blocks) meet all banks
         constexpr uint32_t kBlockPitch = kChunkK * 16 + 32;
 
-        // 16 bytes, or zeros; issued where it stands
-        __device__ __forceinline__ uint4 load_piece(const bf16* src, bool ok)
-        {
-            uint4 v = make_uint4(0, 0, 0, 0);
-            asm volatile(
-                "{\n\t.reg .pred p;\n\tsetp.ne.s32 p, %5, 0;\n\t@p ld.global.nc.v4.u32 {%0, %1, %2, %3}, [%4];\n\t}"
-                : "+r"(v.x), "+r"(v.y), "+r"(v.z), "+r"(v.w)
-                : "l"(src), "r"(int(ok)));
-            return v;
-        }
         __device__ __forceinline__ void store_piece(uint32_t at, uint4 v)
         {
             asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(at), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
@@ -1141,7 +1224,13 @@ namespace isaacb
         if(p.xUp && (p.ks != 1 || p.stride != 1 || p.upC % 8 != 0 || p.transposed))
             return false;
         return p.Cg % 16 == 0 && p.Npad <= 256
-            && ((p.stride == 1 && 2 * p.pad == p.ks - 1) || (p.stride == 2 && !p.transposed && p.ks <= 3 && p.pad <= 1));
+            && ((p.stride == 1 && 2 * p.pad == p.ks - 1) || (p.stride == 2 && !p.transposed && p.ks <= 3 && p.pad <= 1)
+                // both parities' accumulators, twice, fill 512 TMEM columns at 128; of one tap
+                // a parity would have none; and a narrow row leaves most of a tile's pixels
+                // unused: a 2x2 gradient of 32 columns took 27 us here and 22 us by residue
+                // classes (k_conv_gemm), a 3x3 of 64 columns 36 and 67 us, of 128 columns 29
+                // and 90 us
+                || (parity_tiles(p) && p.Npad <= 128 && (p.ks == 2 || p.ks == 3) && p.pad <= 1 && p.Wo >= 64));
     }
     // Swizzled staging for the TMA producer: 16, 32 or 64 channels, each run (an input row,
     // or one parity plane of it at stride 2) one box of Cg * 2-byte pixels, instead of one
@@ -1153,14 +1242,14 @@ namespace isaacb
     }
     size_t conv_row_smem(const ConvGemmParams& p, int stages, bool tma = false)
     {
-        const RowGeom g = row_geom(p.stride, p.ks, p.pad, stages, tma);
+        const RowGeom g = row_geom_of(p, stages, tma);
         const int rowB = tma ? swizzle_row_bytes(p) : 0;
         if(rowB)
         {
             const size_t span = size_t(8) * rowB, pitch = (size_t(g.HWp) * rowB + span - 1) / span * span;
-            return size_t(p.Npad) * p.Kpad * 2 + span + size_t(stages) * p.ks * g.S * pitch + 128;
+            return size_t(p.Npad) * p.Kpad * 2 + span + size_t(stages) * halo_rows(p) * g.S * pitch + 128;
         }
-        return size_t(p.Npad) * p.Kpad * 2 + size_t(stages) * p.ks * (p.Cg / 8) * g.S * g.HWp * 16 + 128;
+        return size_t(p.Npad) * p.Kpad * 2 + size_t(stages) * halo_rows(p) * (p.Cg / 8) * g.S * g.HWp * 16 + 128;
     }
 
     namespace
@@ -1200,7 +1289,7 @@ namespace isaacb
                 {
                     cuuint64_t dims[4] = {C, W, H, B};
                     cuuint64_t strides[3] = {C * 2, W * C * 2, H * W * C * 2};
-                    cuuint32_t box[4] = {cuuint32_t(C), cuuint32_t(g.HWp), 1, 1};
+                    cuuint32_t box[4] = {cuuint32_t(C), cuuint32_t(g.HWn), 1, 1};
                     r = enc(&m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<bf16*>(p.x), dims, strides, box, estr,
                             CU_TENSOR_MAP_INTERLEAVE_NONE, sw, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
@@ -1211,7 +1300,7 @@ namespace isaacb
                         return false; // the parity split views W as (W/2, 2)
                     cuuint64_t dims[5] = {C, 2, W / 2, H, B};
                     cuuint64_t strides[4] = {C * 2, 2 * C * 2, W * C * 2, H * W * C * 2};
-                    cuuint32_t box[5] = {cuuint32_t(C), 1, cuuint32_t(g.HWp), 1, 1};
+                    cuuint32_t box[5] = {cuuint32_t(C), 1, cuuint32_t(g.HWn), 1, 1};
                     r = enc(&m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, const_cast<bf16*>(p.x), dims, strides, box, estr,
                             CU_TENSOR_MAP_INTERLEAVE_NONE, sw, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
@@ -1285,19 +1374,19 @@ namespace isaacb
                 == CUDA_SUCCESS;
         }
 
-        template<bool TMA>
-        void launch_row(const ConvGemmParams& p, int stages, const CUtensorMap& m, cudaStream_t s, int rowB = 0,
-                        const CUtensorMap* m2 = nullptr, int cwc = 0, int cwf = 0)
+        template<bool TMA, bool PAR, bool READS>
+        void launch_row_as(const ConvGemmParams& p, int stages, const CUtensorMap& m, cudaStream_t s, int rowB,
+                           const CUtensorMap* m2, int cwc, int cwf)
         {
             const size_t smem = conv_row_smem(p, stages, TMA) + (cwc ? 1024 : 0);
-            cudaFuncSetAttribute(k_conv_row<TMA>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
-            cudaFuncSetAttribute(k_conv_row<TMA>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-            const int tiles = p.B * p.Ho * ((p.Wo + kTileM - 1) / kTileM);
-            int perSm = ctas_per_sm(k_conv_row<TMA>, row_threads<TMA>(), smem);
-            while(perSm > 1 && perSm * 2 * int(tmem_columns(p.Npad)) > 512)
+            cudaFuncSetAttribute(k_conv_row<TMA, PAR, READS>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+            cudaFuncSetAttribute(k_conv_row<TMA, PAR, READS>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+            const int tiles = p.B * p.Ho * row_tile_count(p);
+            int perSm = ctas_per_sm(k_conv_row<TMA, PAR, READS>, row_threads<TMA>(), smem);
+            while(perSm > 1 && perSm * 2 * int(tmem_columns(accumulator_columns(p))) > 512)
                 --perSm;
             const int slots = num_sms() * perSm;
-            RowGeom g = row_geom(p.stride, p.ks, p.pad, stages, TMA);
+            RowGeom g = row_geom_of(p, stages, TMA);
             g.rowB = TMA ? rowB : 0;
             g.cwc = TMA ? cwc : 0;
             g.cwf = TMA ? cwf : 0;
@@ -1311,7 +1400,18 @@ namespace isaacb
             attr[0].val.programmaticStreamSerializationAllowed = 1;
             cfg.attrs = attr;
             cfg.numAttrs = p.pdl ? 1 : 0;
-            cudaLaunchKernelEx(&cfg, k_conv_row<TMA>, p, g, m, m2 ? *m2 : m);
+            cudaLaunchKernelEx(&cfg, k_conv_row<TMA, PAR, READS>, p, g, m, m2 ? *m2 : m);
+        }
+        template<bool TMA>
+        void launch_row(const ConvGemmParams& p, int stages, const CUtensorMap& m, cudaStream_t s, int rowB = 0,
+                        const CUtensorMap* m2 = nullptr, int cwc = 0, int cwf = 0)
+        {
+            if(parity_tiles(p))
+                launch_row_as<TMA, true, true>(p, stages, m, s, rowB, m2, cwc, cwf);
+            else if(p.mask || p.accumulate)
+                launch_row_as<TMA, false, true>(p, stages, m, s, rowB, m2, cwc, cwf);
+            else
+                launch_row_as<TMA, false, false>(p, stages, m, s, rowB, m2, cwc, cwf);
         }
     } // namespace
 
@@ -1326,7 +1426,7 @@ namespace isaacb
             if(conv_row_smem(p, stages, true) <= 227 * 1024)
             {
                 CUtensorMap m{};
-                RowGeom g = row_geom(p.stride, p.ks, p.pad, stages, true);
+                RowGeom g = row_geom_of(p, stages, true);
                 g.rowB = swizzle_row_bytes(p);
                 CUtensorMap m2{};
                 if(g_rowTma && p.xUp && conv_row_smem(p, stages, true) + 1024 <= 227 * 1024 && encode_cat_maps(p, g, m, m2))

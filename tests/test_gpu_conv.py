@@ -193,3 +193,43 @@ def test_wgrad_tiles(case):
     got = dw.cpu().numpy()[:, :Co]
     _close(got, np.transpose(R.conv_wgrad(x, dy, ks, s, pad), (1, 2, 3, 0)).reshape(ks * ks * Ci, Co), 2e-3, "wgrad")
     assert int(flag.item()) == 0
+
+
+@pytest.mark.parametrize("case", [
+    # B, H, W (of the gradient's output), Ci, Co, ks, pad
+    (2, 5, 256, 32, 64, 3, 1),  # both parities fill a tile exactly
+    (1, 6, 257, 32, 64, 3, 1),  # one even column more
+    (1, 7, 515, 16, 16, 3, 0),  # three tiles, odd sizes, no padding
+    (1, 4, 258, 96, 96, 2, 0),  # 2x2: one tap a parity, channels in chunks of 8
+    (1, 3, 65, 128, 32, 2, 1),  # the widest accumulators, 2x2 with padding
+    (2, 9, 64, 64, 96, 3, 1),  # the narrowest rows that take row tiles
+])
+def test_stride2_dgrad_parity_tiles(case):
+    """Input gradients of stride 2 on row tiles, the output's even and odd columns side by
+    side: TMA and cp.async producers fill the same halo, so they agree bit for bit, and
+    with the reference's sum, masked and accumulated."""
+    B, H, W, Ci, Co, ks, pad = case
+    rng = np.random.default_rng(9)
+    Ho, Wo = R.out_size(H, ks, 2, pad), R.out_size(W, ks, 2, pad)
+    w = R.round_bf16((rng.standard_normal((Co, ks, ks, Ci)) / np.sqrt(ks * ks * Ci)).astype(np.float32))
+    dy = R.round_bf16(rng.standard_normal((B, Ho, Wo, Co)).astype(np.float32))
+    prev = rng.standard_normal((B, H, W, Ci)).astype(np.float32)
+    mask = R.round_bf16(rng.standard_normal((B, H, W, Ci)).astype(np.float32))
+    wt, dyd, md = _bf16(R.pack_weights_transposed(w)), _bf16(dy), _bf16(mask)
+    flag = torch.zeros(1, dtype=torch.int32, device="cuda")
+    lib = _lib.load()
+    outs = []
+    try:
+        for tma in (1, 0):
+            _lib.check(lib.isaacb_conv_set_producer(tma))
+            dx = torch.from_numpy(prev.copy()).cuda()
+            _run("isaacb_conv_forward", x=dyd.data_ptr(), w=wt.data_ptr(), y_f32=dx.data_ptr(), mask=md.data_ptr(), batch=B,
+                 in_h=Ho, in_w=Wo, c_in=Co, out_h=H, out_w=W, c_out=Ci, ksize=ks, stride=2, pad=pad, transposed=1,
+                 accumulate=1, error_flag=flag.data_ptr())
+            torch.cuda.synchronize()
+            outs.append(dx.cpu())
+    finally:
+        _lib.check(lib.isaacb_conv_set_producer(1))
+    assert torch.equal(outs[0], outs[1])
+    _close(outs[0].numpy(), np.where(mask > 0, R.conv_dgrad(dy, w, (H, W), 2, pad), 0.0) + prev, 2e-3, "dgrad")
+    assert int(flag.item()) == 0
