@@ -205,17 +205,20 @@ namespace
         float invCount)
     {
         float acc = 0.0f;
-        const size_t n = size_t(B) * h * w;
-        for(size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x; i < n; i += size_t(gridDim.x) * blockDim.x)
+        // a batch holds at most 2^26 pixels (isaacb_recon_create), so 32-bit indices suffice
+        const uint32_t n = uint32_t(B) * uint32_t(h) * uint32_t(w);
+        for(uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
         {
-            const int x = int(i % w);
-            const size_t t = i / w;
-            const int y = int(t % h), b = int(t / h);
+            const uint32_t t = i / uint32_t(w);
+            const int x = int(i - t * uint32_t(w));
+            const int b = int(t / uint32_t(h)), y = int(t - uint32_t(b) * uint32_t(h));
             const int f = index ? __ldg(index + b) : b;
             const uchar4* lo = reinterpret_cast<const uchar4*>(low) + size_t(f) * h * w;
             const uchar4* hi = reinterpret_cast<const uchar4*>(high) + size_t(f) * 4 * h * w;
             float rv[16], g[16];
-            const float4* rp = reinterpret_cast<const float4*>(r + i * 16);
+            const float4* rp = reinterpret_cast<const float4*>(r + size_t(i) * 16);
+            float4 bl4[4];
+            bilinear2_quad(lo, h, w, x, y, bl4);
 #pragma unroll
             for(int k = 0; k < 4; ++k)
             {
@@ -226,12 +229,12 @@ namespace
             for(int s = 0; s < 4; ++s)
             {
                 const int X = 2 * x + (s & 1), Y = 2 * y + (s >> 1);
-                const float4 bl = bilinear2(lo, h, w, X, Y);
+                const float4 bl = bl4[s];
                 const uchar4 tg = __ldg(hi + size_t(Y) * (2 * w) + X);
-                const float d0 = bl.x + rv[4 * s] - float(tg.x) / 255.0f;
-                const float d1 = bl.y + rv[4 * s + 1] - float(tg.y) / 255.0f;
-                const float d2 = bl.z + rv[4 * s + 2] - float(tg.z) / 255.0f;
-                const float d3 = bl.w + rv[4 * s + 3] - float(tg.w) / 255.0f;
+                const float d0 = bl.x + rv[4 * s] - div255(float(tg.x));
+                const float d1 = bl.y + rv[4 * s + 1] - div255(float(tg.y));
+                const float d2 = bl.z + rv[4 * s + 2] - div255(float(tg.z));
+                const float d3 = bl.w + rv[4 * s + 3] - div255(float(tg.w));
                 acc += d0 * d0 + d1 * d1 + d2 * d2 + d3 * d3;
                 g[4 * s] = gradScale * d0, g[4 * s + 1] = gradScale * d1, g[4 * s + 2] = gradScale * d2, g[4 * s + 3] = gradScale * d3;
             }
@@ -242,7 +245,7 @@ namespace
                 a[k] = g[k];
                 c[k] = g[8 + k];
             }
-            uint4* dp = reinterpret_cast<uint4*>(dr + i * 16);
+            uint4* dp = reinterpret_cast<uint4*>(dr + size_t(i) * 16);
             dp[0] = pack8(a);
             dp[1] = pack8(c);
         }
@@ -276,14 +279,25 @@ namespace
             const size_t i = size_t(y) * w + x;
             const uchar4* lo = reinterpret_cast<const uchar4*>(low);
             const float4* rp = reinterpret_cast<const float4*>(r + i * 16);
+            const bool pairs = (reinterpret_cast<uintptr_t>(out) & 7u) == 0;
+            auto word = [](uchar4 c) { return uint32_t(c.x) | uint32_t(c.y) << 8 | uint32_t(c.z) << 16 | uint32_t(c.w) << 24; };
+            float4 bl[4];
+            bilinear2_quad(lo, h, w, x, y, bl);
+            uchar4 px[4];
 #pragma unroll
             for(int s = 0; s < 4; ++s)
             {
-                const int X = 2 * x + (s & 1), Y = 2 * y + (s >> 1);
-                const float4 bl = bilinear2(lo, h, w, X, Y);
                 const float4 q = rp[s];
-                reinterpret_cast<uchar4*>(out)[size_t(Y) * (2 * w) + X]
-                    = make_uchar4(unit_byte(bl.x + q.x), unit_byte(bl.y + q.y), unit_byte(bl.z + q.z), unit_byte(bl.w + q.w));
+                px[s] = make_uchar4(unit_byte(bl[s].x + q.x), unit_byte(bl[s].y + q.y), unit_byte(bl[s].z + q.z), unit_byte(bl[s].w + q.w));
+            }
+#pragma unroll
+            for(int s = 0; s < 4; s += 2)
+            {
+                uchar4* dst = reinterpret_cast<uchar4*>(out) + size_t(2 * y + (s >> 1)) * (2 * w) + 2 * x;
+                if(pairs)
+                    *reinterpret_cast<uint2*>(dst) = make_uint2(word(px[s]), word(px[s + 1]));
+                else
+                    dst[0] = px[s], dst[1] = px[s + 1];
             }
         }
     }

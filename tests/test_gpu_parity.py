@@ -157,6 +157,24 @@ def test_frame_volume(interp, seed):
     assert_image_parity(got, ref)
 
 
+@pytest.mark.parametrize("fb", [(61, 43), (501, 299), (703, 457)])
+@pytest.mark.parametrize("step,alpha", [(0.5, 0.05), (0.5, 0.9), (5.0, 0.3)])
+def test_frame_march_shapes(fb, step, alpha):
+    """The march takes 8, 4 or 2 samples a trip by the rays an SM gets: rays whose last
+    trip is partly past the end (any length mod 8; a few samples in all at step 5), rays
+    that turn opaque inside a trip, ragged tiles; frame and sample count."""
+    s = gaussian_pair(n=20, fb=fb, step=step)
+    s.transfer = [{0: (0.2, 0.3, 0.9, alpha), 1024: (1.0, 0.5, 0.1, alpha)}] * 2
+    o = build_oracle(s)
+    ref = o.frame()
+    viz = build_gpu(s)
+    viz.setCounting(True)
+    got = viz.doVisualization()
+    assert_image_parity(got, ref)
+    rv, gv = o.samples()[0], viz.counters()[0]
+    assert abs(gv - rv) <= max(2, rv // 2000)
+
+
 def test_frame_dense_early_termination():
     tf = {0: (0.2, 0.3, 0.9, 0.6), 1024: (1.0, 0.5, 0.1, 1.0)}
     s = gaussian_pair(n=32, fb=(64, 64), step=0.25)

@@ -114,6 +114,24 @@ def test_inference_matches_oracle():
     assert np.abs(bl - refb).max() <= 1
 
 
+@pytest.mark.parametrize("h,w", [(8, 9), (9, 8), (21, 300)])
+def test_frame_kernel_edges(h, w):
+    """With all parameters zero the residual is zero and the frame is the bilinear one,
+    byte for byte, whatever the output's alignment (8-byte stores or single pixels); the
+    last row and column take the clamped neighbours."""
+    low = torch.randint(0, 256, (h, w, 4), dtype=torch.uint8, device="cuda")
+    net = Reconstructor(1, h, w, seed=1)
+    net.set_params(np.zeros_like(net.params()))
+    ref = bilinear2(low)
+    buf = torch.zeros(16 * h * w + 4, dtype=torch.uint8, device="cuda")
+    for off in (0, 4):
+        out = buf[off : off + 16 * h * w].view(2 * h, 2 * w, 4)
+        net.infer(low, out=out)
+        assert torch.equal(out, ref)
+    want = np.floor(R.upsample_bilinear2(low.cpu().numpy()[None] / 255.0)[0] * 255.0 + 0.5)
+    assert np.abs(ref.cpu().numpy().astype(np.float64) - want).max() <= 1
+
+
 @pytest.mark.parametrize("h,w", [(64, 128), (68, 128)])
 def test_inference_producers_agree(h, w):
     """The decoder's 1x1 layers read their concatenated input [up(coarse), fine] in place:
