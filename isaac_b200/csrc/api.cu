@@ -278,6 +278,8 @@ namespace
 struct isaacb_ctx
 {
     isaacb_desc desc{};
+    // g.yfast is the slot order of the texture in memory, which every draw reads: it changes
+    // only where a merge, or a graph that holds one, has been enqueued
     Geom g{};
     int nVol = 0, nPart = 0, nTotal = 0;
     int ts = 1024;
@@ -666,10 +668,12 @@ namespace
         return ey > ex ? 1 : 0;
     }
 
-    // the merge's launch parameters from a context's state (no launch, no stream work)
-    void prepare_merge(isaacb_ctx* c, MergeParams& p)
+    // the launch parameters, from a context's state, of a merge that writes slots in order
+    // `yfast` (no launch, no stream work)
+    void prepare_merge(isaacb_ctx* c, int32_t yfast, MergeParams& p)
     {
         p.g = c->g;
+        p.g.yfast = yfast;
         p.nVol = c->nVol;
         p.ts = c->ts;
         p.ditherMode = c->ditherMode;
@@ -1303,14 +1307,14 @@ extern "C"
                     return r;
             }
             c->advectedThisFrame = false;
-            c->g.yfast = slot_order_for_camera(c);
             MergeParams p{};
-            prepare_merge(c, p);
+            prepare_merge(c, slot_order_for_camera(c), p);
             {
                 for(int k = 0; k < ISAACB_TIMING_SLOTS; ++k)
                     c->evUsed[k] = false;
                 PhaseTimer t(c, 0, st);
                 c->updateLaunches += uint32_t(launch_merge(p, st));
+                c->g.yfast = p.g.yfast;
             }
             if(!p.writeIso && c->isoWritten)
             {
@@ -1786,19 +1790,27 @@ namespace
         inverse4(PM, out);
     }
 
-    // Slot order of the textures that the batch's own merges write: the views look from every
-    // side, and y fastest suits any yaw at moderate pitch (slot_order_for_camera: 5.4-6.2 L1
-    // cycles a load up to 20 degrees of pitch, 10-11 at 34) where x fastest is as good only
-    // within 20 degrees of one axis and takes 12-15 beyond 45.  Set before the tables and the
-    // merge parameters are formed.
-    void batch_slot_orders(isaacb_batch* b)
+    // Slot order of the texture that the batch's own merge of context i writes: the views look
+    // from every side, and y fastest suits any yaw at moderate pitch (slot_order_for_camera:
+    // 5.4-6.2 L1 cycles a load up to 20 degrees of pitch, 10-11 at 34) where x fastest is as
+    // good only within 20 degrees of one axis and takes 12-15 beyond 45.
+    int32_t batch_slot_order(const isaacb_batch* b, size_t i)
     {
-        for(isaacb_ctx* c : b->ctxs)
-            c->g.yfast = c->slotOrder >= 0 ? c->slotOrder : 1;
+        const isaacb_ctx* c = b->ctxs[i];
+        return c->slotOrder >= 0 ? c->slotOrder : 1;
+    }
+    // the order that context i's texture has once the batch has drawn: of the merge about to
+    // run (a captured graph's, where there is one), else of the texture in memory
+    int32_t batch_drawn_order(const isaacb_batch* b, size_t i, bool update, bool graph)
+    {
+        if(!update)
+            return b->ctxs[i]->g.yfast;
+        return graph ? b->graphMerges[i].g.yfast : batch_slot_order(b, i);
     }
 
-    // host mirror of the device tables from the contexts' current state; uploaded on `st`
-    isaacb_status batch_refresh(isaacb_batch* b, cudaStream_t st)
+    // host mirror of the device tables from the contexts' current state, for the textures as
+    // they are when the batch draws; uploaded on `st`
+    isaacb_status batch_refresh(isaacb_batch* b, cudaStream_t st, bool update, bool graph)
     {
         if(cudaEventSynchronize(b->tableEvent) != cudaSuccess)
             return batch_fail(ISAACB_CUDA_ERROR, "batch table staging wait");
@@ -1808,6 +1820,7 @@ namespace
             BatchCtx& t = b->ctxPinned[i];
             std::memset(&t, 0, sizeof(t));
             t.g = c->g;
+            t.g.yfast = batch_drawn_order(b, i, update, graph);
             t.volQ = c->volQ;
             t.volFlag = c->volFlag;
             t.step = c->step;
@@ -1866,16 +1879,19 @@ namespace
         b->launches = 0;
         if(update)
         {
-            for(isaacb_ctx* c : b->ctxs)
+            for(size_t i = 0; i < b->ctxs.size(); ++i)
             {
+                isaacb_ctx* c = b->ctxs[i];
                 for(int s = 0; s < c->nVol; ++s)
                     if(!c->src[s] && (c->weight[s] != 0.0f || c->iso[s] != 0.0f))
                         return batch_fail(ISAACB_NOT_READY, "isaacb_batch: a source has no memory");
                 MergeParams p{};
-                prepare_merge(c, p);
-                if(capture)
-                    b->graphMerges.push_back(p);
+                prepare_merge(c, batch_slot_order(b, i), p);
                 b->launches += uint32_t(launch_merge(p, st));
+                if(capture)
+                    b->graphMerges.push_back(p); // the texture has its order once the graph is launched
+                else
+                    c->g.yfast = p.g.yfast;
             }
         }
         if(cudaMemsetAsync(b->counter, 0, sizeof(int32_t), st) != cudaSuccess)
@@ -1930,7 +1946,7 @@ namespace
         for(size_t i = 0; i < b->ctxs.size(); ++i)
         {
             MergeParams p{};
-            prepare_merge(b->ctxs[i], p);
+            prepare_merge(b->ctxs[i], batch_slot_order(b, i), p);
             if(i >= b->graphMerges.size() || std::memcmp(&p, &b->graphMerges[i], sizeof(MergeParams)) != 0)
                 return true;
         }
@@ -2041,11 +2057,9 @@ extern "C"
         if(!b)
             return ISAACB_INVALID_ARG;
         cudaStream_t st = (cudaStream_t) stream;
-        if(update)
-            batch_slot_orders(b);
         isaacb_status r = batch_upload_luts(b, st);
         if(r == ISAACB_OK)
-            r = batch_refresh(b, st);
+            r = batch_refresh(b, st, update != 0, false);
         if(r == ISAACB_OK)
             r = batch_enqueue(b, st, update != 0, false);
         return r;
@@ -2056,11 +2070,9 @@ extern "C"
         if(!b || !stream)
             return batch_fail(ISAACB_INVALID_ARG, "isaacb_batch_capture: needs a non-default stream");
         cudaStream_t st = (cudaStream_t) stream;
-        if(update)
-            batch_slot_orders(b);
         isaacb_status r = batch_upload_luts(b, st);
         if(r == ISAACB_OK)
-            r = batch_refresh(b, st);
+            r = batch_refresh(b, st, update != 0, false);
         if(r != ISAACB_OK)
             return r;
         batch_drop_graph(b);
@@ -2090,8 +2102,6 @@ extern "C"
         if(!b || !b->graphExec)
             return batch_fail(ISAACB_NOT_READY, "isaacb_batch_launch_graph: no captured graph");
         cudaStream_t st = (cudaStream_t) stream;
-        if(b->graphUpdate)
-            batch_slot_orders(b);
         // functors, weights, storage or source memory changed: the merges in the graph are out of date
         if(batch_graph_stale(b))
         {
@@ -2103,12 +2113,14 @@ extern "C"
         // cameras and frame settings live in device tables the graph reads
         isaacb_status r = batch_upload_luts(b, st);
         if(r == ISAACB_OK)
-            r = batch_refresh(b, st);
+            r = batch_refresh(b, st, b->graphUpdate, true);
         if(r != ISAACB_OK)
             return r;
         const cudaError_t e = cudaGraphLaunch(b->graphExec, st);
         if(e != cudaSuccess)
             return batch_fail(ISAACB_CUDA_ERROR, std::string("isaacb_batch_launch_graph: ") + cudaGetErrorString(e));
+        for(size_t i = 0; i < b->graphMerges.size(); ++i)
+            b->ctxs[i]->g.yfast = b->graphMerges[i].g.yfast;
         return ISAACB_OK;
     }
 

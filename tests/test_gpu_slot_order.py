@@ -1,0 +1,123 @@
+"""The slot order that a texture in memory has (Geom::yfast) against the order of the next
+merge: a draw takes the former, whatever has been captured, has failed or is asked for in
+the meantime.  Frames are the same bytes in both orders."""
+
+import math
+
+import numpy as np
+import pytest
+import torch
+
+from harness import build_gpu, gaussian_pair
+from isaac_b200 import _lib, scenes
+from isaac_b200.batch import IsaacBatch
+
+pytestmark = pytest.mark.gpu
+
+FB = (64, 48)
+FRONT = scenes.orbit_camera(*FB, yaw=0.0, pitch=0.6)  # merged x fastest by a context
+SIDE = scenes.orbit_camera(*FB, yaw=math.pi / 2, pitch=0.1)  # y fastest
+
+
+def _viz(seed=1, camera=FRONT):
+    return build_gpu(gaussian_pair(32, fb=FB, seed=seed, P=camera[0], MV=camera[1]))
+
+
+def _frame(viz):
+    out = torch.zeros((FB[1], FB[0], 4), dtype=torch.uint8, device="cuda")
+    viz.render(out)
+    torch.cuda.synchronize()
+    return out.cpu().numpy()
+
+
+def _reference(seed=1, camera=FRONT):
+    viz = _viz(seed, camera)
+    frame = viz.doVisualization()
+    viz.close()
+    assert frame.any()
+    return frame
+
+
+def test_draws_between_capture_and_launch():
+    """A capture merges nothing: the context and the batch draw the texture as it is."""
+    viz = _viz()
+    batch = IsaacBatch([viz], [(0, *FB, *SIDE)])
+    front, side = _reference(), _reference(camera=SIDE)
+    viz.update()
+    torch.cuda.synchronize()
+    stream = torch.cuda.Stream()
+    with torch.cuda.stream(stream):
+        batch.capture(update=True)
+    stream.synchronize()
+    assert np.array_equal(_frame(viz), front)
+    batch.render(update=False)
+    torch.cuda.synchronize()
+    assert np.array_equal(batch.frames[0].cpu().numpy(), side)
+    for _ in range(2):
+        batch.frames[0].zero_()
+        torch.cuda.synchronize()
+        with torch.cuda.stream(stream):
+            batch.launchGraph()
+        stream.synchronize()
+        assert np.array_equal(batch.frames[0].cpu().numpy(), side)
+        assert np.array_equal(_frame(viz), front)
+        viz.update()  # back to the context's own order
+        assert np.array_equal(_frame(viz), front)
+    batch.close()
+    viz.close()
+
+
+@pytest.mark.parametrize("how", ["render", "launchGraph"])
+def test_draws_after_a_failed_update(how):
+    """A batch update that stops at a context without memory leaves that context's texture,
+    and every draw of either context is right afterwards."""
+    vis = [_viz(1), _viz(2)]
+    refs = [_reference(1), _reference(2)]
+    batch = IsaacBatch(vis, [(0, *FB, *SIDE), (1, *FB, *SIDE)])
+    stream = torch.cuda.Stream()
+    for v in vis:
+        v.update()
+    torch.cuda.synchronize()
+    if how == "launchGraph":
+        with torch.cuda.stream(stream):
+            batch.capture(update=True)
+        stream.synchronize()
+    keep = vis[1].volumeSources[0].data.data_ptr()
+    _lib.check(vis[1].lib.isaacb_set_source(vis[1].ctx, 0, None), vis[1].ctx)
+    with torch.cuda.stream(stream):
+        with pytest.raises(_lib.IsaacError) as e:
+            batch.render(update=True) if how == "render" else batch.launchGraph()
+    assert e.value.status == _lib.NOT_READY
+    stream.synchronize()
+    for v, ref in zip(vis, refs):
+        assert np.array_equal(_frame(v), ref)
+    batch.render(update=False)
+    torch.cuda.synchronize()
+    for i in range(2):
+        assert np.array_equal(batch.frames[i].cpu().numpy(), _reference(i + 1, SIDE))
+    _lib.check(vis[1].lib.isaacb_set_source(vis[1].ctx, 0, keep), vis[1].ctx)
+    batch.close()
+    for v in vis:
+        v.close()
+
+
+def test_slot_order_setting_reaches_a_captured_graph():
+    """setSlotOrder after a capture takes effect with the next launch, and the draws that
+    follow read the texture in its new order."""
+    viz = _viz()
+    batch = IsaacBatch([viz], [(0, *FB, *SIDE)])
+    front, side = _reference(), _reference(camera=SIDE)
+    stream = torch.cuda.Stream()
+    viz.update()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(stream):
+        batch.capture(update=True)
+    for order in (0, 1, -1):
+        viz.setSlotOrder(order)
+        with torch.cuda.stream(stream):
+            batch.launchGraph()
+        stream.synchronize()
+        assert np.array_equal(batch.frames[0].cpu().numpy(), side)
+        assert np.array_equal(_frame(viz), front)
+    batch.close()
+    viz.close()
