@@ -344,6 +344,10 @@ struct isaacb_ctx
     unsigned int* emptyDev = nullptr;
     // slot order of the combined textures: -1 per merge from the camera, 0 x, 1 y fastest
     int32_t slotOrder = -1;
+    // the order of every merge from the first update that a stream capture recorded on: its
+    // replays write it without the host's knowledge (-1: none)
+    int32_t heldOrder = -1;
+    bool merged = false; // a texture has been written
     // field-source advection (defaults of lib/isaac.hpp:606-643); the textures start at zero
     bool field[kMaxSources]{};
     uint8_t* adv[kMaxSources]{}; // guarded: (local + 2 * advG) per axis
@@ -652,6 +656,8 @@ namespace
     // speed depends on it: both orders hold the same texels.
     int32_t slot_order_for_camera(const isaacb_ctx* c)
     {
+        if(c->heldOrder >= 0)
+            return c->heldOrder;
         if(c->slotOrder >= 0)
             return c->slotOrder;
         const double textureBytes = double(brick_count(c->g)) * kSlotsPerBrick * sizeof(uint4);
@@ -666,6 +672,17 @@ namespace
             return 0;
         const double ex = std::fabs(ix[0]) / nx, ey = std::fabs(iy[1]) / ny;
         return ey > ex ? 1 : 0;
+    }
+
+    // the order of the merge about to be enqueued on `st`.  Under a stream capture nothing is
+    // merged yet and the merge may run at any time: it keeps the order of the texture in memory,
+    // and so do the merges after it.
+    int32_t slot_order_for_update(isaacb_ctx* c, cudaStream_t st)
+    {
+        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+        if(c->heldOrder < 0 && st && cudaStreamIsCapturing(st, &capture) == cudaSuccess && capture != cudaStreamCaptureStatusNone)
+            c->heldOrder = c->merged ? c->g.yfast : slot_order_for_camera(c);
+        return slot_order_for_camera(c);
     }
 
     // the launch parameters, from a context's state, of a merge that writes slots in order
@@ -1308,13 +1325,14 @@ extern "C"
             }
             c->advectedThisFrame = false;
             MergeParams p{};
-            prepare_merge(c, slot_order_for_camera(c), p);
+            prepare_merge(c, slot_order_for_update(c, st), p);
             {
                 for(int k = 0; k < ISAACB_TIMING_SLOTS; ++k)
                     c->evUsed[k] = false;
                 PhaseTimer t(c, 0, st);
                 c->updateLaunches += uint32_t(launch_merge(p, st));
                 c->g.yfast = p.g.yfast;
+                c->merged = true;
             }
             if(!p.writeIso && c->isoWritten)
             {
@@ -1797,7 +1815,7 @@ namespace
     int32_t batch_slot_order(const isaacb_batch* b, size_t i)
     {
         const isaacb_ctx* c = b->ctxs[i];
-        return c->slotOrder >= 0 ? c->slotOrder : 1;
+        return c->heldOrder >= 0 ? c->heldOrder : c->slotOrder >= 0 ? c->slotOrder : 1;
     }
     // the order that context i's texture has once the batch has drawn: of the merge about to
     // run (a captured graph's, where there is one), else of the texture in memory
@@ -1891,7 +1909,10 @@ namespace
                 if(capture)
                     b->graphMerges.push_back(p); // the texture has its order once the graph is launched
                 else
+                {
                     c->g.yfast = p.g.yfast;
+                    c->merged = true;
+                }
             }
         }
         if(cudaMemsetAsync(b->counter, 0, sizeof(int32_t), st) != cudaSuccess)
@@ -2120,7 +2141,10 @@ extern "C"
         if(e != cudaSuccess)
             return batch_fail(ISAACB_CUDA_ERROR, std::string("isaacb_batch_launch_graph: ") + cudaGetErrorString(e));
         for(size_t i = 0; i < b->graphMerges.size(); ++i)
+        {
             b->ctxs[i]->g.yfast = b->graphMerges[i].g.yfast;
+            b->ctxs[i]->merged = true;
+        }
         return ISAACB_OK;
     }
 

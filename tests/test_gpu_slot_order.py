@@ -121,3 +121,32 @@ def test_slot_order_setting_reaches_a_captured_graph():
         assert np.array_equal(_frame(viz), front)
     batch.close()
     viz.close()
+
+
+def test_update_captured_by_the_caller():
+    """A caller's own graph holds an update: capturing it merges nothing, and after a replay
+    or an update outside the graph, whatever the camera, every draw reads the right order."""
+    viz = _viz()
+    front, side = _reference(), _reference(camera=SIDE)
+    out = torch.zeros((FB[1], FB[0], 4), dtype=torch.uint8, device="cuda")
+    viz.update()
+    assert np.array_equal(_frame(viz), front)
+    viz.setCamera(*SIDE)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        viz.update()
+        viz.render(out)
+    assert np.array_equal(_frame(viz), side)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert np.array_equal(out.cpu().numpy(), side)
+    for camera, want in ((FRONT, front), (SIDE, side)):
+        viz.setCamera(*camera)
+        viz.update()
+        assert np.array_equal(_frame(viz), want)
+        out.zero_()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert np.array_equal(out.cpu().numpy(), side)
+        assert np.array_equal(_frame(viz), want)
+    viz.close()
