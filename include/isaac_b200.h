@@ -185,8 +185,10 @@ isaacb_status isaacb_set_camera(isaacb_ctx* ctx, const double projection[16], co
 isaacb_status isaacb_update(isaacb_ctx* ctx, void* stream);
 
 /* drawCallBack (lib/isaac.hpp:2140-2543): clear, particles, iso, SSAO,
- * shading, volume.  The frame stays in the context's device framebuffer;
- * if rgba_dev is not NULL it is also copied there.  Asynchronous. */
+ * shading, volume.  The frame stays in the context's device framebuffer; if
+ * rgba_dev is not NULL it also gets there: stored by the shading pass where that is
+ * 4-byte aligned memory of this device, copied to any other memory that a device copy
+ * reaches.  Pageable host memory is refused (ISAACB_INVALID_ARG).  Asynchronous. */
 isaacb_status isaacb_render(isaacb_ctx* ctx, void* stream, uint8_t* rgba_dev);
 
 /* One whole doVisualization frame with a host result: update, render and the

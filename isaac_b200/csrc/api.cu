@@ -745,6 +745,35 @@ namespace
 
 namespace
 {
+    // How a frame reaches the memory that the caller asked for.  The pass that shades stores
+    // it there itself only where its stores are sure to be legal: aligned device memory of the
+    // device that it runs on.  Other memory that a copy can reach (another device's, pinned or
+    // managed, unaligned) gets a copy of the framebuffer; pageable memory, which the copy
+    // refuses, is refused before any launch.  Asked anew on every call (0.3 us).
+    enum FrameTarget
+    {
+        FRAME_NONE,
+        FRAME_STORE,
+        FRAME_COPY,
+        FRAME_REFUSED
+    };
+    FrameTarget frame_target(const isaacb_ctx* c, const uint8_t* rgba)
+    {
+        if(!rgba || rgba == reinterpret_cast<const uint8_t*>(c->color))
+            return FRAME_NONE;
+        cudaPointerAttributes attr{};
+        int dev = -1;
+        if(cudaPointerGetAttributes(&attr, rgba) != cudaSuccess || cudaGetDevice(&dev) != cudaSuccess)
+        {
+            cudaGetLastError(); // let the copy say what is wrong
+            return FRAME_COPY;
+        }
+        if(attr.type == cudaMemoryTypeUnregistered)
+            return FRAME_REFUSED;
+        const bool here = attr.type == cudaMemoryTypeDevice && attr.device == dev;
+        return here && (reinterpret_cast<uintptr_t>(rgba) & 3u) == 0 ? FRAME_STORE : FRAME_COPY;
+    }
+
     // largest frame that isaacb_frame reads through its own staging buffer
     constexpr size_t kFrameStaging = 256 * 1024;
 } // namespace
@@ -1410,6 +1439,9 @@ extern "C"
         for(int s = 0; s < c->nPart; ++s)
             if(!c->partSet[s] && c->weight[c->nVol + s] != 0.0f)
                 return fail(c, ISAACB_NOT_READY, "isaacb_render: particle source without memory");
+        const FrameTarget target = frame_target(c, rgba_dev);
+        if(target == FRAME_REFUSED)
+            return fail(c, ISAACB_INVALID_ARG, "isaacb_render: the frame's target is pageable host memory");
         cudaStream_t st = (cudaStream_t) stream;
         isaacb_status r = upload_lut(c, st);
         if(r != ISAACB_OK)
@@ -1482,10 +1514,7 @@ extern "C"
         c->renderLaunches = 0;
         for(int k = 1; k < ISAACB_TIMING_SLOTS; ++k)
             c->evUsed[k] = false;
-        // the pass that shades also writes the caller's frame, unless that is unaligned or
-        // the framebuffer itself
-        const bool direct = rgba_dev && (reinterpret_cast<uintptr_t>(rgba_dev) & 3u) == 0 && rgba_dev != reinterpret_cast<uint8_t*>(c->color);
-        p.out = direct ? reinterpret_cast<uchar4*>(rgba_dev) : nullptr;
+        p.out = target == FRAME_STORE ? reinterpret_cast<uchar4*>(rgba_dev) : nullptr;
         p.shadeDepth = c->renderMode == 2 || (c->renderMode >= 4 && c->renderMode <= 8) ? 1 : 0;
         // the first pass of the frame clears the G-buffer: the particles' where there are
         // any, else the iso surface's or the shading's; SSAO and the per-source kernels that
@@ -1536,7 +1565,7 @@ extern "C"
                 c->renderLaunches += uint32_t(launch_shade_volume_per_source(p, clean, st));
         }
         ISAACB_CUDA(c, cudaGetLastError(), "isaacb_render launch");
-        if(rgba_dev && !direct && rgba_dev != reinterpret_cast<uint8_t*>(c->color))
+        if(target == FRAME_COPY)
         {
             const size_t bytes = size_t(c->desc.framebuffer[0]) * c->desc.framebuffer[1] * 4;
             ISAACB_CUDA(c, cudaMemcpyAsync(rgba_dev, c->color, bytes, cudaMemcpyDeviceToDevice, st), "frame copy");
