@@ -17,20 +17,19 @@
 namespace isaacb
 {
     template<bool LINEAR, bool SKIP, bool YFAST>
-    __device__ __forceinline__ void batch_pixel(
-        const BatchCtx& c, const View& v, float negZero, int px, int py, uchar4* out, unsigned long long& n)
+    __device__ __forceinline__ uchar4 batch_pixel(
+        const BatchCtx& c, const View& v, float negZero, int px, int py, unsigned long long& n)
     {
         uchar4 col = to_byte4(c.bgSwizzled);
         float depth = FLT_MAX;
         Ray ray = pixel_to_ray(v, c.g, px, py);
         const ShadeParams sp{c.renderMode, c.aoWeight, c.bg};
         shade_values(sp, c.g, ray.dir, col, f3(0, 0, 0), 0.0f, depth);
-        *out = col; // read back after the march, which needs the registers
         if(!c.volume || !clip_ray(ray, v, c.g))
-            return;
+            return col;
         ray.endDepth = gmin(ray.endDepth, depth);
         if(ray.endDepth <= ray.startDepth)
-            return;
+            return col;
         const March m = march_setup(ray, c.g, v.scale, c.step);
         const float factor = m.factor * c.totalWeightAll;
         const VolTexRef tex{c.g, c.volQ, c.volFlag, negZero};
@@ -39,7 +38,7 @@ namespace isaacb
             color = march_combined<LINEAR, false, SKIP, YFAST, 1>(tex, m, factor, n);
         else
             color = march_combined<LINEAR, true, SKIP, YFAST, 1>(tex, m, factor, n);
-        *out = over_surface(color, *out);
+        return over_surface(color, col);
     }
 
     // 4 CTAs per SM (64 registers): two merges and 8 views of 512^3 textures take 20.9 ms; 3
@@ -113,19 +112,18 @@ namespace isaacb
             {
                 // auto (-1): skip when the context's last merge found empty bricks
                 const bool skip = sc.skipEmpty >= 0 ? sc.skipEmpty != 0 : __ldg(sc.emptyCount) != 0u;
-                uchar4* out = bv.out + (size_t(py) * sv.W + px);
                 auto pixel = [&](auto linear, auto y) {
-                    if(skip)
-                        batch_pixel<decltype(linear)::value, true, decltype(y)::value>(sc, sv, bp.negZero, px, py, out, n);
-                    else
-                        batch_pixel<decltype(linear)::value, false, decltype(y)::value>(sc, sv, bp.negZero, px, py, out, n);
+                    return skip ? batch_pixel<decltype(linear)::value, true, decltype(y)::value>(sc, sv, bp.negZero, px, py, n)
+                                : batch_pixel<decltype(linear)::value, false, decltype(y)::value>(sc, sv, bp.negZero, px, py, n);
                 };
                 const std::true_type yes;
                 const std::false_type no;
+                uchar4 c;
                 if(sc.interpolation)
-                    yfast ? pixel(yes, yes) : pixel(yes, no);
+                    c = yfast ? pixel(yes, yes) : pixel(yes, no);
                 else
-                    yfast ? pixel(no, yes) : pixel(no, no);
+                    c = yfast ? pixel(no, yes) : pixel(no, no);
+                bv.out[size_t(py) * sv.W + px] = c; // one store, nothing read: the buffer may be host or peer memory
             }
             __syncthreads();
         }

@@ -199,3 +199,37 @@ def test_batch_slot_orders(order, tile):
     batch.close()
     for v in vis:
         v.close()
+
+
+@pytest.mark.parametrize("where", ["device", "pinned"])
+def test_batch_views_sharing_a_buffer_do_not_mix(where):
+    """A view's pixel is stored once and nothing is read from its buffer: of several views
+    drawn into one buffer, in device or host memory, each pixel is one view's."""
+    import ctypes as C
+
+    w, h = 96, 64
+    sc = [gaussian_pair(32, seed=i + 1, background=bg) for i, bg in enumerate([(0.9, 0.1, 0.2, 1.0), (0.0, 0.8, 1.0, 0.3)])]
+    vis = [build_gpu(s) for s in sc]
+    cams = [_camera(w, h, 5 + i, sc[i]) for i in range(2)]
+    refs = [_reference(sc[i], w, h, 5 + i) for i in range(2)]
+    assert (refs[0] != refs[1]).any(axis=-1).mean() > 0.5
+    buf = torch.zeros((h, w, 4), dtype=torch.uint8, device="cuda" if where == "device" else "cpu")
+    if where == "pinned":
+        buf = buf.pin_memory()
+    n = 16
+    views = (_lib.View * n)()
+    for i, v in enumerate(views):
+        v.ctx_index, v.width, v.height, v.rgba_dev = i % 2, w, h, buf.data_ptr()
+        v.projection[:] = [float(x) for x in np.asarray(cams[i % 2][0]).reshape(16)]
+        v.modelview[:] = [float(x) for x in np.asarray(cams[i % 2][1]).reshape(16)]
+    lib, handle = _lib.load(), C.c_void_p()
+    _lib.check(lib.isaacb_batch_create((C.c_void_p * 2)(*[x.ctx for x in vis]), 2, views, n, C.byref(handle)))
+    for _ in range(10):
+        _lib.check(lib.isaacb_batch_render(handle, _lib.current_stream(), 1))
+        torch.cuda.synchronize()
+        got = buf.cpu().numpy()
+        one = (got == refs[0]).all(axis=-1) | (got == refs[1]).all(axis=-1)
+        assert one.all(), int((~one).sum())
+    _lib.check(lib.isaacb_batch_destroy(handle))
+    for v in vis:
+        v.close()
