@@ -233,3 +233,23 @@ def test_batch_views_sharing_a_buffer_do_not_mix(where):
     _lib.check(lib.isaacb_batch_destroy(handle))
     for v in vis:
         v.close()
+
+
+@pytest.mark.parametrize("skip", [0, 1])
+def test_batch_singular_camera_matches_single_views(skip):
+    """Rays without a direction, through a volume whose first brick is empty or not."""
+    w, h = 40, 24
+    P, MV = np.zeros((4, 4)), np.eye(4)
+    for i, transfer in enumerate(({0: (0, 0, 0, 0), 1024: (0, 0, 0, 0)}, {0: (0.2, 0.5, 0.9, 0.1), 1024: (0.9, 0.5, 0.2, 0.8)})):
+        s = gaussian_pair(32, seed=4 + i, fb=(w, h), background=(0.9, 0.3, 0.2, 0.7), transfer=[transfer] * 2, P=P, MV=MV)
+        viz = build_gpu(s)
+        ref = viz.doVisualization()
+        batch = IsaacBatch([viz], [(0, w, h, P, MV)])
+        batch.setConfig(skip_empty=skip)
+        batch.render(update=True)
+        torch.cuda.synchronize()
+        got = batch.frames[0].cpu().numpy()
+        if i == 1 or skip:  # a single view skips where the texture has empty bricks
+            assert np.array_equal(got, ref), image_diff(got, ref)
+        batch.close()
+        viz.close()
