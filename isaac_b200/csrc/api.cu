@@ -642,6 +642,40 @@ namespace
         return c->src[s] ? c->src[s] + (g * pitchZ + g * pitchY + g) * c->desc.feature_dim[s] : nullptr;
     }
 
+    // how close the image axes are to the volume's axes: |cos| between image x and volume x,
+    // image y and volume y (1 the same line, 0 perpendicular or unknown)
+    struct ImageAxes
+    {
+        double x, y;
+    };
+    ImageAxes image_axes(const double* mv)
+    {
+        // rows 0 and 1 of the column-major modelview: the image axes in volume coordinates
+        const double nx = std::sqrt(mv[0] * mv[0] + mv[4] * mv[4] + mv[8] * mv[8]);
+        const double ny = std::sqrt(mv[1] * mv[1] + mv[5] * mv[5] + mv[9] * mv[9]);
+        if(!(nx > 0.0) || !(ny > 0.0))
+            return {0.0, 0.0};
+        return {std::fabs(mv[0]) / nx, std::fabs(mv[5]) / ny};
+    }
+    // Whether a draw of y-fastest slots has a warp's lanes down the image's columns (8 pixels)
+    // or along its rows (4): down columns that stay close to y, along rows where a camera looks
+    // steeply down and the pixels are denser than the voxels.  1920x1080 over 512^3, 0.49 voxels
+    // a pixel, yaw 90 (columns / rows, ms): pitch 25 3.48 / 3.56, 29 3.76 / 3.64, 34 4.06 /
+    // 3.76, 55 4.42 / 3.90, 70 4.48 / 3.78; 960x540 over the same, 0.98: 1.09 / 1.37, 1.13 /
+    // 1.49, 1.23 / 1.55, at pitch 70 1.79 / 1.78; 640x360 over 256^3, 0.74: even at pitch 45,
+    // 0.374 / 0.355 at 70.
+    constexpr double kColumnAxis = 0.87, kDenseVoxels = 0.6;
+    int32_t lane_columns(const Geom& g, const double* proj, const double* mv, int32_t height)
+    {
+        if(image_axes(mv).y >= kColumnAxis)
+            return 1;
+        // voxels a pixel at the volume's centre, whose clip-space w is that of the modelview's
+        // translation
+        const double w = proj[3] * mv[12] + proj[7] * mv[13] + proj[11] * mv[14] + proj[15];
+        const double up = std::sqrt(mv[1] * mv[1] + mv[5] * mv[5] + mv[9] * mv[9]) * std::fabs(proj[5]) * double(height);
+        return std::fabs(w) * double(g.maxGss) < kDenseVoxels * up ? 0 : 1;
+    }
+
     // Slot order of the combined textures for the camera of the merge about to run
     // (Geom::yfast).  The march's warps walk the slots' fast axis with image rows (x fastest)
     // or image columns (y fastest), and L1 serves a load the faster the closer those stay to
@@ -664,14 +698,8 @@ namespace
         const long long warps = (long long) ((c->desc.framebuffer[0] + 7) / 8) * ((c->desc.framebuffer[1] + 3) / 4);
         if(textureBytes < 4.0 * 126.0e6 && warps > 148 * 64)
             return 0;
-        // rows 0 and 1 of the column-major modelview: the image axes in volume coordinates
-        const double ix[3] = {c->mv[0], c->mv[4], c->mv[8]}, iy[3] = {c->mv[1], c->mv[5], c->mv[9]};
-        const double nx = std::sqrt(ix[0] * ix[0] + ix[1] * ix[1] + ix[2] * ix[2]);
-        const double ny = std::sqrt(iy[0] * iy[0] + iy[1] * iy[1] + iy[2] * iy[2]);
-        if(!(nx > 0.0) || !(ny > 0.0))
-            return 0;
-        const double ex = std::fabs(ix[0]) / nx, ey = std::fabs(iy[1]) / ny;
-        return ey > ex ? 1 : 0;
+        const ImageAxes a = image_axes(c->mv);
+        return a.y > a.x ? 1 : 0;
     }
 
     // the order of the merge about to be enqueued on `st`.  Under a stream capture nothing is
@@ -1501,6 +1529,7 @@ extern "C"
         }
         p.psPre = c->psPre;
         p.negZero = -0.0f;
+        p.laneColumns = lane_columns(c->g, c->proj, c->mv, p.v.H);
         p.color = c->color;
         p.depth = c->depth;
         p.normal = c->normal;
@@ -1899,6 +1928,7 @@ namespace
             t.tilesX = int32_t((iv.width + b->cfg.tile_w - 1) / b->cfg.tile_w);
             t.tiles = t.tilesX * int32_t((iv.height + b->cfg.tile_h - 1) / b->cfg.tile_h);
             t.tileBase = base;
+            t.laneColumns = lane_columns(b->ctxs[iv.ctx_index]->g, iv.projection, iv.modelview, t.H);
             t.out = reinterpret_cast<uchar4*>(iv.rgba_dev);
             base += t.tiles;
         }

@@ -235,6 +235,7 @@ namespace isaacb
         PerSourceSrc ps[kMaxSources];
         float4* psPre; // scratch: the weighted premultiplied tables of the active sources
         float negZero; // -0.0f, the addend of packed products that must round on their own (f2p_mul_exact)
+        int32_t laneColumns; // warps over y-fastest slots have their lanes down image columns, else along rows
         // G-buffer
         uchar4* color;
         uchar4* out; // the caller's frame, null: none
@@ -276,6 +277,7 @@ namespace isaacb
         int32_t tilesX;
         int32_t tileBase;
         int32_t tiles;
+        int32_t laneColumns; // as in FrameParams
         uchar4* out;
     };
     struct BatchParams

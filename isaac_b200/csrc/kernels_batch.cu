@@ -126,13 +126,13 @@ namespace isaacb
             }
             __syncthreads();
             // pixel of this thread inside the tile: 8 x 4 pixels a warp, lanes along rows, for
-            // x-fastest slots; lanes down columns for y-fastest ones, of 8 pixels where the
-            // tile has them (k_shade_volume)
-            const bool yfast = sc.g.yfast != 0, tall = yfast && (bp.tileH & 7) == 0;
+            // x-fastest slots; 4 x 8 where the tile has them for y-fastest ones, lanes down
+            // columns or along rows by the view (k_shade_volume)
+            const bool yfast = sc.g.yfast != 0, tall = yfast && (bp.tileH & 7) == 0, down = yfast && bv.laneColumns != 0;
             const int ww = tall ? 4 : 8, wh = tall ? 8 : 4, warpsX = bp.tileW / ww;
             const int w = t >> 5, l = t & 31;
-            const int ox = (w % warpsX) * ww + (yfast ? l / wh : l % ww);
-            const int oy = (w / warpsX) * wh + (yfast ? l % wh : l / ww);
+            const int ox = (w % warpsX) * ww + (down ? l / wh : l % ww);
+            const int oy = (w / warpsX) * wh + (down ? l % wh : l / ww);
             const int local = tile - bv.tileBase;
             const int px = (local % bv.tilesX) * bp.tileW + ox;
             const int py = (local / bv.tilesX) * bp.tileH + oy;

@@ -471,7 +471,8 @@ namespace isaacb
     // axis keep along y.  Against rows of 4 lanes for y-fastest slots that is 5.9 instead of
     // 10.7 cycles a load (a count over sampled warps that gives the 10.6 ncu showed), and
     // the 4 x 512^3 march at 1920x1080 3.46 -> 3.24 ms, at 960x540 0.73 -> 0.63 ms (one
-    // sample a trip).
+    // sample a trip). Where columns leave the y axis, under a camera that looks steeply down,
+    // rows of 4 lanes are better again for dense pixels (FrameParams::laneColumns).
     // CLEAN: the frame's only pass; it clears the G-buffer instead of reading it
     template<bool VOLUME, bool LINEAR, ShadeShape SHAPE, bool YFAST, bool CLEAN>
     __global__ void __launch_bounds__(shade_threads(SHAPE), SHAPE == SHADE_FULL ? 8 : 1) k_shade_volume(const __grid_constant__ FrameParams p)
@@ -482,8 +483,9 @@ namespace isaacb
         constexpr int TW = shade_tile_w(SHAPE, YFAST), TH = shade_tile_h(SHAPE, YFAST);
         constexpr int WW = YFAST ? 4 : 8, WH = 32 / WW, WX = TW / WW; // warp tile and warps per row
         const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-        const int px = int(blockIdx.x) * TW + (w % WX) * WW + (YFAST ? l / WH : l % WW);
-        const int py = int(blockIdx.y) * TH + (w / WX) * WH + (YFAST ? l % WH : l / WW);
+        const bool down = YFAST && p.laneColumns != 0;
+        const int px = int(blockIdx.x) * TW + (w % WX) * WW + (down ? l / WH : l % WW);
+        const int py = int(blockIdx.y) * TH + (w / WX) * WH + (down ? l % WH : l / WW);
         unsigned long long n = 0;
         if(px < p.v.W && py < p.v.H)
         {

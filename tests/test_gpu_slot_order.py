@@ -150,3 +150,26 @@ def test_update_captured_by_the_caller():
         assert np.array_equal(out.cpu().numpy(), side)
         assert np.array_equal(_frame(viz), want)
     viz.close()
+
+
+@pytest.mark.parametrize("interpolation", [True, False])
+@pytest.mark.parametrize("fb", [(101, 77), (37, 29), (8, 3)])
+@pytest.mark.parametrize("yaw,pitch", [(0.3, 0.2), (1.5, 0.5), (1.5, 0.6), (0.8, 1.0), (1.5, 1.5)])
+def test_lanes_along_rows_and_down_columns(yaw, pitch, fb, interpolation):
+    """Both lane orders of y-fastest slots (flat and steep cameras, pixels denser and wider
+    than the voxels, ragged sizes) give the frame of x-fastest slots; batches too."""
+    P, MV = scenes.orbit_camera(*fb, yaw=yaw, pitch=pitch)
+    viz = build_gpu(gaussian_pair(32, fb=fb, P=P, MV=MV, interpolation=interpolation))
+    batch = IsaacBatch([viz], [(0, *fb, P, MV)])
+    frames = []
+    for order in (0, 1):
+        viz.setSlotOrder(order)
+        frames.append(viz.doVisualization())
+        batch.render(update=False)
+        torch.cuda.synchronize()
+        frames.append(batch.frames[0].cpu().numpy())
+    assert frames[0].any()
+    for f in frames[1:]:
+        assert np.array_equal(f, frames[0])
+    batch.close()
+    viz.close()
