@@ -657,6 +657,15 @@ namespace
             return {0.0, 0.0};
         return {std::fabs(mv[0]) / nx, std::fabs(mv[5]) / ny};
     }
+    // fewer than 0.6 voxels a pixel at the volume's centre, whose clip-space w is that of the
+    // modelview's translation
+    bool dense_pixels(const Geom& g, const double* proj, const double* mv, double height)
+    {
+        const double w = proj[3] * mv[12] + proj[7] * mv[13] + proj[11] * mv[14] + proj[15];
+        const double up = std::sqrt(mv[1] * mv[1] + mv[5] * mv[5] + mv[9] * mv[9]) * std::fabs(proj[5]) * height;
+        return std::fabs(w) * double(g.maxGss) < 0.6 * up;
+    }
+
     // Whether a draw of y-fastest slots has a warp's lanes down the image's columns (8 pixels)
     // or along its rows (4): down columns that stay close to y, along rows where a camera looks
     // steeply down and the pixels are denser than the voxels.  1920x1080 over 512^3, 0.49 voxels
@@ -664,42 +673,51 @@ namespace
     // 3.76, 55 4.42 / 3.90, 70 4.48 / 3.78; 960x540 over the same, 0.98: 1.09 / 1.37, 1.13 /
     // 1.49, 1.23 / 1.55, at pitch 70 1.79 / 1.78; 640x360 over 256^3, 0.74: even at pitch 45,
     // 0.374 / 0.355 at 70.
-    constexpr double kColumnAxis = 0.87, kDenseVoxels = 0.6;
-    int32_t lane_columns(const Geom& g, const double* proj, const double* mv, int32_t height)
+    constexpr double kColumnAxis = 0.87;
+    int32_t lane_columns(const Geom& g, const double* proj, const double* mv, double height)
     {
-        if(image_axes(mv).y >= kColumnAxis)
-            return 1;
-        // voxels a pixel at the volume's centre, whose clip-space w is that of the modelview's
-        // translation
-        const double w = proj[3] * mv[12] + proj[7] * mv[13] + proj[11] * mv[14] + proj[15];
-        const double up = std::sqrt(mv[1] * mv[1] + mv[5] * mv[5] + mv[9] * mv[9]) * std::fabs(proj[5]) * double(height);
-        return std::fabs(w) * double(g.maxGss) < kDenseVoxels * up ? 0 : 1;
+        return image_axes(mv).y < kColumnAxis && dense_pixels(g, proj, mv, height) ? 0 : 1;
     }
 
-    // Slot order of the combined textures for the camera of the merge about to run
-    // (Geom::yfast).  The march's warps walk the slots' fast axis with image rows (x fastest)
-    // or image columns (y fastest), and L1 serves a load the faster the closer those stay to
-    // the axis: y fastest is taken when the image y axis is closer to the volume's y axis
-    // than the image x axis to the volume's x.  Counted over sampled warps of a 512^3 volume
-    // at 1920x1080 (L1 cycles a load, x / y fastest): pitch 20 degrees 5.7 / 5.9 at yaw 0,
-    // 7.5 / 6.1 at 30, 12.8 / 6.2 at 45, 14.5 / 5.9 at 90; pitch 34 degrees 7.0 / 10.9 at yaw
-    // 30, 11.8 / 10.5 at 45.  Where L2 holds much of the texture and the frame fills the SMs
-    // the choice is left at x fastest: for the full-feature scene (256^3, 0.33 GB, 1920x1080)
-    // y fastest costs its pixel passes more than it gains (shading and march 236 us against
-    // 252), while small frames gain (500x300 over 128^3: 115 -> 92 us at yaw 60).  Only the
-    // speed depends on it: both orders hold the same texels.
+    // What y-fastest slots gain over x-fastest ones for a camera, in no unit (about a third of
+    // it is the relative time): positive where y fastest is the faster.  The march's warps walk
+    // the slots' fast axis with image rows (x fastest) or image columns (y fastest), and L1 serves
+    // a load the faster the closer those stay to the axis over the face that the rays enter
+    // by.  Two sources of 512^3 at 1920x1080 (x / y fastest, ms; y with the better lanes): pitch
+    // 0 and yaw 0 3.11 / 3.13, 45 3.61 / 3.15, 90 4.27 / 3.13; pitch 34 and yaw 0 3.39 / 3.75, 45
+    // 3.97 / 4.10, 60 4.52 / 3.96, 90 4.64 / 3.76; pitch 55 and yaw 45 3.32 / 4.09, 60 3.87 / 4.01,
+    // 75 4.49 / 3.94; pitch 70 and yaw 60 3.52 / 3.91, 75 4.20 / 3.85.  The orders are even where
+    // the image x axis is as close to x as a power of y's closeness: the square (yaw 47 at pitch
+    // 34, 60 at 45), or 1.3 where the pixels are wide (300x200 over 256^3, x / y in us: pitch 25
+    // and yaw 30 121 / 116, 34 and 45 164 / 154, 45 and 60 165 / 170, 55 and 60 139 / 177); from
+    // 66 degrees of yaw on x fastest only leads where y is all but out of sight.
+    double y_fastest_gain(const Geom& g, const double* proj, const double* mv, double height)
+    {
+        const ImageAxes a = image_axes(mv);
+        return (a.x < 0.4 ? a.y : std::pow(a.y, dense_pixels(g, proj, mv, height) ? 2.0 : 1.3)) - a.x;
+    }
+
+    // the order that context c's settings prescribe, -1: none
+    int32_t prescribed_order(const isaacb_ctx* c)
+    {
+        return c->heldOrder >= 0 ? c->heldOrder : c->slotOrder;
+    }
+
+    // Slot order of the combined textures for the camera of the merge about to run (Geom::yfast).
+    // Where L2 holds much of the texture and the frame fills the SMs the choice is left at x
+    // fastest: for the full-feature scene (256^3, 0.33 GB, 1920x1080) y fastest costs its pixel
+    // passes more than it gains (shading and march 236 us against 252), while small frames gain
+    // (500x300 over 128^3: 115 -> 92 us at yaw 60).  Only the speed depends on it: both orders
+    // hold the same texels.
     int32_t slot_order_for_camera(const isaacb_ctx* c)
     {
-        if(c->heldOrder >= 0)
-            return c->heldOrder;
-        if(c->slotOrder >= 0)
-            return c->slotOrder;
+        if(prescribed_order(c) >= 0)
+            return prescribed_order(c);
         const double textureBytes = double(brick_count(c->g)) * kSlotsPerBrick * sizeof(uint4);
         const long long warps = (long long) ((c->desc.framebuffer[0] + 7) / 8) * ((c->desc.framebuffer[1] + 3) / 4);
         if(textureBytes < 4.0 * 126.0e6 && warps > 148 * 64)
             return 0;
-        const ImageAxes a = image_axes(c->mv);
-        return a.y > a.x ? 1 : 0;
+        return y_fastest_gain(c->g, c->proj, c->mv, c->desc.framebuffer[1]) > 0.0 ? 1 : 0;
     }
 
     // the order of the merge about to be enqueued on `st`.  Under a stream capture nothing is
@@ -1814,6 +1832,8 @@ struct isaacb_batch
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t graphExec = nullptr;
     bool graphUpdate = false;
+    std::vector<size_t> same; // per context, the first index of the same one
+    std::vector<int32_t> orders; // per context, the slot order of the batch's own merges (batch_choose_orders)
     std::vector<MergeParams> graphMerges; // merge parameters a captured graph holds
     uint32_t launches = 0; // kernels the last enqueue (direct or captured) issued
 };
@@ -1866,14 +1886,22 @@ namespace
         inverse4(PM, out);
     }
 
-    // Slot order of the texture that the batch's own merge of context i writes: the views look
-    // from every side, and y fastest suits any yaw at moderate pitch (slot_order_for_camera:
-    // 5.4-6.2 L1 cycles a load up to 20 degrees of pitch, 10-11 at 34) where x fastest is as
-    // good only within 20 degrees of one axis and takes 12-15 beyond 45.
-    int32_t batch_slot_order(const isaacb_batch* b, size_t i)
+    // Slot orders of the textures that the batch's own merges write: by what the views of a
+    // context gain together, each by its pixels.  Eight views from every side at up to 34 degrees
+    // of pitch gain from y fastest (24.1 -> 21.2 ms with two merges), four from the front at 34
+    // degrees or from the top lose by it (14.9 -> 15.7 and 15.2 -> 17.7 ms).
+    void batch_choose_orders(isaacb_batch* b)
     {
-        const isaacb_ctx* c = b->ctxs[i];
-        return c->heldOrder >= 0 ? c->heldOrder : c->slotOrder >= 0 ? c->slotOrder : 1;
+        std::vector<double> gain(b->ctxs.size(), 0.0);
+        for(const isaacb_view& v : b->views)
+            gain[b->same[v.ctx_index]] += double(v.width) * v.height
+                * y_fastest_gain(b->ctxs[v.ctx_index]->g, v.projection, v.modelview, v.height);
+        b->orders.resize(b->ctxs.size());
+        for(size_t i = 0; i < b->ctxs.size(); ++i)
+        {
+            const int32_t p = prescribed_order(b->ctxs[i]);
+            b->orders[i] = p >= 0 ? p : gain[b->same[i]] > 0.0 ? 1 : 0;
+        }
     }
     // the order that context i's texture has once the batch has drawn: of the merge about to
     // run (a captured graph's, where there is one), else of the texture in memory
@@ -1881,7 +1909,7 @@ namespace
     {
         if(!update)
             return b->ctxs[i]->g.yfast;
-        return graph ? b->graphMerges[i].g.yfast : batch_slot_order(b, i);
+        return graph ? b->graphMerges[i].g.yfast : b->orders[i];
     }
 
     // host mirror of the device tables from the contexts' current state, for the textures as
@@ -1963,7 +1991,7 @@ namespace
                     if(!c->src[s] && (c->weight[s] != 0.0f || c->iso[s] != 0.0f))
                         return batch_fail(ISAACB_NOT_READY, "isaacb_batch: a source has no memory");
                 MergeParams p{};
-                prepare_merge(c, batch_slot_order(b, i), p);
+                prepare_merge(c, b->orders[i], p);
                 b->launches += uint32_t(launch_merge(p, st));
                 if(capture)
                     b->graphMerges.push_back(p); // the texture has its order once the graph is launched
@@ -2025,9 +2053,13 @@ namespace
             return false;
         for(size_t i = 0; i < b->ctxs.size(); ++i)
         {
+            if(i >= b->graphMerges.size())
+                return true;
+            // a graph keeps the orders of its capture, whatever the cameras since
+            const int32_t p0 = prescribed_order(b->ctxs[i]);
             MergeParams p{};
-            prepare_merge(b->ctxs[i], batch_slot_order(b, i), p);
-            if(i >= b->graphMerges.size() || std::memcmp(&p, &b->graphMerges[i], sizeof(MergeParams)) != 0)
+            prepare_merge(b->ctxs[i], p0 >= 0 ? p0 : b->graphMerges[i].g.yfast, p);
+            if(std::memcmp(&p, &b->graphMerges[i], sizeof(MergeParams)) != 0)
                 return true;
         }
         return false;
@@ -2061,6 +2093,9 @@ extern "C"
         isaacb_batch* b = new isaacb_batch;
         b->ctxs.assign(ctxs, ctxs + n_ctx);
         b->views.assign(views, views + n_views);
+        std::map<isaacb_ctx*, size_t> first;
+        for(uint32_t i = 0; i < n_ctx; ++i)
+            b->same.push_back(first.emplace(ctxs[i], size_t(i)).first->second);
         int dev = 0;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&b->numSMs, cudaDevAttrMultiProcessorCount, dev);
@@ -2137,6 +2172,8 @@ extern "C"
         if(!b)
             return ISAACB_INVALID_ARG;
         cudaStream_t st = (cudaStream_t) stream;
+        if(update)
+            batch_choose_orders(b);
         isaacb_status r = batch_upload_luts(b, st);
         if(r == ISAACB_OK)
             r = batch_refresh(b, st, update != 0, false);
@@ -2150,6 +2187,8 @@ extern "C"
         if(!b || !stream)
             return batch_fail(ISAACB_INVALID_ARG, "isaacb_batch_capture: needs a non-default stream");
         cudaStream_t st = (cudaStream_t) stream;
+        if(update)
+            batch_choose_orders(b);
         isaacb_status r = batch_upload_luts(b, st);
         if(r == ISAACB_OK)
             r = batch_refresh(b, st, update != 0, false);

@@ -173,3 +173,43 @@ def test_lanes_along_rows_and_down_columns(yaw, pitch, fb, interpolation):
         assert np.array_equal(f, frames[0])
     batch.close()
     viz.close()
+
+
+def test_batch_orders_by_its_views():
+    """One context under views from the front and the side, listed once or twice, single and
+    captured, while cameras move: frames equal single views whatever order is chosen."""
+    viz = _viz()
+    front, side = _reference(), _reference(camera=SIDE)
+    for ctxs, views in (([viz], [(0, *FB, *FRONT)] * 3 + [(0, *FB, *SIDE)]), ([viz, viz], [(0, *FB, *FRONT), (1, *FB, *SIDE), (1, *FB, *SIDE)])):
+        batch = IsaacBatch(ctxs, views)
+        want = [front if v[3] is FRONT[0] and v[4] is FRONT[1] else side for v in views]
+
+        def check():
+            torch.cuda.synchronize()
+            for f, w in zip(batch.frames, want):
+                assert np.array_equal(f.cpu().numpy(), w)
+                f.zero_()
+            assert np.array_equal(_frame(viz), front)
+
+        batch.render(update=True)
+        check()
+        viz.update()
+        batch.render(update=False)
+        check()
+        stream = torch.cuda.Stream()
+        with torch.cuda.stream(stream):
+            batch.capture(update=True)
+            batch.launchGraph()
+        stream.synchronize()
+        check()
+        for i in range(len(views)):  # every view to the other side
+            batch.setCamera(i, *(SIDE if want[i] is front else FRONT))
+            want[i] = side if want[i] is front else front
+        with torch.cuda.stream(stream):
+            batch.launchGraph()
+        stream.synchronize()
+        check()
+        batch.render(update=True)
+        check()
+        batch.close()
+    viz.close()
