@@ -96,3 +96,16 @@ def test_minmax_off_a_16_byte_boundary(offset):
     mn, mx = viz.minMax()
     assert mn[0] == t[..., 0].min().item() and mx[0] == t[..., 0].max().item()
     viz.close()
+
+
+@pytest.mark.parametrize("size", [(1, 5, 3), (37, 9, 4), (260, 3, 2), (40, 6, 5)])
+@pytest.mark.parametrize("count", [1, 2, 3, 4])
+@pytest.mark.parametrize("guard", [0, 1])
+def test_scalar_sources_with_tables_beyond_shared_memory(size, count, guard):
+    """Ragged and aligned rows, with ghost cells or none, with and without iso output."""
+    ts = 8192
+    for iso in ([], [0.0] * (count - 1) + [0.4]):
+        s = _scene(size, (1,) * count, seed=sum(size) + count, guard=guard, transfer_size=ts, iso=iso)
+        s.functions = ["idem"] * count
+        s.transfer = [{0: (0.1, 0.2, 0.3, 0.0), ts // 2: (0.9, 0.4, 0.1, 0.6), ts: (0.2, 0.8, 0.9, 0.9)}] * count
+        _check(s)
