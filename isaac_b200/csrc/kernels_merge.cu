@@ -695,7 +695,9 @@ namespace isaacb
         return true;
     }
 
-    template<bool ISO>
+    // PLAIN: no source has ghost cells, one index for all (pow chain over 400 x 400 x 300 voxels
+    // 1.09 ms an update, 1.11 with an index each)
+    template<bool ISO, bool PLAIN>
     __global__ void __launch_bounds__(256) k_merge_voxels(const __grid_constant__ MergeParams p)
     {
         __shared__ uint8_t sMask[64];
@@ -717,7 +719,7 @@ namespace isaacb
             if(!(vw + it > 0.0f))
                 continue;
             float val;
-            const size_t si = size_t(z) * p.pitchZ[s] + size_t(y) * p.pitchY[s] + x;
+            const size_t si = PLAIN ? i : size_t(z) * p.pitchZ[s] + size_t(y) * p.pitchY[s] + x;
             if(p.chainIdem[s] != 0)
                 val = __ldg(p.src[s] + si * p.fdim[s]); // every functor idem: the x component
             else
@@ -980,8 +982,10 @@ namespace isaacb
                     launch_voxels_n<ISO, true>(p, act, vgrid, s);
                 else if(few)
                     launch_voxels_n<ISO, false>(p, act, vgrid, s);
+                else if(plain)
+                    k_merge_voxels<ISO, true><<<vgrid, 256, 0, s>>>(p);
                 else
-                    k_merge_voxels<ISO><<<vgrid, 256, 0, s>>>(p);
+                    k_merge_voxels<ISO, false><<<vgrid, 256, 0, s>>>(p);
             }
         }
         const dim3 pgrid((p.g.nb[0] + kPackRow - 1) / kPackRow, p.g.nb[1], p.g.nb[2]);

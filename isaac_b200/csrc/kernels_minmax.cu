@@ -18,11 +18,12 @@ namespace isaacb
 {
     constexpr int kMMThreads = 256;
 
-    // voxel i of the interior in x, y, z order
+    // voxel i of the interior in x, y, z order.  PLAIN: no ghost cells
+    template<bool PLAIN>
     __device__ __forceinline__ float mm_value(const MinMaxParams& p, size_t i)
     {
         float v[4];
-        if(p.pitchY != size_t(p.g.ls[0]))
+        if(!PLAIN)
         {
             const size_t row = i / size_t(p.g.ls[0]), z = row / size_t(p.g.ls[1]);
             i = z * p.pitchZ + (row - z * size_t(p.g.ls[1])) * p.pitchY + (i - row * size_t(p.g.ls[0]));
@@ -101,7 +102,9 @@ namespace isaacb
             *p.ticket = 0u;
     }
 
-    // any source or particle source, one value at a time
+    // any source or particle source, one value at a time.  PLAIN: no ghost cells (a pow chain
+    // over 400 x 400 x 300 voxels 0.64 ms, 0.68 with the pitches asked for each value)
+    template<bool PLAIN>
     __global__ void __launch_bounds__(kMMThreads) k_minmax(const __grid_constant__ MinMaxParams p)
     {
         float lo = FLT_MAX, hi = -FLT_MAX;
@@ -110,7 +113,7 @@ namespace isaacb
             const size_t n = size_t(p.g.ls[0]) * p.g.ls[1] * p.g.ls[2];
             for(size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x; i < n; i += size_t(gridDim.x) * blockDim.x)
             {
-                const float v = mm_value(p, i);
+                const float v = mm_value<PLAIN>(p, i);
                 lo = gmin(lo, v);
                 hi = gmax(hi, v);
             }
@@ -179,7 +182,7 @@ namespace isaacb
         }
         if(blockIdx.x == 0 && threadIdx.x < n - 4 * groups)
         {
-            const float v = mm_value(p, 4 * groups + threadIdx.x);
+            const float v = mm_value<true>(p, 4 * groups + threadIdx.x);
             lo = gmin(lo, v);
             hi = gmax(hi, v);
         }
@@ -197,11 +200,15 @@ namespace isaacb
     void launch_minmax(const MinMaxParams& p, cudaStream_t s)
     {
         LineChain line;
-        const bool vec = !p.particle && p.pitchY == size_t(p.g.ls[0]) && (reinterpret_cast<uintptr_t>(p.src) & 15u) == 0
+        const bool plain = p.particle || p.pitchY == size_t(p.g.ls[0]);
+        const bool vec = !p.particle && plain && (reinterpret_cast<uintptr_t>(p.src) & 15u) == 0
             && line_chain_of(p.chain, line);
         if(!vec)
         {
-            k_minmax<<<minmax_blocks(p), kMMThreads, 0, s>>>(p);
+            if(plain)
+                k_minmax<true><<<minmax_blocks(p), kMMThreads, 0, s>>>(p);
+            else
+                k_minmax<false><<<minmax_blocks(p), kMMThreads, 0, s>>>(p);
             return;
         }
         const int blocks = minmax_blocks(p, 4);
@@ -216,6 +223,7 @@ namespace isaacb
 
     // Reference scan-order key of the first +0 and the first -0:
     // keys[0] = first +0, keys[1] = first -0 (64-bit order keys, ULLONG_MAX if none)
+    template<bool PLAIN>
     __global__ void __launch_bounds__(kMMThreads) k_minmax_zero_keys(const __grid_constant__ MinMaxParams p)
     {
         if(!p.particle)
@@ -224,7 +232,7 @@ namespace isaacb
             const size_t n = size_t(LX) * LY * LZ;
             for(size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x; i < n; i += size_t(gridDim.x) * blockDim.x)
             {
-                const float v = mm_value(p, i);
+                const float v = mm_value<PLAIN>(p, i);
                 if(v == 0.0f)
                 {
                     const size_t x = i % LX, y = (i / LX) % LY, z = i / (size_t(LX) * LY);
@@ -258,6 +266,9 @@ namespace isaacb
 
     void launch_minmax_zero_keys(const MinMaxParams& p, cudaStream_t s)
     {
-        k_minmax_zero_keys<<<minmax_blocks(p), kMMThreads, 0, s>>>(p);
+        if(p.particle || p.pitchY == size_t(p.g.ls[0]))
+            k_minmax_zero_keys<true><<<minmax_blocks(p), kMMThreads, 0, s>>>(p);
+        else
+            k_minmax_zero_keys<false><<<minmax_blocks(p), kMMThreads, 0, s>>>(p);
     }
 } // namespace isaacb
