@@ -123,7 +123,8 @@ namespace isaacb
     size_t conv_gemm_smem(int Npad, int Kpad);
     // the row-tile kernel takes this convolution (and then honours xUp)
     bool row_tiles_apply(const ConvGemmParams& p);
+    // false where no kernel takes it: nothing was launched
     bool launch_conv_gemm(ConvGemmParams p, cudaStream_t s);
-    // the weight gradients of n layers (at most kWgradLayers) in one launch
+    // the weight gradients of n layers (1 to kWgradLayers) in one launch; false as above
     bool launch_conv_wgrad(const WgradParams* layers, int n, cudaStream_t s);
 } // namespace isaacb

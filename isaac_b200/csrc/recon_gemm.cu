@@ -1438,8 +1438,9 @@ namespace isaacb
                 return true;
             }
         }
+        // k_conv_gemm knows no second input: it would read x as if that held all Cg channels
         const size_t smem = conv_gemm_smem(p.Npad, p.Kpad);
-        if(smem > 227 * 1024)
+        if(smem > 227 * 1024 || p.xUp)
             return false;
         cudaFuncSetAttribute(k_conv_gemm, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
         cudaFuncSetAttribute(k_conv_gemm, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
@@ -1477,6 +1478,8 @@ namespace isaacb
 
     bool launch_conv_wgrad(const WgradParams* layers, int n, cudaStream_t s)
     {
+        if(n < 1 || n > kWgradLayers)
+            return false;
         WgradTable T{};
         size_t smem = 0, work = 0;
         int npad = 0;

@@ -135,3 +135,19 @@ def test_parser_token_fuzz_matches_oracle():
         e2, b2, p2 = O.parse_chain(text)
         assert (e1, b1) == (e2, b2), text
         assert np.array_equal(np.array(p1, dtype=np.float32), np.array(p2, dtype=np.float32), equal_nan=True), text
+
+
+def test_convolution_launchers_refuse_what_their_kernels_cannot_take(tmp_path):
+    """The internal launchers, which the network's code calls, through a small program: a
+    concatenation that would reach the kernel that ignores it, and too many layers."""
+    import shutil
+    import subprocess
+
+    from isaac_b200 import build as B
+
+    exe = tmp_path / "conv_limits"
+    nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
+    subprocess.run([nvcc, "-std=c++17", "-gencode", "arch=compute_100a,code=sm_100a", str(B.ROOT / "tests" / "cpp" / "conv_limits.cu"),
+                    "-L", str(B.OUT_DIR), "-lisaac_b200", "-Xlinker", f"-rpath={B.OUT_DIR}", "-o", str(exe)], check=True, capture_output=True)
+    r = subprocess.run([str(exe)], capture_output=True, text=True)
+    assert r.returncode == 0, r.stdout + r.stderr
