@@ -338,7 +338,7 @@ struct isaacb_ctx
     float* mmResult = nullptr; // min and max of each source
     unsigned int* mmTicket = nullptr;
     unsigned long long* mmKeys = nullptr;
-    uint8_t* framePinned = nullptr; // staging of isaacb_frame's readback, allocated by its first use
+    uint8_t* framePinned = nullptr; // staging of isaacb_frame's readback, behind the tables in lutPinned (null: too large)
     // count of all-zero bricks of the last merge (device memory); the march reads it and
     // checks brick emptiness only when it is not zero
     unsigned int* emptyDev = nullptr;
@@ -820,7 +820,11 @@ namespace
         return here && (reinterpret_cast<uintptr_t>(rgba) & 3u) == 0 ? FRAME_STORE : FRAME_COPY;
     }
 
-    // largest frame that isaacb_frame reads through its own staging buffer
+    // Largest frame that isaacb_frame reads through its own pinned buffer.  A small frame
+    // reaches pageable memory faster by it than by the driver's own staging; larger ones, and
+    // memory that the caller has pinned, are copied by the driver, which overlaps its pieces.
+    // Whole frames of a 32^3 field, staged / driver in us: 200x150 53 / 55, 256x256 67 / 73,
+    // 512x512 153 / 167 (158 / 147 on another machine), 800x600 273 / 235.
     constexpr size_t kFrameStaging = 256 * 1024;
 } // namespace
 
@@ -925,8 +929,13 @@ extern "C"
         alloc((void**) &c->lutDev, c->lutHost.size() * sizeof(float));
         alloc((void**) &c->lutPre, c->lutHost.size() * sizeof(float));
         alloc((void**) &c->psPre, (c->lutHost.size() + size_t(kMaxSources) * 4) * sizeof(float)); // one entry more each
+        // the staging buffers of the tables and of small frames, one pinned allocation
+        const size_t lutBytes = (c->lutHost.size() * sizeof(float) + 255) / 256 * 256;
+        const size_t staged = npix * sizeof(uchar4) <= kFrameStaging ? npix * sizeof(uchar4) : 0;
         if(e == cudaSuccess)
-            e = cudaMallocHost((void**) &c->lutPinned, c->lutHost.size() * sizeof(float));
+            e = cudaMallocHost((void**) &c->lutPinned, lutBytes + staged);
+        if(e == cudaSuccess && staged)
+            c->framePinned = reinterpret_cast<uint8_t*>(c->lutPinned) + lutBytes;
         if(e == cudaSuccess)
             e = cudaEventCreateWithFlags(&c->lutEvent, cudaEventDisableTiming);
         alloc((void**) &c->volQ, nbr * kSlotsPerBrick * sizeof(uint4));
@@ -994,8 +1003,6 @@ extern "C"
         cudaFree(c->mmResult);
         cudaFree(c->mmTicket);
         cudaFree(c->mmKeys);
-        if(c->framePinned)
-            cudaFreeHost(c->framePinned);
         for(int s = 0; s < kMaxSources; ++s)
         {
             cudaFree(c->adv[s]);
@@ -1632,15 +1639,9 @@ extern "C"
             return r;
         cudaStream_t st = (cudaStream_t) stream;
         const size_t bytes = size_t(c->desc.framebuffer[0]) * c->desc.framebuffer[1] * 4;
-        // A small frame reaches pageable memory through a pinned copy: the driver's own staging
-        // costs more per call (200x150 pixels 59 against 62 us for the whole frame).  Larger
-        // frames (512x512: 158 against 147 us) and memory the caller has pinned are copied by
-        // the driver, which overlaps its pieces.
         cudaPointerAttributes attr{};
-        if(bytes <= kFrameStaging && cudaPointerGetAttributes(&attr, rgba_host) == cudaSuccess && attr.type == cudaMemoryTypeUnregistered)
+        if(c->framePinned && cudaPointerGetAttributes(&attr, rgba_host) == cudaSuccess && attr.type == cudaMemoryTypeUnregistered)
         {
-            if(!c->framePinned)
-                ISAACB_CUDA(c, cudaMallocHost((void**) &c->framePinned, bytes), "frame staging buffer");
             ISAACB_CUDA(c, cudaMemcpyAsync(c->framePinned, c->color, bytes, cudaMemcpyDeviceToHost, st), "frame readback");
             ISAACB_CUDA(c, cudaStreamSynchronize(st), "isaacb_frame");
             std::memcpy(rgba_host, c->framePinned, bytes);

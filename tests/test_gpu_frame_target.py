@@ -7,7 +7,7 @@ import pytest
 import torch
 
 from harness import build_gpu, gaussian_pair
-from isaac_b200 import _lib
+from isaac_b200 import _lib, scenes
 
 pytestmark = pytest.mark.gpu
 
@@ -64,4 +64,24 @@ def test_pageable_memory_is_refused_before_any_launch():
     torch.cuda.synchronize()
     assert (out == SENTINEL).all()
     assert np.array_equal(viz.doVisualization(), ref)
+    viz.close()
+
+
+@pytest.mark.parametrize("fb", [(61, 37), (256, 256), (257, 256)])
+def test_host_frames_pageable_and_pinned(fb):
+    """Frames that pass the context's own pinned buffer, the largest of them and the next
+    size, into memory of either kind, twice each, with one camera and then another."""
+    viz = build_gpu(gaussian_pair(32, fb=fb))
+    dev = torch.empty((fb[1], fb[0], 4), dtype=torch.uint8, device="cuda")
+    pageable = np.full((fb[1], fb[0], 4), SENTINEL, dtype=np.uint8)
+    pinned = torch.full((fb[1], fb[0], 4), SENTINEL, dtype=torch.uint8).pin_memory().numpy()
+    seen = []
+    for seed in (1, 7):
+        viz.setCamera(*scenes.camera(*fb, seed=seed))
+        ref = viz.doVisualization(host=False, out=dev).cpu().numpy()
+        for out in (pageable, pinned, pageable):
+            assert viz.doVisualization(out=out) is out
+            assert np.array_equal(out, ref)
+        seen.append(ref)
+    assert not np.array_equal(*seen)
     viz.close()
