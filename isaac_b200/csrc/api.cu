@@ -714,8 +714,7 @@ namespace
         if(prescribed_order(c) >= 0)
             return prescribed_order(c);
         const double textureBytes = double(brick_count(c->g)) * kSlotsPerBrick * sizeof(uint4);
-        const long long warps = (long long) ((c->desc.framebuffer[0] + 7) / 8) * ((c->desc.framebuffer[1] + 3) / 4);
-        if(textureBytes < 4.0 * 126.0e6 && warps > 148 * 64)
+        if(textureBytes < 4.0 * 126.0e6 && frame_warps_per_sm(int32_t(c->desc.framebuffer[0]), int32_t(c->desc.framebuffer[1])) > kFullWarps)
             return 0;
         return y_fastest_gain(c->g, c->proj, c->mv, c->desc.framebuffer[1]) > 0.0 ? 1 : 0;
     }

@@ -300,6 +300,10 @@ namespace isaacb
     void launch_iso_per_source(const FrameParams& p, cudaStream_t s);
     void launch_ssao(const FrameParams& p, cudaStream_t s);
     void launch_shade_volume(const FrameParams& p, bool volume, bool clean, cudaStream_t s);
+    // warps of 32 pixels that an SM of the current device gets from a frame, rounded up; with
+    // more than kFullWarps the other rays cover a ray's loads (ShadeShape)
+    constexpr long long kFullWarps = 64;
+    long long frame_warps_per_sm(int32_t width, int32_t height);
     // the per-source volume pass can be a frame's only one (clean)
     bool per_source_specialised(const FrameParams& p);
     // returns the number of kernels it launched

@@ -445,7 +445,7 @@ namespace isaacb
         SHADE_MID,
         SHADE_FEW
     };
-    constexpr int kShadeFewWarps = 24, kShadeMidWarps = 64; // most warps per SM of FEW and MID
+    constexpr long long kShadeFewWarps = 24; // most warps per SM of FEW; of MID kFullWarps
     __host__ __device__ constexpr int shade_threads(ShadeShape sh)
     {
         return sh == SHADE_FEW ? 64 : 128;
@@ -540,10 +540,9 @@ namespace isaacb
             clean ? launch_shade_volume_as<SHAPE, false, true>(p, volume, s) : launch_shade_volume_as<SHAPE, false, false>(p, volume, s);
     }
 
-    void launch_shade_volume(const FrameParams& p, bool volume, bool clean, cudaStream_t s)
+    long long frame_warps_per_sm(int32_t width, int32_t height)
     {
-        // SMs, once per device
-        static std::atomic<int> smCount[64]{};
+        static std::atomic<int> smCount[64]{}; // asked once per device
         int dev = 0, sms = 148;
         cudaGetDevice(&dev);
         if(dev >= 0 && dev < 64)
@@ -555,10 +554,16 @@ namespace isaacb
             }
             sms = smCount[dev].load();
         }
-        const long long warps = (long long) ((p.v.W + 7) / 8) * ((p.v.H + 3) / 4);
-        if(!volume || warps > (long long) sms * kShadeMidWarps)
+        const long long warps = (long long) ((width + 7) / 8) * ((height + 3) / 4);
+        return (warps + sms - 1) / sms;
+    }
+
+    void launch_shade_volume(const FrameParams& p, bool volume, bool clean, cudaStream_t s)
+    {
+        const long long warps = frame_warps_per_sm(p.v.W, p.v.H);
+        if(!volume || warps > kFullWarps)
             launch_shade_volume_shape<SHADE_FULL>(p, volume, clean, s);
-        else if(warps > (long long) sms * kShadeFewWarps)
+        else if(warps > kShadeFewWarps)
             launch_shade_volume_shape<SHADE_MID>(p, volume, clean, s);
         else
             launch_shade_volume_shape<SHADE_FEW>(p, volume, clean, s);

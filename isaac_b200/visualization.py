@@ -305,7 +305,7 @@ class IsaacVisualization:
 
     def setSlotOrder(self, order: int = -1):
         """Slot order inside the combined texture's bricks: -1 chosen by each merge from its
-        camera (textures beyond 4x L2, frames up to 300,000 pixels), 0 x fastest, 1 y fastest.  Speed only."""
+        camera (textures beyond 4x L2, frames of up to 64 warps of pixels an SM), 0 x fastest, 1 y fastest.  Speed only."""
         check(self.lib.isaacb_set_slot_order(self.ctx, int(order)), self.ctx)
 
     def setRenderOptimization(self, on: bool):
