@@ -37,7 +37,7 @@ typedef enum isaacb_status
     ISAACB_INVALID_ARG = 1,
     ISAACB_PARSE_ERROR = 2, /* functor chain had an error code; the parsed prefix is applied */
     ISAACB_CUDA_ERROR = 3,
-    ISAACB_TIMEOUT = 4,
+    ISAACB_TIMEOUT = 4, /* no call returns it at present */
     ISAACB_OOM = 5,
     ISAACB_NOT_READY = 6 /* a required input (source pointer, camera) was never set */
 } isaacb_status;

@@ -371,10 +371,12 @@ namespace isaacb
     // the full-feature scene (256^3, 5 floats a voxel, iso output) and 250 us on a scalar
     // with an advected vector field; this form takes 193 and 137 (one voxel a thread at three
     // CTAs per SM 221 and 161, four a thread 290 and 138).
-        constexpr int kRowsThreads = 512, kRowsPer = 2, kRowsMaxSources = 4;
+    constexpr int kRowsThreads = 512, kRowsPer = 2, kRowsMaxSources = 4;
     // tables of one CTA, so that two fit on an SM (6 tables of 1024 entries)
     constexpr size_t kRowsSmem = 96 * 1024;
 
+    // division by an invariant divisor as a multiply and a shift (Granlund and Montgomery, 1994:
+    // the multiplier floor(2^(31 + l) / d) + 1 with 2^l >= d is exact for 31-bit dividends)
     struct FastDiv
     {
         uint32_t d, m, s; // n / d == umulhi(n, m) >> s for n < 2^31 (d > 1)

@@ -903,41 +903,41 @@ namespace isaacb
                             const uint64_t swDesc = (tc::smem_desc(0, 16u, swSpan) & ~uint64_t(0x3FFF))
                                 | (uint64_t(rowB == 32 ? 6 : rowB == 64 ? 4 : 2) << 61);
                             for(int cx = 0; cx < nPar; ++cx, acc = 0)
-                            for(int ty = 0; ty < nRows; ++ty)
-                                for(int tx = par ? (cx + pad) & 1 : 0; tx < ks; tx += tapStep)
-                                {
-                                    const int col = par ? ((cx + pad - tx) >> 1) + 1 : p.transposed ? 2 * pad - tx : tx;
-                                    const int q = col & (S - 1), idx0 = S == 1 ? col : (col >> 1);
-                                    const uint32_t d = dTile + uint32_t(cx * p.Npad);
-                                    uint32_t addr = st + uint32_t(ty * S + q) * rowPitch + uint32_t(idx0 * rowB);
-                                    uint32_t bOff = uint32_t(((ty0 + tapStep * ty) * ks + tx) * p.Cg);
-                                    for(int jp = 0; jp < nC / 2; ++jp)
+                                for(int ty = 0; ty < nRows; ++ty)
+                                    for(int tx = par ? (cx + pad) & 1 : 0; tx < ks; tx += tapStep)
                                     {
-                                        tc::mma_bf16(d, swDesc | uint64_t((addr >> 4) & 0x3FFFu), bBase + bOff, idesc, acc);
-                                        acc = 1;
-                                        addr += 32u;
-                                        bOff += 16u;
+                                        const int col = par ? ((cx + pad - tx) >> 1) + 1 : p.transposed ? 2 * pad - tx : tx;
+                                        const int q = col & (S - 1), idx0 = S == 1 ? col : (col >> 1);
+                                        const uint32_t d = dTile + uint32_t(cx * p.Npad);
+                                        uint32_t addr = st + uint32_t(ty * S + q) * rowPitch + uint32_t(idx0 * rowB);
+                                        uint32_t bOff = uint32_t(((ty0 + tapStep * ty) * ks + tx) * p.Cg);
+                                        for(int jp = 0; jp < nC / 2; ++jp)
+                                        {
+                                            tc::mma_bf16(d, swDesc | uint64_t((addr >> 4) & 0x3FFFu), bBase + bOff, idesc, acc);
+                                            acc = 1;
+                                            addr += 32u;
+                                            bOff += 16u;
+                                        }
                                     }
-                                }
                         }
                         else
-                        for(int cx = 0; cx < nPar; ++cx, acc = 0)
-                        for(int ty = 0; ty < nRows; ++ty)
-                            for(int tx = par ? (cx + pad) & 1 : 0; tx < ks; tx += tapStep)
-                            {
-                                const int col = par ? ((cx + pad - tx) >> 1) + 1 : p.transposed ? 2 * pad - tx : tx;
-                                const int q = col & (S - 1), idx0 = S == 1 ? col : (col >> 1);
-                                const uint32_t d = dTile + uint32_t(cx * p.Npad);
-                                uint32_t aOff = uint32_t((ty * nC * S + q) * HWp + idx0);
-                                uint32_t bOff = uint32_t(((ty0 + tapStep * ty) * ks + tx) * p.Cg);
-                                for(int jp = 0; jp < nC / 2; ++jp)
-                                {
-                                    tc::mma_bf16(d, aBase + aOff, bBase + bOff, idesc, acc);
-                                    acc = 1;
-                                    aOff += uint32_t(2 * S * HWp);
-                                    bOff += 16u;
-                                }
-                            }
+                            for(int cx = 0; cx < nPar; ++cx, acc = 0)
+                                for(int ty = 0; ty < nRows; ++ty)
+                                    for(int tx = par ? (cx + pad) & 1 : 0; tx < ks; tx += tapStep)
+                                    {
+                                        const int col = par ? ((cx + pad - tx) >> 1) + 1 : p.transposed ? 2 * pad - tx : tx;
+                                        const int q = col & (S - 1), idx0 = S == 1 ? col : (col >> 1);
+                                        const uint32_t d = dTile + uint32_t(cx * p.Npad);
+                                        uint32_t aOff = uint32_t((ty * nC * S + q) * HWp + idx0);
+                                        uint32_t bOff = uint32_t(((ty0 + tapStep * ty) * ks + tx) * p.Cg);
+                                        for(int jp = 0; jp < nC / 2; ++jp)
+                                        {
+                                            tc::mma_bf16(d, aBase + aOff, bBase + bOff, idesc, acc);
+                                            acc = 1;
+                                            aOff += uint32_t(2 * S * HWp);
+                                            bOff += 16u;
+                                        }
+                                    }
                         tc::mma_commit(&sEmpty[s]);
                         tc::mma_commit(&sAccFull[a]);
                     }
