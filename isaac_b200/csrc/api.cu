@@ -679,6 +679,12 @@ namespace
         return image_axes(mv).y < kColumnAxis && dense_pixels(g, proj, mv, height) ? 0 : 1;
     }
 
+    // a combined texture of at least four times the L2 cache
+    bool beyond_l2(const Geom& g)
+    {
+        return double(brick_count(g)) * kSlotsPerBrick * sizeof(uint4) >= 4.0 * 126.0e6;
+    }
+
     // What y-fastest slots gain over x-fastest ones for a camera, in no unit (about a third of
     // it is the relative time): positive where y fastest is the faster.  The march's warps walk
     // the slots' fast axis with image rows (x fastest) or image columns (y fastest), and L1 serves
@@ -688,13 +694,14 @@ namespace
     // 3.97 / 4.10, 60 4.52 / 3.96, 90 4.64 / 3.76; pitch 55 and yaw 45 3.32 / 4.09, 60 3.87 / 4.01,
     // 75 4.49 / 3.94; pitch 70 and yaw 60 3.52 / 3.91, 75 4.20 / 3.85.  The orders are even where
     // the image x axis is as close to x as a power of y's closeness: the square (yaw 47 at pitch
-    // 34, 60 at 45), or 1.3 where the pixels are wide (300x200 over 256^3, x / y in us: pitch 25
-    // and yaw 30 121 / 116, 34 and 45 164 / 154, 45 and 60 165 / 170, 55 and 60 139 / 177); from
-    // 66 degrees of yaw on x fastest only leads where y is all but out of sight.
+    // 34, 60 at 45), or 1.3 where the pixels are wide or L2 holds much of the texture (300x200
+    // over 256^3, x / y in us: pitch 25 and yaw 30 121 / 116, 34 and 45 164 / 154, 45 and 60 165
+    // / 170, 55 and 60 139 / 177; over 100^3: 44.7 / 42.8 and 53.8 / 51.7); from 66 degrees of
+    // yaw on x fastest only leads where y is all but out of sight.
     double y_fastest_gain(const Geom& g, const double* proj, const double* mv, double height)
     {
         const ImageAxes a = image_axes(mv);
-        return (a.x < 0.4 ? a.y : std::pow(a.y, dense_pixels(g, proj, mv, height) ? 2.0 : 1.3)) - a.x;
+        return (a.x < 0.4 ? a.y : std::pow(a.y, beyond_l2(g) && dense_pixels(g, proj, mv, height) ? 2.0 : 1.3)) - a.x;
     }
 
     // the order that context c's settings prescribe, -1: none
@@ -713,8 +720,7 @@ namespace
     {
         if(prescribed_order(c) >= 0)
             return prescribed_order(c);
-        const double textureBytes = double(brick_count(c->g)) * kSlotsPerBrick * sizeof(uint4);
-        if(textureBytes < 4.0 * 126.0e6 && frame_warps_per_sm(int32_t(c->desc.framebuffer[0]), int32_t(c->desc.framebuffer[1])) > kFullWarps)
+        if(!beyond_l2(c->g) && frame_warps_per_sm(int32_t(c->desc.framebuffer[0]), int32_t(c->desc.framebuffer[1])) > kFullWarps)
             return 0;
         return y_fastest_gain(c->g, c->proj, c->mv, c->desc.framebuffer[1]) > 0.0 ? 1 : 0;
     }
