@@ -160,8 +160,9 @@ isaacb_status isaacb_set_storage(isaacb_ctx* ctx, uint32_t src, int32_t dtype);
 /* Slot order inside the combined texture's bricks (no reference counterpart; it
  * changes speed only, never a texel or a pixel).  -1 (default): chosen by each merge
  * from its camera for textures larger than 4x the L2 cache and for frames of up to 64
- * warps of pixels an SM (300,000 on 148 SMs), x fastest otherwise (in a batch's merges from the views' cameras;
- * a captured batch keeps its order); 0: x fastest; 1: y fastest.  Takes effect at the next update; once an update has been recorded by a
+ * warps of pixels an SM (300,000 on 148 SMs), x fastest otherwise; in a batch's merges
+ * from the views' cameras, where a captured batch keeps its order; 0: x fastest; 1: y
+ * fastest.  Takes effect at the next update; once an update has been recorded by a
  * stream capture, the context keeps the order that its texture had then. */
 isaacb_status isaacb_set_slot_order(isaacb_ctx* ctx, int32_t order);
 /* Background colour as handed to the draw callback (lib/isaac.hpp:2245-2249
