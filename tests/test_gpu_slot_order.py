@@ -213,3 +213,34 @@ def test_batch_orders_by_its_views():
         check()
         batch.close()
     viz.close()
+
+
+def test_batch_over_a_context_whose_update_was_captured():
+    """A batch merges in the order that the caller's graph writes, also where its own graph was
+    captured before: after either one's merge every draw is right."""
+    viz = _viz()
+    front, side = _reference(), _reference(camera=SIDE)
+    batch = IsaacBatch([viz], [(0, *FB, *SIDE)])
+    viz.update()
+    torch.cuda.synchronize()
+    stream = torch.cuda.Stream()
+    with torch.cuda.stream(stream):
+        batch.capture(update=True)
+        batch.launchGraph()  # y fastest, by its view
+    stream.synchronize()
+    viz.update()  # x fastest, by the camera
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        viz.update()
+    for merge in (graph.replay, lambda: batch.render(update=True), graph.replay, batch.launchGraph, graph.replay, viz.update, graph.replay):
+        with torch.cuda.stream(stream):
+            merge()
+        stream.synchronize()
+        assert np.array_equal(_frame(viz), front)
+        batch.frames[0].zero_()
+        batch.render(update=False)
+        torch.cuda.synchronize()
+        assert np.array_equal(batch.frames[0].cpu().numpy(), side)
+    batch.close()
+    viz.close()
