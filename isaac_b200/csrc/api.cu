@@ -694,14 +694,15 @@ namespace
     // 3.97 / 4.10, 60 4.52 / 3.96, 90 4.64 / 3.76; pitch 55 and yaw 45 3.32 / 4.09, 60 3.87 / 4.01,
     // 75 4.49 / 3.94; pitch 70 and yaw 60 3.52 / 3.91, 75 4.20 / 3.85.  The orders are even where
     // the image x axis is as close to x as a power of y's closeness: the square (yaw 47 at pitch
-    // 34, 60 at 45), or 1.3 where the pixels are wide or L2 holds much of the texture (300x200
-    // over 256^3, x / y in us: pitch 25 and yaw 30 121 / 116, 34 and 45 164 / 154, 45 and 60 165
-    // / 170, 55 and 60 139 / 177; over 100^3: 44.7 / 42.8 and 53.8 / 51.7); from 66 degrees of
-    // yaw on x fastest only leads where y is all but out of sight.
-    double y_fastest_gain(const Geom& g, const double* proj, const double* mv, double height)
+    // 34, 60 at 45; six 256x256 views of 128^3 at 34 and 45 385 / 392 us), or 1.3 where the pixels
+    // are wide or the draw leaves the SMs part empty (`full` false; 300x200 over 256^3, x / y in
+    // us: pitch 25 and yaw 30 121 / 116, 34 and 45 164 / 154, 45 and 60 165 / 170, 55 and 60 139 /
+    // 177; over 100^3: 44.7 / 42.8 and, at 34 and 40, 53.8 / 51.7); from 66 degrees of yaw on x
+    // fastest only leads where y is all but out of sight.
+    double y_fastest_gain(const Geom& g, const double* proj, const double* mv, double height, bool full)
     {
         const ImageAxes a = image_axes(mv);
-        return (a.x < 0.4 ? a.y : std::pow(a.y, beyond_l2(g) && dense_pixels(g, proj, mv, height) ? 2.0 : 1.3)) - a.x;
+        return (a.x < 0.4 ? a.y : std::pow(a.y, full && dense_pixels(g, proj, mv, height) ? 2.0 : 1.3)) - a.x;
     }
 
     // the order that context c's settings prescribe, -1: none
@@ -720,9 +721,10 @@ namespace
     {
         if(prescribed_order(c) >= 0)
             return prescribed_order(c);
-        if(!beyond_l2(c->g) && frame_warps_per_sm(int32_t(c->desc.framebuffer[0]), int32_t(c->desc.framebuffer[1])) > kFullWarps)
+        const bool full = frame_warps_per_sm(int32_t(c->desc.framebuffer[0]), int32_t(c->desc.framebuffer[1])) > kFullWarps;
+        if(!beyond_l2(c->g) && full)
             return 0;
-        return y_fastest_gain(c->g, c->proj, c->mv, c->desc.framebuffer[1]) > 0.0 ? 1 : 0;
+        return y_fastest_gain(c->g, c->proj, c->mv, c->desc.framebuffer[1], full) > 0.0 ? 1 : 0;
     }
 
     // the order of the merge about to be enqueued on `st`.  Under a stream capture nothing is
@@ -1901,7 +1903,7 @@ namespace
         std::vector<double> gain(b->ctxs.size(), 0.0);
         for(const isaacb_view& v : b->views)
             gain[b->same[v.ctx_index]] += double(v.width) * v.height
-                * y_fastest_gain(b->ctxs[v.ctx_index]->g, v.projection, v.modelview, v.height);
+                * y_fastest_gain(b->ctxs[v.ctx_index]->g, v.projection, v.modelview, v.height, true);
         b->orders.resize(b->ctxs.size());
         for(size_t i = 0; i < b->ctxs.size(); ++i)
         {
